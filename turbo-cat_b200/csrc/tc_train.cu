@@ -398,41 +398,10 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 struct HistShape {
-  static constexpr int W = 32;                          // histogram columns (features) of an item
-  static constexpr int WARPS = HIST_THREADS / 32;
-  static constexpr int S = 2;                           // staging depth per warp (batches in flight)
+  static constexpr int W = 32;                          // histogram columns (features) of an item at most
   static constexpr int FIELDS = 4;                      // u32 accumulators per (slot, column)
-  static constexpr size_t hist_bytes = (size_t)kSlots * FIELDS * W * 4;    // 128 KB
-  static constexpr size_t warp_bytes = (size_t)S * HIST_BATCH * (W + 8);   // bins + (grad, hess)
-  static constexpr size_t smem = hist_bytes + WARPS * warp_bytes;
+  static constexpr size_t smem = (size_t)kSlots * FIELDS * W * 4;  // 128 KB
 };
-static_assert(HistShape::smem <= 227 * 1024 - 1024, "histogram shared memory");
-
-// Work item -> segment (class, pair) through the cumulative item counts.
-__device__ __forceinline__ int find_seg(const int32_t* cum, int nseg, int item) {
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (cum[mid] <= item) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
-// Bin slots of a histogram column: a feature with n_edges edges uses bins
-// 0 .. n_edges (span = n_edges + 1) and the NaN slot 255, so the slots past
-// its span are free.  A feature without NaN rows keeps private copies of its
-// column there for different warps (copy c of bin b in slot c*span + b, at
-// most 255/span copies, so bin + offset never reaches 255), which spreads the
-// updates of few-bin features over more addresses.  A feature with NaN rows
-// keeps one copy.
-struct HistCol {
-  int span, copies;
-};
-__device__ __forceinline__ HistCol hist_col(const DevPtrs& P, int f, int nf) {
-  if (f >= nf) return {255, 1};
-  const int span = (int)P.n_edges[f] + 1;
-  return {span, P.nan_any[f] ? 1 : min(HIST_THREADS / 32, max(1, 255 / span))};
-}
 
 __device__ __forceinline__ void red_add_u32(uint32_t a, uint32_t v) {
   asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -465,19 +434,132 @@ __device__ __forceinline__ int fix_exponent(double S, double rows) {
   return max(-126, min(100, e));
 }
 __device__ __forceinline__ float exp2i(int e) { return __int_as_float((e + 127) << 23); }
+__device__ __forceinline__ double exp2d(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 
-struct FixRow {
-  uint32_t ghi, glo, hhi, hlo;
+// x * 2^e of a row as (hi, lo): two unsigned words whose sums are exact.
+__device__ __forceinline__ uint2 fix_pair(float x, float scale) {
+  const long long v = __float2ll_rn(x * scale);  // exact product: scale is a power of two
+  return make_uint2((uint32_t)(v >> 16), (uint32_t)v & 0xffffu);
+}
+
+// One item of the histogram kernel: rows [start, end) of segment (class k,
+// pair p), feature group g.
+struct HistItem {
+  int32_t k, p, g, start, end;
 };
-__device__ __forceinline__ FixRow fix_row(float g, float h, float sg, float sh) {
-  FixRow r;
-  const long long vg = __float2ll_rn(g * sg);  // exact product: sg is a power of two
-  r.ghi = (uint32_t)(vg >> 16);
-  r.glo = (uint32_t)vg & 0xffffu;
-  const long long vh = __float2ll_rn(h * sh);
-  r.hhi = (uint32_t)(vh >> 16);
-  r.hlo = (uint32_t)vh & 0xffffu;
-  return r;
+
+// A row's slice of a feature group: W4 words, in order.
+template <int W4>
+__device__ __forceinline__ void load_slice(uint32_t (&w)[W4], const uint8_t* src) {
+  if constexpr (W4 == 8) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(src)), b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+    w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+  } else if constexpr (W4 == 4) {
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(src));
+    w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+  } else if constexpr (W4 == 2) {
+    const uint2 a = __ldg(reinterpret_cast<const uint2*>(src));
+    w[0] = a.x; w[1] = a.y;
+  } else {
+    w[0] = __ldg(reinterpret_cast<const uint32_t*>(src));
+  }
+}
+
+// The updates of rows [start, end) of one item by the whole block: every warp
+// takes 32-row batches (warp w: w, w + warps, ...), lane l row l of a batch.
+// Row ids of gathered rows are loaded two batches ahead, the rows' slices
+// and (grad, hess) one batch ahead, all in registers.
+//
+// Lane l updates the 4 * W4 columns of its own row in an order rotated by its
+// index: word (j + l / 4) % W4, byte (i + l) % 4 in step (j, i), in copy
+// l / (4 W4) of the group's columns, so that the 32 lanes of every step hit 32
+// different banks; the rotation of the words is a barrel shift of selects.
+//
+// What bounds it: the shared-memory pipe.  32-bit `red.shared.add` with 32
+// different banks per instruction issues at one warp instruction per clock
+// and SM (measured: 31 lanes / clk / SM at 255, 32 and 4 bins), and a slice
+// of 32 bytes per row costs 8 wavefronts per 32 rows, so four atomics per
+// pair allow 7.5 pairs / clk / SM.  With a row per lane nothing else of the
+// loop needs that pipe; with four rows per step and eight lanes per row (each
+// converting the row again, bounds and padding tested per update) the loop
+// took 110 instructions and 21 wavefronts per 128 pairs.  Root level of 2.5M
+// rows x 200 features: 518 -> 372 us (5.0 pairs / clk / SM over the launch);
+// 1M x 50, ten classes, all levels: 2098 -> 1473 us.
+template <bool CNT, int W4>
+__device__ __forceinline__ void hist_rows(uint32_t hbase, int start, int end, bool gathered,
+                                          const uint32_t* __restrict__ rows, const float2* __restrict__ gh,
+                                          const uint8_t* __restrict__ tile, float sg, float sh) {
+  constexpr int B = HIST_BATCH, NW = HIST_THREADS / 32;
+  constexpr uint32_t FB = 4 * HistShape::W;  // bytes between two fields of a slot
+  const uint32_t lane = threadIdx.x & 31;
+  const int nb = (end - start + B - 1) / B;
+  uint32_t sel[4], off[4];  // step i's byte-permute selector (byte to bits 8..15) and column offset
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t b = ((uint32_t)i + lane) & 3u;
+    sel[i] = 0x4404u | (b << 4);
+    off[i] = 4u * b;
+  }
+  const uint32_t lane_base = hbase + 4u * (lane / (4 * W4)) * (4 * W4);
+  uint32_t rid = 0, nxt[W4];
+  float2 vn = make_float2(0.0f, 0.0f);
+  auto fetch_id = [&](int bi) {
+    const int r = start + bi * B + (int)lane;
+    if (r < end) rid = gathered ? __ldg(rows + r) : (uint32_t)r;
+  };
+  // rows past the item's end keep bins and (grad, hess) of an earlier row or
+  // zeros: they are masked where the batch is counted
+  auto fetch_row = [&](int bi) {
+    const int r = start + bi * B + (int)lane;
+    if (r < end) {
+      load_slice<W4>(nxt, tile + (size_t)rid * (4 * W4));
+      vn = gh[r];
+    }
+  };
+#pragma unroll
+  for (int j = 0; j < W4; ++j) nxt[j] = 0u;
+  int bi = (int)(threadIdx.x >> 5);
+  fetch_id(bi);
+  fetch_row(bi);
+  fetch_id(bi + NW);
+  for (; bi < nb; bi += NW) {
+    uint32_t w[W4];
+    const bool in = start + bi * B + (int)lane < end;
+    {
+      // rotate left by lane / 4 words
+      uint32_t t[W4];
+#pragma unroll
+      for (int j = 0; j < W4; ++j) w[j] = nxt[j];
+#pragma unroll
+      for (int m = 1; m < W4; m <<= 1) {
+        const bool rot = (lane >> 2) & (uint32_t)m;
+#pragma unroll
+        for (int j = 0; j < W4; ++j) t[j] = rot ? w[(j + m) % W4] : w[j];
+#pragma unroll
+        for (int j = 0; j < W4; ++j) w[j] = t[j];
+      }
+    }
+    const uint2 fg = fix_pair(vn.x, sg);
+    const uint2 fh = CNT ? make_uint2(1u, 0u) : fix_pair(vn.y, sh);
+    fetch_row(bi + NW);      // the next batch's rows and the ids of the batch after
+    fetch_id(bi + 2 * NW);   // arrive behind this batch's updates
+    if (in) {
+#pragma unroll
+      for (int j = 0; j < W4; ++j) {
+        const uint32_t base = lane_base + 16u * (((uint32_t)j + (lane >> 2)) & (W4 - 1));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          // __byte_perm gives bin * 256; a slot is 512 bytes
+          const uint32_t a = base + off[i] + 2u * __byte_perm(w[j], 0u, sel[i]);
+          red_add_u32(a, fg.x);
+          red_add_u32(a + FB, fg.y);
+          red_add_u32(a + 2 * FB, fh.x);
+          if (!CNT) red_add_u32(a + 3 * FB, fh.y);
+        }
+      }
+    }
+  }
 }
 
 // Persistent blocks (one per SM) over work items; an item is one chunk of one
@@ -487,52 +569,33 @@ __device__ __forceinline__ FixRow fix_row(float g, float h, float sg, float sh) 
 // (grad, hess) to every group.
 //
 // An item starts with a pass over its rows' (grad, hess) (contiguous in list
-// order) for the sums that fix its scales.  Then every warp runs its own copy
-// pipeline: lane l stages row l of a 32-row batch (its 32-byte group slice
-// from the feature-group tiles, and its (grad, hess)) by cp.async into the
-// warp's private buffers, one batch ahead of the updates, with the row ids of
-// gathered rows fetched a further batch ahead; no block barrier is taken
-// until the item is done.  The item ends by adding its exact sums, converted
-// to FP64, to the segment's FP64 accumulator in global memory.
+// order) for the sums that fix its scales; then the warps count its rows
+// (hist_rows, no block barrier until the item is done); it ends by adding its
+// exact sums, converted to FP64, to the segment's FP64 accumulator in global
+// memory.
 //
 // Shared histogram layout: column fastest, so a column always hits the same
-// bank: uint32 hist[(4 * slot + field) * 32 + column].  A wide group is
-// updated four rows at a time: lane (r = l/8, c = l%8) loads the 4 bins of
-// columns 4c..4c+3 of row r of the quad as one word and, in step s, updates
-// column 4c + (s + r) % 4, so the 32 lanes of every step hit 32 different
-// banks.  A group of at most 16 features is packed: with p2 = next power of
-// two >= its width, the 32 columns hold 32/p2 private copies and one warp
-// instruction updates 32/p2 rows; the copies are summed when the item ends.
-// Columns past a group's width (padding bytes, all bin 0: one hot address)
-// are not updated.  Each lane keeps the shared address of (its warp's copy of)
-// every column it updates, so an update is a byte permute, an add and the
-// integer atomics.
+// bank: uint32 hist[(4 * slot + field) * 32 + bank].  A group of w bytes per
+// row (w = 32, 16, 8, 4) keeps 32 / w private copies of its columns in the 32
+// banks, summed when the item ends.  Columns past a group's width (padding,
+// always bin 0) are updated like the others and never read.
 template <bool CNT>
 __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, int d) {
   using S_ = HistShape;
-  constexpr int W = S_::W, S = S_::S, B = HIST_BATCH;
-  constexpr uint32_t SLOT_BYTES = 4 * S_::FIELDS * W;   // 512: the 4 fields of one slot
-  constexpr uint32_t FB = 4 * W;                         // bytes between two fields of a slot
+  constexpr int W = S_::W, NW = HIST_THREADS / 32;
   extern __shared__ __align__(16) unsigned char smraw[];
   uint32_t* hist = reinterpret_cast<uint32_t*>(smraw);
   const uint32_t hbase = (uint32_t)__cvta_generic_to_shared(hist);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-  uint8_t* w_bins = smraw + S_::hist_bytes + (size_t)warp * S_::warp_bytes;        // [S][B][W]
-  float2* w_gh = reinterpret_cast<float2*>(w_bins + (size_t)S * B * W);            // [S][B]
-  __shared__ double s_sum[2][HIST_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  __shared__ double s_sum[2][NW];
+  __shared__ int s_next;
+  __shared__ HistItem s_item;
   const int P2 = pairs_at(d);
   const int nseg = c.K * P2;
   const int n_items = P.cum[nseg];
-  const int R = *P.rchunk;
   const int Pmax = 1 << (c.D - 1);
-  // quad mapping of this lane: row qr of a quad, columns 4*c4 .. 4*c4+3;
-  // byte-permute selectors that move byte (s + qr) % 4 of the word to bits 8..15
-  const int qr = lane >> 3, c4 = lane & 7;
-  uint32_t sel[4];
-#pragma unroll
-  for (int s = 0; s < 4; ++s) sel[s] = 0x4404u | ((uint32_t)((s + qr) & 3) << 4);
-  for (int q = threadIdx.x; q < kSlots * S_::FIELDS * W; q += blockDim.x) hist[q] = 0u;
-  __syncthreads();
+  if ((int)blockIdx.x >= n_items) return;  // the first item by index, the others from the counter
+  const int R = *P.rchunk;
   // Items are claimed from a counter (blocks that drew cheap items take
   // more), the next one while the current one runs.  Item ci*G + g is chunk
   // ci (over all segments) of group g; a narrow last group costs a fraction
@@ -544,232 +607,105 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     if (gw == c.G || cl >= n_items) return cl;
     return cl < n_chunks * gw ? (cl / gw) * c.G + cl % gw : (cl - n_chunks * gw) * c.G + gw;
   };
-  __shared__ int s_item[2];
-  if (threadIdx.x == 0) s_item[0] = claim_to_item(atomicAdd(P.hist_ctr, 1));
+  // The one thread whose segment holds the item publishes it: one load for
+  // every thread instead of a search with a load per step.
+  auto decode = [&](int it) {
+    for (int q = threadIdx.x; q < nseg; q += HIST_THREADS) {
+      const int c0 = P.cum[q];
+      if (c0 <= it && it < P.cum[q + 1]) {
+        const int ch = (it - c0) / c.G;
+        const int k = q / P2, p = q - k * P2;
+        // the segment's ceil(len / R) chunks have equal sizes (within one row)
+        const int s0 = d == 0 ? 0 : P.seg_start[k * Pmax + p];
+        const int sl = d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
+        const int nch = (sl + R - 1) / R;
+        s_item = HistItem{k, p, (it - c0) - ch * c.G, s0 + (int)((long long)sl * ch / nch),
+                          s0 + (int)((long long)sl * (ch + 1) / nch)};
+      }
+    }
+  };
+  decode(claim_to_item(blockIdx.x));
+  {
+    uint4* z = reinterpret_cast<uint4*>(hist);
+    for (int q = threadIdx.x; q < kSlots * S_::FIELDS * W / 4; q += HIST_THREADS) z[q] = make_uint4(0u, 0u, 0u, 0u);
+  }
   __syncthreads();
-  int item = s_item[0];
-  for (int it = 1; item < n_items; ++it) {
-    if (threadIdx.x == 0) s_item[it & 1] = claim_to_item(atomicAdd(P.hist_ctr, 1));
-    const int seg = find_seg(P.cum, nseg, item);
-    const int local = item - P.cum[seg];
-    const int ch_idx = local / c.G;
-    const int g = local - ch_idx * c.G;
-    const int k = seg / P2, p = seg - k * P2;
+  for (;;) {
+    const int k = s_item.k, p = s_item.p, g = s_item.g, start = s_item.start, end = s_item.end;
+    if (threadIdx.x == 0) s_next = claim_to_item(atomicAdd(P.hist_ctr, 1));
     const int g0 = g * W;
     const int gsize = min(W, (int)c.f - g0);
-    const int p2 = gsize <= 1 ? 1 : (gsize <= 2 ? 2 : (gsize <= 4 ? 4 : (gsize <= 8 ? 8 : (gsize <= 16 ? 16 : 32))));
-    const bool narrow = p2 <= 16;
-    // the segment's ceil(len / R) chunks have equal sizes (within one row)
-    const int s0 = d == 0 ? 0 : P.seg_start[k * Pmax + p];
-    const int sl = d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
-    const int nch = (sl + R - 1) / R;
-    const int start = s0 + (int)((long long)sl * ch_idx / nch);
-    const int end = s0 + (int)((long long)sl * (ch_idx + 1) / nch);
+    const uint32_t wid = (uint32_t)g + 1 == c.groups ? c.wlast : 32u;  // bytes per row of the group
     const uint32_t* rows = P.rows + (size_t)k * c.n;
     // (grad, hess) in list order: the root's rows are 0..n-1, a smaller
     // child's were copied next to its row ids by the scatter kernel
     const float2* gh = (d == 0 ? P.gh : P.cgh) + (size_t)k * c.n;
-    // the item's scales: FP64 sums of |grad| and |hess| over its rows (every
-    // thread a fixed stride, the warps in a fixed order)
+    // the item's scales: FP64 sums of |grad| and |hess| over its rows
     int eg, eh;
     float sg, sh;
     {
       double sa = 0.0, sb = 0.0;
 #pragma unroll 4
-      for (int r = start + threadIdx.x; r < end; r += blockDim.x) {
+      for (int r = start + threadIdx.x; r < end; r += HIST_THREADS) {
         const float2 v = gh[r];
         sa += (double)fabsf(v.x);
-        sb += (double)fabsf(v.y);
+        if (!CNT) sb += (double)fabsf(v.y);
       }
       for (int o = 16; o; o >>= 1) {
         sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        sb += __shfl_xor_sync(0xffffffffu, sb, o);
+        if (!CNT) sb += __shfl_xor_sync(0xffffffffu, sb, o);
       }
       if (lane == 0) { s_sum[0][warp] = sa; s_sum[1][warp] = sb; }
       __syncthreads();
-      sa = 0.0;
-      sb = 0.0;
-      for (int w = 0; w < nwarps; ++w) { sa += s_sum[0][w]; sb += s_sum[1][w]; }
+      sa = s_sum[0][lane];
+      sb = s_sum[1][lane];
+      for (int o = 16; o; o >>= 1) {
+        sa += __shfl_xor_sync(0xffffffffu, sa, o);
+        if (!CNT) sb += __shfl_xor_sync(0xffffffffu, sb, o);
+      }
       eg = fix_exponent(sa, (double)(end - start));
       eh = CNT ? 0 : fix_exponent(sb, (double)(end - start));
       sg = exp2i(eg);
       sh = exp2i(eh);
     }
-    // shared address of this warp's copy of each column the lane updates;
-    // columns past the group's width are skipped (their padding bytes are
-    // all bin 0, a single hot address)
-    uint32_t ab[4];
-    uint32_t live = 0;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      const int col = 4 * c4 + ((s + qr) & 3);
-      const HistCol hc = hist_col(P, g0 + col, (int)c.f);
-      ab[s] = hbase + SLOT_BYTES * (uint32_t)((warp % hc.copies) * hc.span) + 4u * col;
-      if (col < gsize) live |= 1u << s;
-    }
-    // the two 16-byte pieces of a row's group slice in the feature-group
-    // tiles; the last group's narrower block copies only its width
-    const uint32_t gwid = (uint32_t)g + 1 == c.groups ? c.wlast : 32u;
     const uint8_t* tile = P.bins_t + (uint64_t)g * c.gstride;
-    const int nb = (end - start + B - 1) / B;   // batches in the item; warp w takes w, w+nwarps, ...
-    uint32_t rid_next = 0;
-#define TC_FETCH_ID(bi)                                                                      \
-    {                                                                                        \
-      const int r_ = start + (bi) * B + lane;                                                \
-      rid_next = ((bi) < nb && r_ < end) ? (d == 0 ? (uint32_t)r_ : rows[r_]) : 0u;          \
-    }
-#define TC_ISSUE(bi, st_)                                                                    \
-    {                                                                                        \
-      if ((bi) < nb && start + (bi) * B + lane < end) {                                      \
-        uint8_t* dst_ = w_bins + ((size_t)(st_) * B + lane) * W;                             \
-        const uint8_t* src_ = tile + (size_t)rid_next * gwid;                                \
-        if (gwid == 32) {                                                                    \
-          cp_async16(dst_, src_);                                                            \
-          cp_async16(dst_ + 16, src_ + 16);                                                  \
-        } else if (gwid == 16) {                                                             \
-          cp_async16(dst_, src_);                                                            \
-        } else if (gwid == 8) {                                                              \
-          cp_async8(dst_, src_);                                                             \
-        } else {                                                                             \
-          cp_async4(dst_, src_);                                                             \
-        }                                                                                    \
-        cp_async8(w_gh + (st_) * B + lane, gh + start + (bi) * B + lane);                     \
-      }                                                                                      \
-      cp_async_commit();                                                                     \
-    }
-    int bi = warp;
-    TC_FETCH_ID(bi);
-    TC_ISSUE(bi, 0);
-    TC_FETCH_ID(bi + nwarps);
-    for (int t = 0; bi < nb; ++t, bi += nwarps) {
-      const int st = t & 1;
-      TC_ISSUE(bi + nwarps, st ^ 1);       // the next batch streams in while this one is counted
-      TC_FETCH_ID(bi + 2 * nwarps);        // row ids for the batch after, behind this batch's updates
-      cp_async_wait<1>();
-      __syncwarp();
-      const int nvalid = min(B, end - (start + bi * B));
-      const uint8_t* sb = w_bins + (size_t)st * B * W;
-      const float2* sv = w_gh + st * B;
-      if (!narrow) {
-        // the batch's bins and (grad, hess) go to registers first, so the
-        // loads are not ordered behind the updates (they share the memory space)
-        const uint32_t* sw = reinterpret_cast<const uint32_t*>(sb);
-        uint32_t wd[B / 4];
-        float vx[B / 4], vy[B / 4];
-#pragma unroll
-        for (int qd = 0; qd < B / 4; ++qd) {
-          const int row = 4 * qd + qr;
-          const float2 v = sv[row];
-          vx[qd] = v.x;
-          vy[qd] = v.y;
-          wd[qd] = sw[row * (W / 4) + c4];
-        }
-#pragma unroll
-        for (int qd = 0; qd < B / 4; ++qd) {
-          if (4 * qd + qr < nvalid) {
-            const FixRow fr = fix_row(vx[qd], vy[qd], sg, sh);
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-              // __byte_perm gives bin * 256; a slot is SLOT_BYTES = 512 bytes
-              const uint32_t a = ab[s] + 2u * __byte_perm(wd[qd], 0u, sel[s]);
-              if (live & (1u << s)) {
-                red_add_u32(a, fr.ghi);
-                red_add_u32(a + FB, fr.glo);
-                if (CNT) {
-                  red_add_u32(a + 2 * FB, 1u);
-                } else {
-                  red_add_u32(a + 2 * FB, fr.hhi);
-                  red_add_u32(a + 3 * FB, fr.hlo);
-                }
-              }
-            }
-          }
-        }
-      } else {
-        // packed narrow group: lane (copy, column) of rows i .. i + 32/p2 - 1,
-        // four instructions' rows loaded ahead of their updates
-        const int rpi = 32 / p2;
-        const int my_row = lane / p2, my_col = lane - my_row * p2;
-        const HistCol hc = hist_col(P, g0 + my_col, (int)c.f);
-        const uint32_t abn = hbase + SLOT_BYTES * (uint32_t)((warp % hc.copies) * hc.span) + 4u * lane;
-        for (int i0 = 0; i0 < B; i0 += 4 * rpi) {
-          uint32_t bb[4];
-          float gx[4], gy[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int row = min(i0 + u * rpi + my_row, B - 1);
-            const float2 v = sv[row];
-            gx[u] = v.x;
-            gy[u] = v.y;
-            bb[u] = sb[row * W + my_col];
-          }
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (i0 + u * rpi + my_row < nvalid && my_col < gsize) {
-              const FixRow fr = fix_row(gx[u], gy[u], sg, sh);
-              const uint32_t a = abn + SLOT_BYTES * bb[u];
-              red_add_u32(a, fr.ghi);
-              red_add_u32(a + FB, fr.glo);
-              if (CNT) {
-                red_add_u32(a + 2 * FB, 1u);
-              } else {
-                red_add_u32(a + 2 * FB, fr.hhi);
-                red_add_u32(a + 3 * FB, fr.hlo);
-              }
-            }
-          }
-        }
-      }
-      __syncwarp();
-    }
-#undef TC_FETCH_ID
-#undef TC_ISSUE
-    cp_async_wait<0>();
+    if (wid == 32) hist_rows<CNT, 8>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
+    else if (wid == 16) hist_rows<CNT, 4>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
+    else if (wid == 8) hist_rows<CNT, 2>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
+    else hist_rows<CNT, 1>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
     __syncthreads();
-    // add the item's exact sums (copies summed as integers), converted to
-    // FP64, to the segment's FP64 accumulator (zero sums are not sent), and
-    // clear the histogram for the next item; a thread clears exactly the
-    // slots it reads
-    double2* dst = P.acc + (((size_t)k * Pmax + p) * c.f + g0) * kSlots;
-    const int ncp = narrow ? 32 / p2 : 1;     // packed copies of a narrow group
-    // blockDim.x is a multiple of W: a thread's column is the same on every pass
-    const int col = threadIdx.x % W;
-    const HistCol fc = hist_col(P, g0 + col, (int)c.f);
-    for (int q = threadIdx.x; q < kSlots * W; q += blockDim.x) {
-      const int b = q / W;
-      long long G = 0, H = 0;
-      if (!narrow || col < p2) {
-        const int kc = b == kNanBin ? 1 : (b < fc.span ? fc.copies : 0);
-        for (int cc = 0; cc < kc; ++cc) {
-          const int slot = b == kNanBin ? kNanBin : cc * fc.span + b;
-          for (int cp = 0; cp < ncp; ++cp) {
-            uint32_t* o = hist + 4 * slot * W + cp * p2 * (narrow ? 1 : 0) + col;
-            G += (long long)(int32_t)o[0] * 65536 + (long long)o[W];
-            if (CNT) H += (long long)o[2 * W];
-            else H += (long long)(int32_t)o[2 * W] * 65536 + (long long)o[3 * W];
-            if (!narrow) {
-              o[0] = 0u;
-              o[W] = 0u;
-              o[2 * W] = 0u;
-              o[3 * W] = 0u;
-            }
-          }
+    const int next = s_next;
+    // add the item's exact sums, converted to FP64, to the segment's FP64
+    // accumulator (zero sums are not sent), and clear the histogram for the
+    // next item; a thread clears exactly the slots it reads.  Lane = bank: the
+    // copies of a narrow group are summed by shuffles.
+    {
+      double2* dst = P.acc + (((size_t)k * Pmax + p) * c.f + g0) * kSlots;
+      const int col = lane & (int)(wid - 1);
+      const double ug = exp2d(-eg), uh = CNT ? (double)c.hconst : exp2d(-eh);
+#pragma unroll 4
+      for (int b = warp; b < kSlots; b += NW) {
+        uint32_t* o = hist + 4 * b * W + lane;
+        long long G = (long long)(int32_t)o[0] * 65536 + (long long)o[W];
+        long long H = CNT ? (long long)o[2 * W] : (long long)(int32_t)o[2 * W] * 65536 + (long long)o[3 * W];
+        o[0] = 0u;
+        o[W] = 0u;
+        o[2 * W] = 0u;
+        if (!CNT) o[3 * W] = 0u;
+        for (uint32_t m = wid; m < 32; m <<= 1) {
+          G += __shfl_xor_sync(0xffffffffu, G, m);
+          H += __shfl_xor_sync(0xffffffffu, H, m);
+        }
+        if (lane < gsize) {
+          double2* ad = dst + (size_t)col * kSlots + b;
+          if (G) atomicAdd(&ad->x, (double)G * ug);
+          if (H) atomicAdd(&ad->y, (double)H * uh);
         }
       }
-      if (col < gsize) {
-        const double gd = ldexp((double)G, -eg);
-        const double hd = CNT ? (double)c.hconst * (double)H : ldexp((double)H, -eh);
-        double2* o = dst + (size_t)col * kSlots + b;
-        if (gd != 0.0) atomicAdd(&o->x, gd);
-        if (hd != 0.0) atomicAdd(&o->y, hd);
-      }
     }
-    if (narrow) {
-      __syncthreads();
-      for (int q = threadIdx.x; q < kSlots * S_::FIELDS * 32; q += blockDim.x) hist[q] = 0u;
-    }
+    if (next >= n_items) return;
+    decode(next);
     __syncthreads();
-    item = s_item[it & 1];
   }
 }
 
@@ -1397,7 +1333,7 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   }
   if (tid == 0) {
     P.cum[nsg] = min(s_carry, c.item_cap);
-    *P.hist_ctr = 0;
+    *P.hist_ctr = c.hist_grid;  // items 0 .. grid - 1 belong to the blocks by index
     if (d < 16) {
       P.lvl_rows[d] = (uint64_t)s_rows;
       P.lvl_nodes[d] = (uint32_t)s_nodes;
