@@ -59,6 +59,8 @@ constexpr int SCAN_WARPS = 8;     // warps per scan block
 constexpr int SCAN_NODES = 16;    // nodes per scan block (2 per warp; measured: 32 per block 4% slower on 1M x 100 depth 8)
 static_assert(SCAN_WARPS * 32 == 256, "a scan block also runs the 256-thread pick");
 constexpr int PLAN_THREADS = 1024;
+constexpr int kHistItemRows = 2048;   // an item's fixed cost in rows of a full group
+constexpr int kHistRowsSplit = 4096;  // chunks are not cut below this to make more waves
 constexpr int kHistRowsMax = 65535;  // rows of a histogram item: its 16-bit low fields sum without overflow
 constexpr int VALID_BLOCKS = 296;  // blocks of the validation kernel (fixed: its partial sums have a fixed order)
 
@@ -102,8 +104,8 @@ struct DevCfg {
   int32_t msl;
   float lr, lam, l1, mcw, msg, mds, gamma, alpha;
   int32_t G, W;                  // feature groups, group width (32*J)
+  int32_t gwide, row_words;      // groups wider than 16 features; 4-byte words of a row over all groups
   int32_t PB;                    // partition blocks
-  int32_t item_cap;              // capacity of the partial buffer (items)
   int32_t n_scan_groups_max;
   int32_t hist_grid;             // persistent histogram blocks
   int32_t target_items;          // work items aimed for per histogram launch
@@ -486,10 +488,12 @@ __device__ __forceinline__ void load_slice(uint32_t (&w)[W4], const uint8_t* src
 // took 110 instructions and 21 wavefronts per 128 pairs.  Root level of 2.5M
 // rows x 200 features: 518 -> 372 us (5.0 pairs / clk / SM over the launch);
 // 1M x 50, ten classes, all levels: 2098 -> 1473 us.
-template <bool CNT, int W4>
+// `scales` (the pass that fixes the item's scales, with the block's barrier)
+// runs behind the first loads.
+template <bool CNT, int W4, class Scales>
 __device__ __forceinline__ void hist_rows(uint32_t hbase, int start, int end, bool gathered,
                                           const uint32_t* __restrict__ rows, const float2* __restrict__ gh,
-                                          const uint8_t* __restrict__ tile, float sg, float sh) {
+                                          const uint8_t* __restrict__ tile, Scales scales) {
   constexpr int B = HIST_BATCH, NW = HIST_THREADS / 32;
   constexpr uint32_t FB = 4 * HistShape::W;  // bytes between two fields of a slot
   const uint32_t lane = threadIdx.x & 31;
@@ -523,6 +527,8 @@ __device__ __forceinline__ void hist_rows(uint32_t hbase, int start, int end, bo
   fetch_id(bi);
   fetch_row(bi);
   fetch_id(bi + NW);
+  float sg, sh;
+  scales(sg, sh);
   for (; bi < nb; bi += NW) {
     uint32_t w[W4];
     const bool in = start + bi * B + (int)lane < end;
@@ -589,7 +595,7 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ double s_sum[2][NW];
   __shared__ int s_next;
-  __shared__ HistItem s_item;
+  __shared__ HistItem s_item[2];
   const int P2 = pairs_at(d);
   const int nseg = c.K * P2;
   const int n_items = P.cum[nseg];
@@ -602,14 +608,14 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
   // of a wide one, so its items are handed out after all the wide ones and
   // fill the gaps at the end.
   const int n_chunks = n_items / c.G;
-  const int gw = (c.G > 1 && (int)c.f - (c.G - 1) * W <= 16) ? c.G - 1 : c.G;  // wide groups
+  const int gw = c.gwide;
   auto claim_to_item = [&](int cl) {
-    if (gw == c.G || cl >= n_items) return cl;
+    if (gw == 0 || gw == c.G || cl >= n_items) return cl;
     return cl < n_chunks * gw ? (cl / gw) * c.G + cl % gw : (cl - n_chunks * gw) * c.G + gw;
   };
   // The one thread whose segment holds the item publishes it: one load for
   // every thread instead of a search with a load per step.
-  auto decode = [&](int it) {
+  auto decode = [&](int it, int ph) {
     for (int q = threadIdx.x; q < nseg; q += HIST_THREADS) {
       const int c0 = P.cum[q];
       if (c0 <= it && it < P.cum[q + 1]) {
@@ -619,19 +625,19 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
         const int s0 = d == 0 ? 0 : P.seg_start[k * Pmax + p];
         const int sl = d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
         const int nch = (sl + R - 1) / R;
-        s_item = HistItem{k, p, (it - c0) - ch * c.G, s0 + (int)((long long)sl * ch / nch),
-                          s0 + (int)((long long)sl * (ch + 1) / nch)};
+        s_item[ph] = HistItem{k, p, (it - c0) - ch * c.G, s0 + (int)((long long)sl * ch / nch),
+                              s0 + (int)((long long)sl * (ch + 1) / nch)};
       }
     }
   };
-  decode(claim_to_item(blockIdx.x));
+  decode(claim_to_item(blockIdx.x), 0);
   {
     uint4* z = reinterpret_cast<uint4*>(hist);
     for (int q = threadIdx.x; q < kSlots * S_::FIELDS * W / 4; q += HIST_THREADS) z[q] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
-  for (;;) {
-    const int k = s_item.k, p = s_item.p, g = s_item.g, start = s_item.start, end = s_item.end;
+  for (int ph = 0;; ph ^= 1) {
+    const int k = s_item[ph].k, p = s_item[ph].p, g = s_item[ph].g, start = s_item[ph].start, end = s_item[ph].end;
     if (threadIdx.x == 0) s_next = claim_to_item(atomicAdd(P.hist_ctr, 1));
     const int g0 = g * W;
     const int gsize = min(W, (int)c.f - g0);
@@ -641,9 +647,8 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     // child's were copied next to its row ids by the scatter kernel
     const float2* gh = (d == 0 ? P.gh : P.cgh) + (size_t)k * c.n;
     // the item's scales: FP64 sums of |grad| and |hess| over its rows
-    int eg, eh;
-    float sg, sh;
-    {
+    int eg = 0, eh = 0;
+    auto scales = [&](float& sg, float& sh) {
       double sa = 0.0, sb = 0.0;
 #pragma unroll 4
       for (int r = start + threadIdx.x; r < end; r += HIST_THREADS) {
@@ -667,14 +672,15 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
       eh = CNT ? 0 : fix_exponent(sb, (double)(end - start));
       sg = exp2i(eg);
       sh = exp2i(eh);
-    }
+    };
     const uint8_t* tile = P.bins_t + (uint64_t)g * c.gstride;
-    if (wid == 32) hist_rows<CNT, 8>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
-    else if (wid == 16) hist_rows<CNT, 4>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
-    else if (wid == 8) hist_rows<CNT, 2>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
-    else hist_rows<CNT, 1>(hbase, start, end, d > 0, rows, gh, tile, sg, sh);
+    if (wid == 32) hist_rows<CNT, 8>(hbase, start, end, d > 0, rows, gh, tile, scales);
+    else if (wid == 16) hist_rows<CNT, 4>(hbase, start, end, d > 0, rows, gh, tile, scales);
+    else if (wid == 8) hist_rows<CNT, 2>(hbase, start, end, d > 0, rows, gh, tile, scales);
+    else hist_rows<CNT, 1>(hbase, start, end, d > 0, rows, gh, tile, scales);
     __syncthreads();
     const int next = s_next;
+    if (next < n_items) decode(next, ph ^ 1);  // its loads run behind the flush
     // add the item's exact sums, converted to FP64, to the segment's FP64
     // accumulator (zero sums are not sent), and clear the histogram for the
     // next item; a thread clears exactly the slots it reads.  Lane = bank: the
@@ -704,7 +710,6 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
       }
     }
     if (next >= n_items) return;
-    decode(next);
     __syncthreads();
   }
 }
@@ -1179,6 +1184,7 @@ constexpr int kPlanSegs = 4096;  // (class, pair) segment lengths the plan keeps
 __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int d) {
   __shared__ long long s_rows;
   __shared__ int s_nodes;
+  __shared__ int s_live;            // non-empty segments of the level
   __shared__ int s_warp[32];
   __shared__ int s_carry;
   __shared__ int s_len[kPlanSegs];  // [class][pair] rows of level d (0: the class grows no more)
@@ -1188,7 +1194,7 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   const int np2 = pairs_at(d);
   const int nsg = c.K * np2;
   const bool cached = nsg <= kPlanSegs;
-  if (tid == 0) { s_rows = 0; s_nodes = 0; }
+  if (tid == 0) { s_rows = 0; s_nodes = 0; s_live = 0; }
   __syncthreads();
   // Per class, one warp each (classes w, w + warps, ...): no block barriers.
   for (int k = warp; k < c.K; k += nwarps) {
@@ -1243,7 +1249,7 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     }
     if (!done) {
       // segment starts (exclusive scan over the pairs' lengths), 32 at a time
-      int carry = 0;
+      int carry = 0, live = 0;
       for (int base = 0; base < np2; base += 32) {
         const int p = base + lane;
         const int len = p < np2 ? (d == 0 ? (int)c.n : P.seg_len[k * Pmax + p]) : 0;
@@ -1257,8 +1263,10 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
           if (cached) s_len[k * np2 + p] = len;
         }
         carry += __shfl_sync(0xffffffffu, x, 31);
+        live += __popc(__ballot_sync(0xffffffffu, len > 0));
       }
       if (lane == 0) {
+        atomicAdd(&s_live, live);
         atomicAdd(reinterpret_cast<unsigned long long*>(&s_rows), (unsigned long long)carry);
         atomicAdd(&s_nodes, np2);
       }
@@ -1279,17 +1287,31 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     if (P.cs[k].done) return 0;
     return d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
   };
-  // Rows per chunk for this level: the smallest R (from the even split up)
-  // for which the level has at most target_items items.  Every group counts,
-  // the narrow last one too: measured, items that all run in one wave beat
-  // a second wave of cheap narrow items after the wide ones.
+  // Rows per chunk R for this level.  `load` is a block's even share of the
+  // level in rows of a full group, an item's fixed cost (claim, scales,
+  // flush: kHistItemRows rows) included.  One wave: R = load.  More waves (the
+  // autotuner's choice) even out the blocks on large levels, but no chunk is
+  // cut below kHistRowsSplit rows for that: on levels of many short segments
+  // the items' fixed costs would be most of the level (2.5M x 200, depth 8,
+  // level 7, 154k rows in 64 segments: 97 us at 512-row chunks, 67 here; level
+  // 6, 31k rows: 46 and 35).  R then grows until the items fit whole waves; in
+  // one wave every group counts, the narrow ones too (21 chunks of 7 groups in
+  // one wave: 135 us on level 1, 829k rows; 23 chunks whose narrow items run
+  // after the wide ones: 157).  Segments that do not fill a wave between them
+  // add an item each.
   __shared__ int s_R;
   __shared__ long long s_cnt;
-  const int gw = c.G;
-  if (tid == 0) {
-    int R = c.rows_fixed;
-    if (R <= 0) R = (int)max((long long)c.rows_min, (s_rows * gw + c.target_items - 1) / c.target_items);
-    s_R = min(R, kHistRowsMax);
+  const int waves = max(1, c.target_items / c.hist_grid);
+  const int gw = waves == 1 || c.gwide == 0 ? c.G : c.gwide;
+  const long long load = (s_rows * c.row_words / 8 + (long long)s_live * c.G * kHistItemRows) / c.hist_grid + 1;
+  long long allowed = 0;
+  {
+    long long R = c.rows_fixed;
+    if (R <= 0) R = max((long long)c.rows_min, min(load, max(load / waves, (long long)kHistRowsSplit)));
+    R = min(R, (long long)kHistRowsMax);
+    allowed = max(1LL, (load + R / 2) / R) * c.hist_grid;
+    if (2LL * s_live * gw > allowed) allowed += (long long)s_live * gw;
+    if (tid == 0) s_R = (int)R;
   }
   __syncthreads();
   for (int round = 0; c.rows_fixed <= 0 && round < 16; ++round) {
@@ -1303,8 +1325,8 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     __syncthreads();
     const long long items = s_cnt * gw;
     __syncthreads();
-    if (items <= c.target_items) break;
-    if (tid == 0) s_R = (int)min((long long)kHistRowsMax, (long long)Rt * items / c.target_items + 1);
+    if (items <= allowed || Rt >= kHistRowsMax) break;
+    if (tid == 0) s_R = (int)min((long long)kHistRowsMax, (long long)Rt * items / allowed + 1);
     __syncthreads();
   }
   if (tid == 0) {
@@ -1326,13 +1348,13 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     __syncthreads();
     int before = s_carry;
     for (int w = 0; w < warp; ++w) before += s_warp[w];
-    if (sgi < nsg) P.cum[sgi] = min(before + x - chunks, c.item_cap);
+    if (sgi < nsg) P.cum[sgi] = before + x - chunks;
     __syncthreads();
     if (tid == blockDim.x - 1) s_carry = before + x;
     __syncthreads();
   }
   if (tid == 0) {
-    P.cum[nsg] = min(s_carry, c.item_cap);
+    P.cum[nsg] = s_carry;
     *P.hist_ctr = c.hist_grid;  // items 0 .. grid - 1 belong to the blocks by index
     if (d < 16) {
       P.lvl_rows[d] = (uint64_t)s_rows;
@@ -1770,7 +1792,7 @@ tc_status tc_trainer::setup(int) {
 }
 
 // Feature-group width (32*J columns) and work items per histogram launch
-// (waves x resident histogram blocks); (re)sizes the partial buffer.
+// (waves x resident histogram blocks).
 tc_status tc_trainer::configure(int J_, int waves) {
   const uint32_t f = cfg.f;
   const int K = cfg.K, D = cfg.D;
@@ -1780,15 +1802,13 @@ tc_status tc_trainer::configure(int J_, int waves) {
   const int G = (int)((f + W - 1) / W);
   hist_grid = ctx->sm_count;  // one 1024-thread block per SM
   hist_waves = waves;
-  long long cap = (long long)waves * hist_grid + (long long)K * Pmax * G + 1;
-  if (cfg.rows_fixed) cap += (long long)K * G * ((cfg.n + cfg.rows_fixed - 1) / cfg.rows_fixed + 1);
-  cap += (long long)K * G * (cfg.n / kHistRowsMax + 1);  // chunks of at most kHistRowsMax rows
   cfg.G = G;
   cfg.W = W;
+  cfg.gwide = G - (cfg.wlast <= 16 ? 1 : 0);
+  cfg.row_words = 8 * (G - 1) + (int)cfg.wlast / 4;
   cfg.hist_grid = hist_grid;
   cfg.target_items = waves * hist_grid;
   cfg.rows_min = hist_rows_min;
-  cfg.item_cap = (int)cap;
 
   TC_TRY(cum.alloc(ctx, (size_t)K * Pmax * G + 1, "chunk counts"));
   ptr.cum = cum.p;
