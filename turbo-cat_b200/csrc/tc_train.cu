@@ -685,32 +685,44 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     __syncthreads();
     const int next = s_next;
     if (next < n_items) decode(next, ph ^ 1);  // its loads run behind the flush
-    // add the item's exact sums, converted to FP64, to the segment's FP64
-    // accumulator (zero sums are not sent), and clear the histogram for the
-    // next item; a thread clears exactly the slots it reads.  Lane = bank: the
-    // copies of a narrow group are summed by shuffles.
+    // The item's exact sums, converted to FP64, go to the segment's FP64
+    // accumulator (zero sums are not sent) and the histogram is cleared.  Two
+    // passes, since the sums lie column-fastest in shared memory and bin-fastest
+    // in global memory.  First lane = bank: a slot's four fields become its
+    // (grad, hess) doubles in place (32 columns x 16 bytes, the column's unit
+    // rotated by an exclusive or with the bin so that the second pass reads
+    // without conflicts); the copies of a narrow group are summed by shuffles.
     {
-      double2* dst = P.acc + (((size_t)k * Pmax + p) * c.f + g0) * kSlots;
-      const int col = lane & (int)(wid - 1);
       const double ug = exp2d(-eg), uh = CNT ? (double)c.hconst : exp2d(-eh);
-#pragma unroll 4
+#pragma unroll 2
       for (int b = warp; b < kSlots; b += NW) {
         uint32_t* o = hist + 4 * b * W + lane;
         long long G = (long long)(int32_t)o[0] * 65536 + (long long)o[W];
         long long H = CNT ? (long long)o[2 * W] : (long long)(int32_t)o[2 * W] * 65536 + (long long)o[3 * W];
-        o[0] = 0u;
-        o[W] = 0u;
-        o[2 * W] = 0u;
-        if (!CNT) o[3 * W] = 0u;
         for (uint32_t m = wid; m < 32; m <<= 1) {
           G += __shfl_xor_sync(0xffffffffu, G, m);
           H += __shfl_xor_sync(0xffffffffu, H, m);
         }
-        if (lane < gsize) {
-          double2* ad = dst + (size_t)col * kSlots + b;
-          if (G) atomicAdd(&ad->x, (double)G * ug);
-          if (H) atomicAdd(&ad->y, (double)H * uh);
-        }
+        __syncwarp();
+        double2* u = reinterpret_cast<double2*>(hist + 4 * b * W) + (lane ^ (b & 31));
+        *u = lane < gsize ? make_double2((double)G * ug, (double)H * uh) : make_double2(0.0, 0.0);
+      }
+    }
+    __syncthreads();
+    // Then a warp per column: 16 bins x (grad, hess), 256 contiguous bytes, per
+    // instruction.  What bounds the flush: L2 operations, one per 32-byte sector
+    // of an instruction; with a lane per column every lane's atomic was a sector
+    // of its own.  Histogram per iteration: 1M x 100 MSE 362 -> 313 us, 2.5M x
+    // 200 focal 806 -> 777 us, 1M x 50 ten classes 1382 -> 1320 us.
+    if (warp < gsize) {
+      double* dst = reinterpret_cast<double*>(P.acc + (((size_t)k * Pmax + p) * c.f + g0 + warp) * kSlots);
+#pragma unroll 4
+      for (int i = 0; i < kSlots / 16; ++i) {
+        const int b = 16 * i + (lane >> 1);
+        double* u = reinterpret_cast<double*>(hist + 4 * b * W) + 2 * (warp ^ (b & 31)) + (lane & 1);
+        const double v = *u;
+        *u = 0.0;
+        if (v != 0.0) atomicAdd(dst + 32 * i + lane, v);
       }
     }
     if (next >= n_items) return;
