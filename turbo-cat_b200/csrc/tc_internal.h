@@ -184,10 +184,12 @@ struct tc_model {
   // device copies used by the predict kernels
   DevBuf<uint2> d_splits;           // [T][D] (feature, threshold bits), padded to depth D
   DevBuf<float> d_leaves;           // [T][2^D] (weights folded in, padded trees' leaves spread)
-  DevBuf<uint2> d_bsplits;          // binned form: [T][D] (virtual feature's column, byte-wise 128 - k)
+  DevBuf<uint32_t> d_bsplits;       // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class
+  DevBuf<float> d_bleaves;          // binned form, several classes: leaves in the order of d_bsplits
   DevBuf<float> d_bord;             // binned form: borders of every virtual feature, Eytzinger order
   DevBuf<uint2> d_vdesc;            // binned form: (feature, border offset | search steps << 24)
   int n_virtual = 0, n_bord = 0;
+  int bin_stride = 0;               // bytes of a bin column: 256 or 128 rows (0: no binned form)
   // regular (depth-wise) trees of a model the reference trained with
   // mode="small" (served for prediction only; tc_predict.cu)
   bool regular = false;
@@ -230,7 +232,8 @@ struct ReqDesc {
 struct ModelDesc {
   const uint2* splits;   // float form
   const float* leaves;
-  const uint2* bsplits;  // binned form (nullptr: the model has none)
+  const uint32_t* bsplits;  // binned form, class by class (nullptr: the model has none)
+  const float* bleaves;     // its leaves, in the same order
   const float* bord;
   const uint2* vdesc;
   int32_t n_trees;
@@ -240,22 +243,27 @@ struct ModelDesc {
   float base;
   int32_t n_virtual;
   int32_t n_bord;
-  int32_t pad;
+  int32_t bin_stride;
 };
-// Coalesced prediction over a request table: job j covers tiles
-// [tile_begin[j], tile_begin[j+1]) of PRED_ROWS rows each.
 // Launch shape of a batch: dynamic shared memory and stage sizes that fit
-// every model of the batch.
+// every model of the batch, and the largest tile they allow.
 struct PredictPlan {
   size_t smem;
   int leaf_stage;   // floats of one leaf stage
-  int split_stage;  // splits of one split stage
+  int split_stage;  // 8-byte units of one split stage
+  int chunk;        // trees per chunk at most
+  int stage_rows;   // rows staged at a time (binned walk)
+  int max_tile;     // 256 rows, or 128
 };
 PredictPlan predict_plan(const tc_model* const* models, int n);
+// Rows of a launch's tiles, from its count of 128-row tiles.
+int predict_tile_rows(const tc_ctx* ctx, const PredictPlan& plan, uint64_t tiles_of_half);
+uint32_t predict_tiles(uint32_t n, int tile_rows);
+// Coalesced prediction over a request table: job j covers tiles
+// [tile_begin[j], tile_begin[j+1]) of tile_rows rows each.
 tc_status predict_batched(tc_ctx* ctx, const ModelDesc* d_models, const ReqDesc* d_reqs, int n_reqs,
-                          const uint32_t* d_tile_begin, uint32_t n_tiles, const PredictPlan& plan,
+                          const uint32_t* d_tile_begin, int tile_rows, uint32_t n_tiles, const PredictPlan& plan,
                           cudaStream_t stream);
-uint32_t predict_tiles(uint32_t n);
 ModelDesc model_desc(const tc_model* m);
 
 }  // namespace tc

@@ -12,35 +12,46 @@
 // Device model.  Every tree is padded to the model's depth D (a padding
 // split's bit is always 0; leaf l of a tree of depth d moves to l << (D - d))
 // and the tree weight is folded into the leaves.  Float form: splits are
-// (feature, threshold bits), the padding threshold NaN.  Binned form
-// (single-output models): per feature, the model's distinct thresholds sorted
-// and cut into virtual features of at most 127 borders; a row's bin on a
-// virtual feature is the number of its borders <= x (NaN: 0), and
-// x >= threshold  <=>  bin >= k, k the threshold's rank in its virtual
-// feature + 1 (the same float compare, so the leaf index is exact).  The
-// binarisation restates Dataset::apply_bins (src/core/dataset.cpp:346-379)
-// with the model's borders in place of the training edges.
+// (feature, threshold bits), the padding threshold NaN.  Binned form: per
+// feature, the model's distinct thresholds sorted and cut into virtual
+// features of at most 127 borders; a row's bin on a virtual feature is the
+// number of its borders <= x (NaN: 0), and x >= threshold  <=>  bin >= k, k the
+// threshold's rank in its virtual feature + 1 (the same float compare, so the
+// leaf index is exact).  The binarisation restates Dataset::apply_bins
+// (src/core/dataset.cpp:346-379) with the model's borders in place of the
+// training edges.
 //
-// Kernel layout: a block owns a tile of 128 rows of one job (one request of a
-// coalesced serving batch, or the whole input of a single call); the tile's
-// rows are staged row-major in shared memory (odd row stride: threads reading
-// the same feature of different rows hit different banks).  Trees stream
-// through shared memory in chunks (splits and leaves, two chunks in flight:
-// cp.async, the next chunk lands while the current one is walked).
+// Kernel layout: a block of 16 warps owns a tile of 256 rows (128 when the
+// launch has too few rows to fill the device) of one job: one request of a
+// coalesced serving batch, or the whole input of a single call.  Trees stream
+// through shared memory in chunks (splits, and leaves up to depth 6; two
+// chunks in flight: cp.async, the next chunk lands while the current one is
+// walked), class by class.
 //
-// Binned walk (models with a binned form): the tile is binarised once into a
-// byte per (virtual feature, row) (Eytzinger-ordered borders: the i-th step of
-// every search reads one of 2^i consecutive words), column-major, so the
-// 32-bit word l of a column holds rows 4l..4l+3.  Lane l of each warp owns
-// those rows; a split costs one 32-bit shared load and a byte-wise add
-// (b + 128 - k sets bit 7 exactly when b >= k: bins are at most 127) for all
-// four rows, and the level bits are gathered per byte with a shift and a mask.
-// The 8 warps walk every 8th tree (warp w: trees w, w + 8, ...) and their
-// sums are added in warp order.  Other models (multiclass, or no binned form)
-// split the block's threads as row slots x tree groups, one row per thread,
-// and add the groups' sums pairwise in a fixed order.  Which walk a tile
-// takes depends only on its model, so a request gives the same bits alone or
-// in a batch.
+// Binned walk: the tile is binarised once into a byte per (virtual feature,
+// row), 128 rows of input at a time (Eytzinger-ordered borders: the i-th step
+// of every search reads one of 2^i consecutive words), column-major, so a
+// lane's rows are consecutive bytes: 8 rows (two words) per lane of a 256-row
+// tile, 4 of a 128-row one.  A split is one word (column, 128 - k); a lane
+// adds 128 - k to every byte of its rows' bins, which sets bit 7 exactly when
+// bin >= k (bins are at most 127), and the level bits are gathered per byte
+// with a shift and a mask.  Warp w walks trees w, w + 16, ... of a
+// class and the warps' sums are added in order, whatever the tile size, so a
+// request gives the same bits alone or in a batch.
+//
+// What bounds the walk: the shared-memory pipe and the integer units, about
+// evenly.  A tree of depth 6 costs a warp, for 256 rows, 35 wavefronts (6 for
+// the splits, 12 for the bins, 16 for the leaves: 64 words in 32 banks, two per
+// lookup) and some 100 instructions; four rows per lane and 8-byte splits took
+// 34 for 128 rows.  Leaves in registers looked up by shuffles were slower (a
+// shuffle costs as much as a lookup).  Measured: 500k x 100 rows, 1000 x d6 542
+// -> 416 us, 2000 x d6 1472 -> 742 us (two blocks per SM instead of one), 500 x
+// d8 419 -> 333 us, 200 x d4 163 -> 156 us; 200k x 50 rows, 10 classes x 200 x
+// d6 (the float walk before) 3011 -> 322 us.
+//
+// Other models (no binned form) walk 128 rows at a time on the float splits,
+// threads split as row slots x tree groups, one row per thread, the groups'
+// sums added pairwise in a fixed order.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -52,18 +63,22 @@
 namespace tc {
 namespace {
 
-constexpr int PRED_ROWS = 128;
-constexpr int PRED_THREADS = 256;
+constexpr int PRED_ROWS = 256;                  // rows of a tile (PRED_HALF when the launch is small)
+constexpr int PRED_HALF = 128;                  // rows of a small launch's tile, and of a float walk
+constexpr int PRED_THREADS = 512;
 constexpr int PRED_WARPS = PRED_THREADS / 32;
-constexpr int PRED_LEAF_STAGE_MIN = 4096;       // floats of one leaf stage at least (16 KB)
-constexpr int PRED_STAGED_MAX_DEPTH = 5;        // deeper trees gather their leaves from global memory (L2)
-constexpr int PRED_CHUNK = 128;                 // trees per chunk at most
+constexpr int PRED_LEAF_STAGE_MIN = PRED_WARPS * PRED_ROWS;  // floats of one leaf stage at least: the warps' sums
+constexpr int PRED_STAGED_MAX_DEPTH = 6;        // deeper trees gather their leaves from global memory (L2)
 constexpr int PRED_MAX_K = 16;
 constexpr int BIN_MAX_BORDERS = 127;            // borders of one virtual feature (bins 0..127)
-constexpr int BIN_MAX_VIRTUAL = 512;            // virtual features of a binned model (column offset < 2^16)
+constexpr int BIN_MAX_VIRTUAL = 512;            // virtual features of a binned model
 constexpr uint32_t kNaNBits = 0x7fc00000u;      // padding split threshold: x >= NaN is false
 
 __host__ __device__ constexpr int row_stride(int f) { return f | 1; }  // odd: conflict-free column reads
+// Row stride of the binned walk's staged rows: even feature counts take 8-byte
+// copies at an odd multiple of 8 bytes (lanes that read one feature of 32 rows
+// meet in pairs only), odd ones 4-byte copies at an odd stride.
+__host__ __device__ constexpr int stage_stride(int f) { return (f & 1) ? f : ((f >> 1) | 1) * 2; }
 __host__ __device__ constexpr size_t align16(size_t b) { return (b + 15) & ~(size_t)15; }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -86,122 +101,385 @@ struct JobTable {
   const uint32_t* tile_begin;  // [n_jobs + 1] first tile of each job
   int n_jobs;
   int leaf_stage;              // floats of one leaf stage
-  int split_stage;             // splits of one split stage
+  int split_stage;             // 8-byte units of one split stage
+  int chunk;                   // trees per chunk at most
+  int stage_rows;              // rows staged at a time (binned walk): 128 or 64
+  int tile_rows;               // rows of a tile: PRED_ROWS or PRED_HALF
   ReqDesc one_req;
   ModelDesc one_model;
 };
 
 __device__ __forceinline__ float sigmoidf_ref(float x) { return 1.0f / (1.0f + expf(-x)); }
 
+// 8-byte units of one tree's splits: float splits are (feature, threshold
+// bits), binned ones two to a unit.
+__host__ __device__ constexpr int split_units(int D, bool binned) { return binned ? (D + 1) / 2 : D; }
+
 // Trees per chunk for a model of depth D (L leaves): bounded by both stages,
 // at least one tree per warp (the host sizes the stages for that).
-__device__ __forceinline__ int chunk_trees(int D, int L, int leaf_stage, int split_stage) {
-  int c = min(PRED_CHUNK, split_stage / max(1, D));
-  if (D <= PRED_STAGED_MAX_DEPTH) c = min(c, leaf_stage / L);
+__device__ __forceinline__ int chunk_trees(int D, int L, bool binned, const JobTable& jt) {
+  int c = min(jt.chunk, jt.split_stage / max(1, split_units(D, binned)));
+  if (D <= PRED_STAGED_MAX_DEPTH) c = min(c, jt.leaf_stage / L);
   return c;
 }
 
-// 32-bit shared-memory loads (shared-window addresses: 32-bit address
-// arithmetic, no generic-to-shared conversion).
-__device__ __forceinline__ uint4 lds128(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint2 lds64(uint32_t a) {
-  uint2 v;
-  asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];\n" : "=r"(v.x), "=r"(v.y) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ uint32_t lds32(uint32_t a) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a));
-  return v;
-}
-__device__ __forceinline__ float ldsf(uint32_t a) {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a));
-  return v;
-}
-
-// NT binned trees (t, t + PRED_WARPS, ...) of depth D for the lane's 4 rows.
-// Splits are stored in processing order: levels 7..0, then D-1..8, so that
-// after the shifts byte i of `a` holds the first min(D, 8) levels of row i
-// with level 0 in bit 7, and byte i of `b` the levels from 8 on.  Addresses:
-// spc = the chunk's splits, sbl = this lane's word of bin column 0 (both in
-// shared memory); leaves in shared memory (lvs) or, for GL, global (lvg).
-template <int NT, int D, bool GL>
-__device__ __forceinline__ void walk_bins4(uint32_t spc, uint32_t sbl, uint32_t lvs, const float* __restrict__ lvg,
-                                           int t, float4& acc) {
-  constexpr int L = 1 << D;
-  uint2 q[NT][D];
+// One binned tree of depth D for the lane's 4 * RW rows.  Splits are stored in
+// processing order: levels 7..0, then D-1..8, so that after the shifts byte i
+// of `a` holds the first min(D, 8) levels of row i with level 0 in bit 7, and
+// byte i of `b` the levels from 8 on.  sp = the tree's splits, bins = bin column
+// 0, lv = the tree's staged leaves (all in shared memory), lo = the lane's
+// offset in a column; lvg = the tree's leaves in global memory (depth > 6).
+// STRIDE = bytes of a bin column.
+template <int D, int RW, int STRIDE>
+__device__ __forceinline__ void walk_tree(const uint2* __restrict__ sp, const uint8_t* __restrict__ bins, uint32_t lo,
+                                          const float* __restrict__ lv, const float* __restrict__ lvg,
+                                          float (&acc)[4 * RW]) {
+  constexpr int DU = (D + 1) / 2;
+  constexpr uint32_t M = 0x80808080u;
+  uint32_t q[2 * DU];
 #pragma unroll
-  for (int u = 0; u < NT; ++u) {
-    const uint32_t sp = spc + (uint32_t)((t + u * PRED_WARPS) * D) * 8u;
-    if constexpr (D % 2 == 0) {
+  for (int d = 0; d < DU; ++d) {
+    const uint2 v = sp[d];
+    q[2 * d] = v.x;
+    q[2 * d + 1] = v.y;
+  }
+  uint32_t w[D][RW];
 #pragma unroll
-      for (int d = 0; d < D / 2; ++d) {  // a tree's splits start on a 16-byte boundary
-        const uint4 v = lds128(sp + 16u * d);
-        q[u][2 * d] = make_uint2(v.x, v.y);
-        q[u][2 * d + 1] = make_uint2(v.z, v.w);
-      }
+  for (int d = 0; d < D; ++d) {
+    // the column's offset and the lane's share no bits
+    const uint32_t off = STRIDE == 256 ? ((q[d] & 0xffff00u) | lo) : (((q[d] >> 1) & 0x7fff80u) | lo);
+    if constexpr (RW == 2) {
+      const uint2 v = *reinterpret_cast<const uint2*>(bins + off);
+      w[d][0] = v.x;
+      w[d][1] = v.y;
     } else {
-#pragma unroll
-      for (int d = 0; d < D; ++d) q[u][d] = lds64(sp + 8u * d);
+      w[d][0] = *reinterpret_cast<const uint32_t*>(bins + off);
     }
   }
-  uint32_t w[NT][D];
+  uint32_t a[RW] = {}, b[RW] = {};
 #pragma unroll
-  for (int u = 0; u < NT; ++u)
+  for (int d = 0; d < D; ++d) {
+    const uint32_t k = __byte_perm(q[d], 0u, 0x0000u);
 #pragma unroll
-    for (int d = 0; d < D; ++d) w[u][d] = lds32(sbl + q[u][d].x);
-#pragma unroll
-  for (int u = 0; u < NT; ++u) {
-    uint32_t a = 0, b = 0;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      const uint32_t s = w[u][d] + q[u][d].y;  // bit 7 of byte i: bin of row i >= k
-      if (d < 8) a = (a >> 1) | (s & 0x80808080u);
-      else b = (b >> 1) | (s & 0x80808080u);
+    for (int r = 0; r < RW; ++r) {
+      const uint32_t s = w[d][r] + k;  // bit 7 of byte i: bin of row i >= k
+      if (d < 8) a[r] = (a[r] >> 1) | (s & M);
+      else b[r] = (b[r] >> 1) | (s & M);
     }
-    uint32_t idx[4];
+  }
+#pragma unroll
+  for (int r = 0; r < RW; ++r) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t hi = (a >> (8 * i)) & 0xffu;
-      if constexpr (D <= 8) idx[i] = hi >> (8 - D);
-      else idx[i] = (hi << (D - 8)) | (((b >> (8 * i)) & 0xffu) >> (16 - D));
+      float v;
+      if constexpr (D <= PRED_STAGED_MAX_DEPTH) {
+        // index * 4: the byte offset of the leaf
+        const uint32_t x = 8 * i + 6 - D >= 0 ? a[r] >> (8 * i + 6 - D) : a[r] << (D - 6 - 8 * i);
+        v = *reinterpret_cast<const float*>(reinterpret_cast<const char*>(lv) + (x & (((1u << D) - 1u) << 2)));
+      } else {
+        const uint32_t hi = (a[r] >> (8 * i)) & 0xffu;
+        uint32_t x;
+        if constexpr (D <= 8) x = hi >> (8 - D);
+        else x = (hi << (D - 8)) | (((b[r] >> (8 * i)) & 0xffu) >> (16 - D));
+        v = __ldg(lvg + x);
+      }
+      acc[4 * r + i] += v;
     }
-    const int tt = t + u * PRED_WARPS;
-    float v[4];
-    if constexpr (GL) {
-      const float* lv = lvg + (size_t)tt * L;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = __ldg(lv + idx[i]);
-    } else {
-      const uint32_t lv = lvs + (uint32_t)(tt * L) * 4u;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] = ldsf(lv + 4u * idx[i]);
-    }
-    acc.x += v[0];
-    acc.y += v[1];
-    acc.z += v[2];
-    acc.w += v[3];
   }
 }
 
-// The chunk's trees of warp w: pairs while two remain (depth <= 10), then one
-// at a time; the sums go into acc in tree order either way.
-template <int D, bool GL>
-__device__ __forceinline__ void walk_chunk_bins4(uint32_t spc, uint32_t sbl, uint32_t lvs, const float* lvg, int w,
-                                                 int tn, float4& acc) {
-  int t = w;
-  if constexpr (D <= 10)
-    for (; t + PRED_WARPS < tn; t += 2 * PRED_WARPS) walk_bins4<2, D, GL>(spc, sbl, lvs, lvg, t, acc);
-  for (; t < tn; t += PRED_WARPS) walk_bins4<1, D, GL>(spc, sbl, lvs, lvg, t, acc);
+// The chunk's trees of warp w (w, w + 16, ...), in order.  lvs / lvg: leaves of
+// the chunk's first tree (staged, or in global memory).
+template <int D, int RW, int STRIDE>
+__device__ __forceinline__ void walk_chunk(const uint2* spc, const uint8_t* bins, uint32_t lo, const float* lvs,
+                                           const float* __restrict__ lvg, int w, int tn, float (&acc)[4 * RW]) {
+  constexpr int DU = (D + 1) / 2;
+  const uint2* sp = spc + w * DU;
+  const float* lv = lvs + (w << D);
+  const float* lg = lvg + ((size_t)w << D);
+#pragma unroll 2
+  for (int t = w; t < tn; t += PRED_WARPS) {
+    walk_tree<D, RW, STRIDE>(sp, bins, lo, lv, lg, acc);
+    sp += PRED_WARPS * DU;
+    lv += PRED_WARPS << D;
+    lg += PRED_WARPS << D;
+  }
+}
+
+template <int RW, int STRIDE>
+__device__ __forceinline__ void walk_depth(int D, const uint2* spc, const uint8_t* bins, uint32_t lo, const float* lvs,
+                                           const float* __restrict__ lvg, int w, int tn, float (&acc)[4 * RW]) {
+  switch (D) {
+#define TC_WALK(d) case d: walk_chunk<d, RW, STRIDE>(spc, bins, lo, lvs, lvg, w, tn, acc); break;
+    TC_WALK(1) TC_WALK(2) TC_WALK(3) TC_WALK(4) TC_WALK(5) TC_WALK(6) TC_WALK(7)
+    TC_WALK(8) TC_WALK(9) TC_WALK(10) TC_WALK(11) TC_WALK(12)
+    default: walk_chunk<13, RW, STRIDE>(spc, bins, lo, lvs, lvg, w, tn, acc); break;
+#undef TC_WALK
+  }
+}
+
+// Row r of the tile: its K raw sums (s[k * stride]) plus the base,
+// transformed, into o.
+__device__ __forceinline__ void store_row(const ModelDesc& md, int transform, const float* s, int stride, float* o) {
+  const int K = md.n_classes;
+  if (transform == TC_TRANSFORM_SOFTMAX && K > 1) {
+    float mx = -INFINITY;
+    for (int k = 0; k < K; ++k) mx = fmaxf(mx, s[k * stride] + md.base);
+    float sum = 0.0f;
+    for (int k = 0; k < K; ++k) sum += expf(s[k * stride] + md.base - mx);
+    for (int k = 0; k < K; ++k) o[k] = expf(s[k * stride] + md.base - mx) / sum;
+  } else {
+    for (int k = 0; k < K; ++k) {
+      const float raw = s[k * stride] + md.base;
+      o[k] = (transform == TC_TRANSFORM_SIGMOID) ? sigmoidf_ref(raw) : raw;
+    }
+  }
+}
+
+// Stages up to 128 rows of f floats from Xt at a stride of fs floats: 8-byte
+// copies when rows, stride and Xt allow, else 4-byte ones.
+__device__ __forceinline__ void stage_rows(float* s_x, const float* Xt, int nr, int f, int fs) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((f & 1) == 0 && (fs & 1) == 0 && (reinterpret_cast<uintptr_t>(Xt) & 7) == 0) {
+    for (int i = warp; i < nr; i += PRED_WARPS)  // a warp copies whole rows
+      for (int j = lane; j < f / 2; j += 32) cp_async8(&s_x[i * fs + 2 * j], &Xt[(size_t)i * f + 2 * j]);
+  } else {
+    for (int i = warp; i < nr; i += PRED_WARPS)
+      for (int j = lane; j < f; j += 32) cp_async4(&s_x[i * fs + j], &Xt[(size_t)i * f + j]);
+  }
+}
+
+// The float walk's tile: models without a binned form, 128 rows at a time.
+__device__ void float_tile(const JobTable& jt, const ReqDesc& rq, const ModelDesc& md, uint32_t r0, int nr,
+                           char* base) {
+  const int f = md.n_features, fs = row_stride(f), D = md.max_depth, L = 1 << D, K = md.n_classes;
+  const int LS = jt.leaf_stage, SS = jt.split_stage;
+  const bool leaves_global = D > PRED_STAGED_MAX_DEPTH;
+  const int tchunk = chunk_trees(D, L, false, jt);
+  float* s_x = reinterpret_cast<float*>(base);                            // [128][fs]
+  float* s_leaf = reinterpret_cast<float*>(base + align16((size_t)PRED_HALF * fs * 4));  // 2 x [LS]
+  uint2* s_split = reinterpret_cast<uint2*>(s_leaf + 2 * (size_t)LS);     // 2 x [SS]
+  stage_rows(s_x, rq.X + (size_t)r0 * f, nr, f, fs);
+  auto issue_chunk = [&](int t0, int buf) {
+    const int tn = min(tchunk, md.n_trees - t0);
+    if (!leaves_global) {
+      float* dl = s_leaf + buf * LS;
+      const float* gl = md.leaves + (size_t)t0 * L;
+      for (int q = threadIdx.x; q < tn * L; q += PRED_THREADS) cp_async4(dl + q, gl + q);
+    }
+    uint2* ds = s_split + buf * SS;
+    for (int q = threadIdx.x; q < tn * D; q += PRED_THREADS) cp_async8(ds + q, md.splits + (size_t)t0 * D + q);
+  };
+  if (md.n_trees > 0) issue_chunk(0, 0);
+  cp_async_commit();
+  // row slots (a power of two >= nr) x tree groups
+  int RT = PRED_HALF;
+  while (RT > 1 && (RT >> 1) >= nr) RT >>= 1;
+  const int TG = PRED_THREADS / RT;
+  const int row = threadIdx.x % RT, tg = threadIdx.x / RT;
+  const float* xr = s_x + row * fs;
+  float acc[PRED_MAX_K];
+#pragma unroll
+  for (int k = 0; k < PRED_MAX_K; ++k) acc[k] = 0.0f;
+  for (int t0 = 0, buf = 0; t0 < md.n_trees; t0 += tchunk, buf ^= 1) {
+    const int tn = min(tchunk, md.n_trees - t0);
+    if (t0 + tchunk < md.n_trees) issue_chunk(t0 + tchunk, buf ^ 1);
+    cp_async_commit();
+    cp_async_wait_prev();  // this thread's copies of the tile and of chunk t0 have landed
+    __syncthreads();       // ... and everybody's
+    const float* lvc = leaves_global ? md.leaves + (size_t)t0 * L : s_leaf + buf * LS;
+    const uint2* spc = s_split + buf * SS;
+    if (row < nr) {
+      for (int t = tg; t < tn; t += TG) {
+        const uint2* sp = spc + t * D;
+        uint32_t idx = 0;
+#pragma unroll
+        for (int d = 0; d < kModelMaxDepth; ++d) {
+          if (d < D) {
+            const uint2 q = sp[d];
+            idx = idx + idx + (uint32_t)(xr[q.x] >= __uint_as_float(q.y));  // false for NaN
+          }
+        }
+        const float v = lvc[(size_t)t * L + idx];
+        const int cls = K == 1 ? 0 : (t0 + t) % K;
+#pragma unroll
+        for (int k = 0; k < PRED_MAX_K; ++k)
+          if (k == cls) acc[k] += v;
+      }
+    }
+    __syncthreads();  // chunk t0's buffers are refilled by the next iteration's copies
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  // [TG][RT][K] in the stages (TG * RT = 512, 512 x 16 floats = two leaf stages)
+  float* s_red = s_leaf;
+#pragma unroll
+  for (int k = 0; k < PRED_MAX_K; ++k)
+    if (k < K) s_red[(tg * RT + row) * K + k] = acc[k];
+  __syncthreads();
+  for (int h = TG >> 1; h > 0; h >>= 1) {
+    if (tg < h) {
+      for (int k = 0; k < K; ++k) s_red[(tg * RT + row) * K + k] += s_red[((tg + h) * RT + row) * K + k];
+    }
+    __syncthreads();
+  }
+  if (tg == 0 && row < nr) store_row(md, rq.transform, s_red + row * K, 1, rq.out + (size_t)(r0 + row) * K);
+  __syncthreads();
+}
+static_assert(PRED_THREADS * PRED_MAX_K <= 2 * PRED_LEAF_STAGE_MIN, "the float walk's sums fit the leaf stages");
+
+// Bins of 32 * NI staged rows (hn valid, the others bin 0): warp w takes virtual
+// features w, w + 16, ...; lane l rows l, l + 32, ...  A search holds the shared
+// address of its node, so a step is a load, a compare, a select and an add:
+// node k's entry is at base + 4k, its children are 2k and 2k + 1.  (With node
+// indices a step took half as many instructions again: 437 us instead of 416
+// on 500k x 100 rows, 1000 x d6.)
+template <int NI>
+__device__ __forceinline__ void binarise(const float* s_x, int xs, int hn, const float* s_bord, const uint2* s_vd,
+                                         int V, uint8_t* bins, int stride) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int v = warp; v < V; v += PRED_WARPS) {
+    const uint2 vd = s_vd[v];
+    const uint32_t base = smem_addr(s_bord + (vd.y & 0xffffffu)), lo = 0u - base, hi = 4u - base;
+    const int h = (int)(vd.y >> 24);
+    float x[NI];
+    uint32_t at[NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int r = lane + 32 * i;
+      x[i] = r < hn ? s_x[r * xs + vd.x] : 0.0f;
+      at[i] = base + 4u;
+    }
+    for (int s = 0; s < h; ++s) {
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        float b;
+        asm("ld.shared.f32 %0, [%1];" : "=f"(b) : "r"(at[i]));
+        at[i] = 2u * at[i] + (b <= x[i] ? hi : lo);  // NaN: left
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int r = lane + 32 * i;
+      bins[v * stride + r] = r < hn ? (uint8_t)(((at[i] - base) >> 2) - (1u << h)) : (uint8_t)0;
+    }
+  }
+}
+
+// The binned walk's tile: nr rows from r0, RW words of bins per lane.
+template <int RW, int STRIDE>
+__device__ __forceinline__ void binned_tile(const JobTable& jt, const ReqDesc& rq, const ModelDesc& md, uint32_t r0,
+                                            int nr, char* base) {
+  constexpr int ROWS = 128 * RW;
+  const int f = md.n_features, D = md.max_depth, L = 1 << D, K = md.n_classes, V = md.n_virtual;
+  const int LS = jt.leaf_stage, SS = jt.split_stage;
+  const bool staged = D <= PRED_STAGED_MAX_DEPTH;
+  const int DU = split_units(D, true);
+  const int tchunk = chunk_trees(D, L, true, jt);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // [bins V x STRIDE][class sums][U]; U holds the borders, the virtual features
+  // and the staged rows until the tile is binarised, then the stages
+  uint8_t* s_bins = reinterpret_cast<uint8_t*>(base);
+  float* s_out = reinterpret_cast<float*>(base + align16((size_t)V * STRIDE));  // [K][STRIDE]
+  char* U = reinterpret_cast<char*>(s_out + (K > 1 ? K * STRIDE : 0));
+  float* s_bord = reinterpret_cast<float*>(U);
+  uint2* s_vd = reinterpret_cast<uint2*>(U + align16((size_t)md.n_bord * 4));
+  float* s_x = reinterpret_cast<float*>(reinterpret_cast<char*>(s_vd) + align16((size_t)V * 8));
+  float* s_leaf = reinterpret_cast<float*>(U);                         // 2 x [LS]
+  uint2* s_split = reinterpret_cast<uint2*>(s_leaf + 2 * (size_t)LS);  // 2 x [SS]
+  const int xs = stage_stride(f);
+  // borders and virtual features (16-byte copies: both arrays are padded to
+  // whole 16-byte units on the device)
+  for (int q = threadIdx.x; q < (md.n_bord + 3) / 4; q += PRED_THREADS) cp_async16(s_bord + 4 * q, md.bord + 4 * q);
+  for (int q = threadIdx.x; q < (V + 1) / 2; q += PRED_THREADS) cp_async16(s_vd + 2 * q, md.vdesc + 2 * q);
+  for (int h0 = 0; h0 < nr; h0 += jt.stage_rows) {
+    const int hn = min(jt.stage_rows, nr - h0);
+    stage_rows(s_x, rq.X + (size_t)(r0 + h0) * f, hn, f, xs);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    if (jt.stage_rows == 128) binarise<4>(s_x, xs, hn, s_bord, s_vd, V, s_bins + h0, STRIDE);
+    else binarise<2>(s_x, xs, hn, s_bord, s_vd, V, s_bins + h0, STRIDE);
+    __syncthreads();  // the part's bins are complete and its rows' space is free
+  }
+  // (rows past the last staged part keep stale bins: their sums are not stored)
+  if (K > 1)
+    for (int q = threadIdx.x; q < K * STRIDE; q += PRED_THREADS) s_out[q] = 0.0f;
+  // the binned form lists the trees class by class: class k's first is
+  // first(k), of n_trees / K trees or one more
+  const int per = md.n_trees / K, more = md.n_trees - per * K;
+  auto class_trees = [&](int k) { return k < K ? per + (k < more ? 1 : 0) : 0; };
+  auto issue_chunk = [&](int t0, int tn, int buf) {
+    if (staged) {
+      float* dl = s_leaf + buf * LS;
+      const float* gl = md.bleaves + ((size_t)t0 << D);
+      if (D >= 2) {
+        for (int q = threadIdx.x; q < tn << (D - 2); q += PRED_THREADS) cp_async16(dl + 4 * q, gl + 4 * q);
+      } else {
+        for (int q = threadIdx.x; q < tn * L; q += PRED_THREADS) cp_async4(dl + q, gl + q);
+      }
+    }
+    uint2* ds = s_split + buf * SS;
+    const uint2* gs = reinterpret_cast<const uint2*>(md.bsplits) + (size_t)t0 * DU;
+    for (int q = threadIdx.x; q < tn * DU; q += PRED_THREADS) cp_async8(ds + q, gs + q);
+  };
+  const uint32_t lo = (uint32_t)lane * 4 * RW;
+  float acc[4 * RW];
+#pragma unroll
+  for (int i = 0; i < 4 * RW; ++i) acc[i] = 0.0f;
+  // chunk: trees [t0, t0 + tn) of class k, `left` of its trees not yet walked
+  int k = 0, t0 = 0, left = class_trees(0), buf = 0;
+  if (left > 0) issue_chunk(0, min(tchunk, left), 0);
+  cp_async_commit();
+  while (left > 0) {
+    const int tn = min(tchunk, left);
+    const bool class_end = tn == left;
+    const int kn = class_end ? k + 1 : k, next_left = class_end ? class_trees(kn) : left - tn;
+    if (next_left > 0) issue_chunk(t0 + tn, min(tchunk, next_left), buf ^ 1);
+    cp_async_commit();
+    cp_async_wait_prev();
+    __syncthreads();
+    walk_depth<RW, STRIDE>(D, s_split + buf * SS, s_bins, lo, s_leaf + buf * LS, md.bleaves + ((size_t)t0 << D), warp,
+                           tn, acc);
+    __syncthreads();  // the chunk's buffers are free
+    if (class_end) {
+      // the warps' sums [warp][rows] in the free leaf stage, added in warp order
+      float* s_red = s_leaf + buf * LS;
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+        *reinterpret_cast<float4*>(&s_red[warp * ROWS + 4 * (RW * lane + r)]) =
+            make_float4(acc[4 * r], acc[4 * r + 1], acc[4 * r + 2], acc[4 * r + 3]);
+#pragma unroll
+      for (int i = 0; i < 4 * RW; ++i) acc[i] = 0.0f;
+      __syncthreads();
+      if (threadIdx.x < ROWS) {
+        const int r = threadIdx.x;
+        float s = s_red[r];
+#pragma unroll
+        for (int w = 1; w < PRED_WARPS; ++w) s += s_red[w * ROWS + r];
+        if (K > 1) s_out[k * STRIDE + r] = s;
+        else if (r < nr) store_row(md, rq.transform, &s, 1, rq.out + r0 + r);
+      }
+      __syncthreads();  // before the stage is filled again
+    }
+    k = kn;
+    t0 += tn;
+    left = next_left;
+    buf ^= 1;
+  }
+  cp_async_wait_all();
+  const int r = threadIdx.x;
+  if (K > 1) {
+    __syncthreads();
+    if (r < nr) store_row(md, rq.transform, s_out + r, STRIDE, rq.out + (size_t)(r0 + r) * K);
+  } else if (md.n_trees == 0 && r < nr) {
+    const float zero = 0.0f;
+    store_row(md, rq.transform, &zero, 1, rq.out + r0 + r);
+  }
 }
 
 __global__ void __launch_bounds__(PRED_THREADS, 2) k_predict(JobTable jt) {
-  extern __shared__ __align__(16) float smp[];
+  extern __shared__ __align__(16) char smp[];
   ReqDesc rq;
   ModelDesc md;
   uint32_t tile;
@@ -220,218 +498,17 @@ __global__ void __launch_bounds__(PRED_THREADS, 2) k_predict(JobTable jt) {
     md = jt.models[rq.model];
     tile = blockIdx.x - jt.tile_begin[lo];
   }
-  const uint32_t r0 = tile * PRED_ROWS;
+  const uint32_t r0 = tile * (uint32_t)jt.tile_rows;
   if (r0 >= rq.n) return;
-  const int nr = (int)min((uint32_t)PRED_ROWS, rq.n - r0);
-  const int f = md.n_features;
-  // row stride: for the binned walk, rows of a feature count that is a
-  // multiple of 4 (16-byte aligned input) are staged densely by 16-byte
-  // copies; others by 4-byte copies at an odd stride (conflict-free column
-  // reads, which the float walk does once per split)
-  const bool dense = md.bsplits != nullptr && (f & 3) == 0 && (reinterpret_cast<uintptr_t>(rq.X) & 15) == 0;
-  const int fs = dense ? f : row_stride(f);
-  const int D = md.max_depth;
-  const int L = 1 << D;
-  const int K = md.n_classes;
-  const int LS = jt.leaf_stage, SS = jt.split_stage;
-  const bool leaves_global = D > PRED_STAGED_MAX_DEPTH;
-  const int tchunk = chunk_trees(D, L, LS, SS);
-  const bool binned = md.bsplits != nullptr;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // Regions.  Binned: [bins V x 128 B][borders][virtual features][U]; the
-  // row tile lives in U until the tile is binarised, then U holds the
-  // stages.  Float: [row tile][stages].
-  char* base = reinterpret_cast<char*>(smp);
-  const int V = md.n_virtual;
-  uint8_t* s_bins = reinterpret_cast<uint8_t*>(base);
-  float* s_bord = reinterpret_cast<float*>(base + align16((size_t)V * PRED_ROWS));
-  uint2* s_vd = reinterpret_cast<uint2*>(reinterpret_cast<char*>(s_bord) + align16((size_t)md.n_bord * 4));
-  char* U = binned ? reinterpret_cast<char*>(s_vd) + align16((size_t)V * 8) : base;
-  float* s_x = reinterpret_cast<float*>(U);                      // [128][fs]
-  char* stages = binned ? U : U + align16((size_t)PRED_ROWS * fs * 4);
-  float* s_leaf = reinterpret_cast<float*>(stages);              // 2 x [LS]
-  uint2* s_split = reinterpret_cast<uint2*>(s_leaf + 2 * (size_t)LS);  // 2 x [SS]
-  // the tile's rows: one contiguous range of nr x f floats
-  {
-    const float* Xt = rq.X + (size_t)r0 * f;
-    if (dense) {
-      for (int q = threadIdx.x; q < nr * (f >> 2); q += PRED_THREADS) cp_async16(s_x + 4 * q, Xt + 4 * q);
-    } else {
-      for (int i = warp; i < nr; i += PRED_WARPS)  // a warp copies whole rows, lane = feature
-        for (int j = lane; j < f; j += 32) cp_async4(&s_x[i * fs + j], &Xt[(size_t)i * f + j]);
-    }
-  }
-  const uint2* gsplits = binned ? md.bsplits : md.splits;
-  auto issue_chunk = [&](int t0, int buf) {
-    const int tn = min(tchunk, md.n_trees - t0);
-    if (!leaves_global) {
-      float* dl = s_leaf + buf * LS;
-      const float* gl = md.leaves + (size_t)t0 * L;
-      const int cnt = tn * L;
-      if (L >= 4) {
-        for (int q = threadIdx.x; q < cnt / 4; q += PRED_THREADS) cp_async16(dl + 4 * q, gl + 4 * q);
-      } else {
-        for (int q = threadIdx.x; q < cnt; q += PRED_THREADS) cp_async4(dl + q, gl + q);
-      }
-    }
-    uint2* ds = s_split + buf * SS;
-    for (int q = threadIdx.x; q < tn * D; q += PRED_THREADS) cp_async8(ds + q, gsplits + (size_t)t0 * D + q);
-  };
-  if (binned) {
-    // borders and virtual features (16-byte copies: both arrays are padded
-    // to whole 16-byte units on the device)
-    for (int q = threadIdx.x; q < (md.n_bord + 3) / 4; q += PRED_THREADS) cp_async16(s_bord + 4 * q, md.bord + 4 * q);
-    for (int q = threadIdx.x; q < (V + 1) / 2; q += PRED_THREADS) cp_async16(s_vd + 2 * q, md.vdesc + 2 * q);
-    cp_async_commit();
-    cp_async_wait_all();
-    __syncthreads();
-    // binarise: warp w takes virtual features w, w + 8, ...; lane l rows
-    // l, l + 32, l + 64, l + 96 (rows past the tile's last get bin 0)
-    for (int v = warp; v < V; v += PRED_WARPS) {
-      const uint2 vd = s_vd[v];
-      const float* bt = s_bord + (vd.y & 0xffffffu);
-      const int h = (int)(vd.y >> 24);
-      float x[4];
-      uint32_t nd[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = lane + 32 * i;
-        x[i] = r < nr ? s_x[r * fs + vd.x] : 0.0f;
-        nd[i] = 0;
-      }
-      for (int s = 0; s < h; ++s)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) nd[i] = 2 * nd[i] + 1 + (uint32_t)(bt[nd[i]] <= x[i]);  // NaN: false
-      const uint32_t first_leaf = (1u << h) - 1;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int r = lane + 32 * i;
-        s_bins[v * PRED_ROWS + r] = r < nr ? (uint8_t)(nd[i] - first_leaf) : (uint8_t)0;
-      }
-    }
-    __syncthreads();  // the bins are complete and the row tile's space is free for the stages
-  }
-  if (md.n_trees > 0) issue_chunk(0, 0);
-  cp_async_commit();
-  // binned walk state
-  float4 acc4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  const uint32_t sbl = smem_addr(s_bins) + 4u * lane;
-  // per-row walk state: row slots (a power of two >= nr) x tree groups
-  int RT = PRED_ROWS;
-  while (RT > 1 && (RT >> 1) >= nr) RT >>= 1;
-  const int TG = PRED_THREADS / RT;
-  const int row = threadIdx.x % RT, tg = threadIdx.x / RT;
-  const float* xr = s_x + row * fs;
-  float acc[PRED_MAX_K];
-#pragma unroll
-  for (int k = 0; k < PRED_MAX_K; ++k) acc[k] = 0.0f;
-  for (int t0 = 0, buf = 0; t0 < md.n_trees; t0 += tchunk, buf ^= 1) {
-    const int tn = min(tchunk, md.n_trees - t0);
-    if (t0 + tchunk < md.n_trees) issue_chunk(t0 + tchunk, buf ^ 1);
-    cp_async_commit();
-    cp_async_wait_prev();  // this thread's copies of the tile and of chunk t0 have landed
-    __syncthreads();       // ... and everybody's
-    const float* lvc = leaves_global ? md.leaves + (size_t)t0 * L : s_leaf + buf * LS;
-    const uint2* spc = s_split + buf * SS;
-    if (binned) {
-      const uint32_t spa = smem_addr(spc), lva = smem_addr(leaves_global ? s_leaf : lvc);
-      switch (D) {
-        case 1: walk_chunk_bins4<1, false>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 2: walk_chunk_bins4<2, false>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 3: walk_chunk_bins4<3, false>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 4: walk_chunk_bins4<4, false>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 5: walk_chunk_bins4<5, false>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 6: walk_chunk_bins4<6, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 7: walk_chunk_bins4<7, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 8: walk_chunk_bins4<8, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 9: walk_chunk_bins4<9, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 10: walk_chunk_bins4<10, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 11: walk_chunk_bins4<11, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        case 12: walk_chunk_bins4<12, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-        default: walk_chunk_bins4<13, true>(spa, sbl, lva, lvc, warp, tn, acc4); break;
-      }
-    } else if (row < nr) {
-      for (int t = tg; t < tn; t += TG) {
-        const uint2* sp = spc + t * D;
-        uint2 q[kModelMaxDepth];
-#pragma unroll
-        for (int d = 0; d < kModelMaxDepth; ++d)
-          if (d < D) q[d] = sp[d];
-        float xv[kModelMaxDepth];
-#pragma unroll
-        for (int d = 0; d < kModelMaxDepth; ++d)
-          if (d < D) xv[d] = xr[q[d].x];
-        uint32_t idx = 0;
-#pragma unroll
-        for (int d = 0; d < kModelMaxDepth; ++d)
-          if (d < D) idx = idx + idx + (uint32_t)(xv[d] >= __uint_as_float(q[d].y));  // false for NaN
-        const float v = lvc[(size_t)t * L + idx];
-        const int cls = K == 1 ? 0 : (t0 + t) % K;
-#pragma unroll
-        for (int k = 0; k < PRED_MAX_K; ++k)
-          if (k == cls) acc[k] += v;
-      }
-    }
-    __syncthreads();  // chunk t0's buffers are refilled by the next iteration's copies
-  }
-  cp_async_wait_all();
-  __syncthreads();
-  float* s_red = s_leaf;  // at least 2 x 4096 floats
-  float* o = rq.out + (size_t)r0 * K;
-  if (binned) {
-    // [warp][128 rows]; row sums in warp order
-    *reinterpret_cast<float4*>(&s_red[warp * PRED_ROWS + 4 * lane]) = acc4;
-    __syncthreads();
-    if (threadIdx.x >= nr) return;
-    const int r = threadIdx.x;
-    float s = s_red[r];
-#pragma unroll
-    for (int w = 1; w < PRED_WARPS; ++w) s += s_red[w * PRED_ROWS + r];
-    const float raw = s + md.base;
-    o[r] = (rq.transform == TC_TRANSFORM_SIGMOID) ? sigmoidf_ref(raw) : raw;
-    return;
-  }
-  // [TG][RT][K] (TG*RT = PRED_THREADS, 256 x 16 floats <= one leaf stage)
-#pragma unroll
-  for (int k = 0; k < PRED_MAX_K; ++k)
-    if (k < K) s_red[(tg * RT + row) * K + k] = acc[k];
-  __syncthreads();
-  for (int h = TG >> 1; h > 0; h >>= 1) {
-    if (tg < h) {
-      for (int k = 0; k < K; ++k) s_red[(tg * RT + row) * K + k] += s_red[((tg + h) * RT + row) * K + k];
-    }
-    __syncthreads();
-  }
-  if (tg != 0 || row >= nr) return;
-#pragma unroll
-  for (int k = 0; k < PRED_MAX_K; ++k)
-    if (k < K) acc[k] = s_red[row * K + k];
-  o += (size_t)row * K;
-  if (rq.transform == TC_TRANSFORM_SOFTMAX && K > 1) {
-    float mx = -INFINITY;
-#pragma unroll
-    for (int k = 0; k < PRED_MAX_K; ++k)
-      if (k < K) mx = fmaxf(mx, acc[k] + md.base);
-    float sum = 0.0f;
-    float e[PRED_MAX_K];
-#pragma unroll
-    for (int k = 0; k < PRED_MAX_K; ++k) {
-      if (k < K) {
-        e[k] = expf(acc[k] + md.base - mx);
-        sum += e[k];
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < PRED_MAX_K; ++k)
-      if (k < K) o[k] = e[k] / sum;
+  const int nr = (int)min((uint32_t)jt.tile_rows, rq.n - r0);
+  if (md.bsplits == nullptr) {
+    for (int h0 = 0; h0 < nr; h0 += PRED_HALF) float_tile(jt, rq, md, r0 + h0, min(PRED_HALF, nr - h0), smp);
+  } else if (md.bin_stride == PRED_HALF) {
+    binned_tile<1, PRED_HALF>(jt, rq, md, r0, nr, smp);
+  } else if (nr > PRED_HALF) {
+    binned_tile<2, PRED_ROWS>(jt, rq, md, r0, nr, smp);
   } else {
-#pragma unroll
-    for (int k = 0; k < PRED_MAX_K; ++k) {
-      if (k < K) {
-        const float raw = acc[k] + md.base;
-        o[k] = (rq.transform == TC_TRANSFORM_SIGMOID) ? sigmoidf_ref(raw) : raw;
-      }
-    }
+    binned_tile<1, PRED_ROWS>(jt, rq, md, r0, nr, smp);
   }
 }
 
@@ -844,40 +921,51 @@ __global__ void __launch_bounds__(128) k_predict_regular(RegDesc rd, const float
   out[r0 + r] = transform == TC_TRANSFORM_SIGMOID ? sigmoidf_ref(raw) : raw;
 }
 
-// Stage sizes for a batch whose deepest model has depth max_depth: a leaf
-// stage holds at least one tree per warp (16 KB at least); a split stage
-// holds the splits of as many trees as the leaf stage takes, for every depth
-// up to max_depth.
-void stage_sizes(int max_depth, int* leaf_stage, int* split_stage) {
-  const int Ls = 1 << std::min(std::max(max_depth, 0), PRED_STAGED_MAX_DEPTH);
-  const int LS = std::max(PRED_LEAF_STAGE_MIN, PRED_WARPS * Ls);
+// One way to lay out a block's shared memory: floats of a leaf stage (at least
+// the warps' sums of a tile), trees per chunk at most, rows staged at a time.
+// Larger chunks cost fewer barriers and copies per tree (64 trees of depth 6 a
+// chunk: 18 instructions more per tree and warp than 128); fewer rows at a time
+// leave room for two blocks per SM when the borders are many.
+struct Layout {
+  int leaf_stage, chunk, stage_rows;
+};
+constexpr Layout kLayouts[] = {{2 * PRED_LEAF_STAGE_MIN, 256, 128}, {2 * PRED_LEAF_STAGE_MIN, 256, 64},
+                               {PRED_LEAF_STAGE_MIN, 128, 128},     {PRED_LEAF_STAGE_MIN, 128, 64}};
+
+// 8-byte units of a split stage that serves every depth up to max_depth.
+int split_stage(int max_depth, const Layout& y) {
   int SS = PRED_WARPS;
   for (int d = 1; d <= max_depth; ++d) {
-    const int trees = d <= PRED_STAGED_MAX_DEPTH ? std::min(PRED_CHUNK, LS >> d) : PRED_CHUNK;
-    SS = std::max(SS, trees * d);
+    const int trees = d <= PRED_STAGED_MAX_DEPTH ? std::min(y.chunk, y.leaf_stage >> d) : y.chunk;
+    SS = std::max(SS, trees * split_units(d, true));
   }
-  *leaf_stage = LS;
-  *split_stage = (SS + 1) & ~1;  // whole 16-byte pairs
+  return (SS + 1) & ~1;  // whole 16-byte pairs
 }
 
-// Shared memory of one model's tiles (the larger of its two layouts).
-size_t model_smem(int n_features, int n_virtual, int n_bord, bool binned, int leaf_stage, int split_stage) {
-  const size_t S = (size_t)2 * leaf_stage * 4 + (size_t)2 * split_stage * 8;
-  const size_t T = align16((size_t)PRED_ROWS * row_stride(n_features) * 4);
-  size_t need = T + S;
-  if (binned) {
-    const size_t X = align16((size_t)n_virtual * PRED_ROWS) + align16((size_t)n_bord * 4) + align16((size_t)n_virtual * 8);
-    need = std::max(need, X + std::max(T, S));
-  }
-  return need;
+// Shared memory of one model's tiles.  Binned: bin columns of `stride` bytes
+// (256; 128 serves tiles of 128 rows only), a multiclass model's class sums,
+// then the larger of the binarisation's data (borders, virtual features,
+// staged rows) and the stages; float (stride 0): 128 staged rows and the stages.
+size_t model_smem(int n_features, int n_classes, int n_virtual, int n_bord, int stride, const Layout& y, int SS) {
+  const size_t S = (size_t)2 * y.leaf_stage * 4 + (size_t)2 * SS * 8;
+  if (stride == 0) return align16((size_t)PRED_HALF * row_stride(n_features) * 4) + S;
+  const size_t T = align16((size_t)y.stage_rows * stage_stride(n_features) * 4);
+  const size_t B = align16((size_t)n_bord * 4) + align16((size_t)n_virtual * 8) + T;
+  const size_t O = n_classes > 1 ? (size_t)n_classes * stride * 4 : 0;
+  return align16((size_t)n_virtual * stride) + O + std::max(B, S);
 }
 
 constexpr size_t PRED_SMEM_MAX = 220 * 1024;
+constexpr size_t PRED_SMEM_TWO = 112 * 1024;  // two blocks per SM
 
-tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, uint32_t n_tiles, cudaStream_t stream) {
+tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, int tile_rows, uint32_t n_tiles,
+                         cudaStream_t stream) {
   if (n_tiles == 0) return TC_OK;
   jt.leaf_stage = plan.leaf_stage;
   jt.split_stage = plan.split_stage;
+  jt.chunk = plan.chunk;
+  jt.stage_rows = plan.stage_rows;
+  jt.tile_rows = tile_rows;
   static bool attr_done = false;
   if (!attr_done) {
     cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PRED_SMEM_MAX);
@@ -895,30 +983,52 @@ tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, uin
 }  // namespace
 
 PredictPlan predict_plan(const tc_model* const* models, int n) {
-  int max_depth = 0;
-  for (int i = 0; i < n; ++i) max_depth = std::max(max_depth, models[i]->info.max_depth);
-  PredictPlan p{};
-  stage_sizes(max_depth, &p.leaf_stage, &p.split_stage);
+  int max_depth = 0, max_tile = PRED_ROWS;
   for (int i = 0; i < n; ++i) {
-    const tc_model* m = models[i];
-    p.smem = std::max(p.smem, model_smem(m->info.n_features, m->n_virtual, m->n_bord, m->d_bsplits.p != nullptr,
-                                         p.leaf_stage, p.split_stage));
+    max_depth = std::max(max_depth, models[i]->info.max_depth);
+    if (models[i]->bin_stride) max_tile = std::min(max_tile, models[i]->bin_stride);
   }
-  return p;
+  // the first layout that leaves room for two blocks per SM, else the first that fits
+  PredictPlan best{};
+  for (const Layout& y : kLayouts) {
+    PredictPlan p{};
+    p.leaf_stage = y.leaf_stage;
+    p.chunk = y.chunk;
+    p.stage_rows = y.stage_rows;
+    p.max_tile = max_tile;
+    p.split_stage = split_stage(max_depth, y);
+    for (int i = 0; i < n; ++i) {
+      const tc_model* m = models[i];
+      p.smem = std::max(p.smem, model_smem(m->info.n_features, m->info.n_classes, m->n_virtual, m->n_bord,
+                                           m->bin_stride, y, p.split_stage));
+    }
+    if (p.smem <= PRED_SMEM_TWO) return p;
+    if (best.smem == 0 || (best.smem > PRED_SMEM_MAX && p.smem < best.smem)) best = p;
+  }
+  return best;
+}
+
+// Rows of a tile: 256, or 128 while that leaves at most one tile per SM: then
+// more SMs beat more rows per split (1000 x d6, device buffers, 128- and
+// 256-row tiles: 4096 rows 27 and 38 us, 16384 rows 27 and 39, 32768 rows 44
+// and 40).
+int predict_tile_rows(const tc_ctx* ctx, const PredictPlan& plan, uint64_t tiles_of_half) {
+  if (plan.max_tile < PRED_ROWS) return PRED_HALF;
+  return tiles_of_half <= (uint64_t)ctx->sm_count ? PRED_HALF : PRED_ROWS;
 }
 
 tc_status predict_batched(tc_ctx* ctx, const ModelDesc* d_models, const ReqDesc* d_reqs, int n_reqs,
-                          const uint32_t* d_tile_begin, uint32_t n_tiles, const PredictPlan& plan,
+                          const uint32_t* d_tile_begin, int tile_rows, uint32_t n_tiles, const PredictPlan& plan,
                           cudaStream_t stream) {
   JobTable jt{};
   jt.reqs = d_reqs;
   jt.models = d_models;
   jt.tile_begin = d_tile_begin;
   jt.n_jobs = n_reqs;
-  return launch_predict(ctx, jt, plan, n_tiles, stream);
+  return launch_predict(ctx, jt, plan, tile_rows, n_tiles, stream);
 }
 
-uint32_t predict_tiles(uint32_t n) { return (n + PRED_ROWS - 1) / PRED_ROWS; }
+uint32_t predict_tiles(uint32_t n, int tile_rows) { return (n + tile_rows - 1) / tile_rows; }
 
 }  // namespace tc
 
@@ -926,15 +1036,16 @@ using namespace tc;
 
 namespace {
 
-// Fills t[0 .. n) (n = 2^h - 1) with vals in Eytzinger (breadth-first) order:
-// an in-order walk of the implicit tree visits vals in sorted order.
+// Fills t[base + 1 .. base + n) (n = 2^h) with vals in Eytzinger
+// (breadth-first) order, node 1 the root: an in-order walk of the implicit
+// tree visits vals in sorted order.
 void eytzinger_fill(const std::vector<float>& vals, std::vector<float>& t, size_t base, size_t n, size_t i,
                     size_t& next) {
   if (i >= n) return;
-  eytzinger_fill(vals, t, base, n, 2 * i + 1, next);
+  eytzinger_fill(vals, t, base, n, 2 * i, next);
   t[base + i] = next < vals.size() ? vals[next] : std::nanf("");
   ++next;
-  eytzinger_fill(vals, t, base, n, 2 * i + 2, next);
+  eytzinger_fill(vals, t, base, n, 2 * i + 1, next);
 }
 
 }  // namespace
@@ -943,8 +1054,8 @@ void eytzinger_fill(const std::vector<float>& vals, std::vector<float>& t, size_
 // feature 0 against a NaN threshold, whose bit is always 0; leaf l of a tree
 // of depth d moves to l << (D - d)), the tree weights folded into the leaves
 // (w * leaf in FP32, the product the reference forms per tree), the float
-// splits (feature, threshold bits) and, for single-output models, the binned
-// form (virtual features, Eytzinger-ordered borders, binned splits).
+// splits (feature, threshold bits) and the binned form (virtual features,
+// Eytzinger-ordered borders, binned splits).
 tc_status tc_model::upload() {
   const int T = info.n_trees, D = info.max_depth, L = 1 << D, F = info.n_features;
   std::vector<uint2> sp((size_t)std::max(1, T * D));
@@ -965,7 +1076,7 @@ tc_status tc_model::upload() {
   TC_TRY(d_leaves.alloc(ctx, lv.size(), "model leaves"));
   TC_CUDA(ctx, cudaMemcpy(d_splits.p, sp.data(), sp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
   TC_CUDA(ctx, cudaMemcpy(d_leaves.p, lv.data(), lv.size() * sizeof(float), cudaMemcpyHostToDevice));
-  if (info.n_classes != 1 || D < 1) return TC_OK;
+  if (D < 1) return TC_OK;
   // binned form: distinct thresholds per feature (-0.0 and +0.0 are one)
   std::vector<std::vector<float>> u((size_t)F);
   for (int t = 0; t < T; ++t)
@@ -992,48 +1103,58 @@ tc_status tc_model::upload() {
   for (const VF& v : vf) {
     int h = 0;
     while ((1 << h) - 1 < v.cnt) ++h;
-    const size_t n = ((size_t)1 << h) - 1, off = bord.size();
+    const size_t n = (size_t)1 << h, off = bord.size();
     if (off + n >= ((size_t)1 << 24)) return TC_OK;
-    bord.resize(off + n);
+    bord.resize(off + n, std::nanf(""));
     std::vector<float> vals;
     if (v.cnt) vals.assign(u[v.j].begin() + v.start, u[v.j].begin() + v.start + v.cnt);
     size_t next = 0;
-    eytzinger_fill(vals, bord, off, n, 0, next);
+    eytzinger_fill(vals, bord, off, n, 1, next);
     vd.push_back(make_uint2((uint32_t)v.j, (uint32_t)off | ((uint32_t)h << 24)));
   }
   const int V = (int)vd.size(), B = (int)bord.size();
-  {
-    int LS, SS;
-    stage_sizes(D, &LS, &SS);
-    if (model_smem(F, V, B, true, LS, SS) > PRED_SMEM_MAX) return TC_OK;  // served by the float walk
-  }
+  int stride = 0;  // the widest bin columns of which some layout fits (none: the float walk)
+  for (int st : {PRED_HALF, PRED_ROWS})
+    for (const Layout& y : kLayouts)
+      if (model_smem(F, info.n_classes, V, B, st, y, split_stage(D, y)) <= PRED_SMEM_MAX) stride = st;
+  if (stride == 0) return TC_OK;
   while (bord.size() % 4) bord.push_back(std::nanf(""));  // whole 16-byte copies
   if (vd.size() % 2) vd.push_back(make_uint2(0, 0));
-  // binned splits in processing order: levels min(D,8)-1 .. 0, then D-1 .. 8
-  std::vector<uint2> bs((size_t)T * D);
-  for (int t = 0; t < T; ++t) {
+  // binned splits in processing order: levels min(D,8)-1 .. 0, then D-1 .. 8;
+  // a tree's splits are padded to whole 8-byte units
+  const int DS = 2 * split_units(D, true);
+  std::vector<uint32_t> bs((size_t)T * DS, 0u);  // padding: k = 128, never reached by a bin
+  const int K = info.n_classes;
+  std::vector<int> order;  // class by class (tree t is class t % K)
+  for (int k = 0; k < K; ++k)
+    for (int t = k; t < T; t += K) order.push_back(t);
+  for (int q = 0; q < T; ++q) {
+    const int t = order[q];
     for (int p = 0; p < D; ++p) {
       const int lev = D <= 8 ? D - 1 - p : (p < 8 ? 7 - p : D - 1 - (p - 8));
-      uint2 q = make_uint2(0, 0);  // padding: k = 128, never reached by a bin
-      if (lev < depth[t]) {
-        const float th = threshold[(size_t)t * D + lev];
-        if (!std::isnan(th)) {
-          const int j = feature[(size_t)t * D + lev];
-          const int r = (int)(std::lower_bound(u[j].begin(), u[j].end(), th) - u[j].begin());
-          const int v = first_v[j] + r / BIN_MAX_BORDERS, k = r % BIN_MAX_BORDERS + 1;
-          q = make_uint2((uint32_t)v * PRED_ROWS, (uint32_t)(128 - k) * 0x01010101u);
-        }
-      }
-      bs[(size_t)t * D + p] = q;
+      if (lev >= depth[t]) continue;
+      const float th = threshold[(size_t)t * D + lev];
+      if (std::isnan(th)) continue;
+      const int j = feature[(size_t)t * D + lev];
+      const int r = (int)(std::lower_bound(u[j].begin(), u[j].end(), th) - u[j].begin());
+      const int v = first_v[j] + r / BIN_MAX_BORDERS;
+      bs[(size_t)q * DS + p] = (uint32_t)v << 8 | (uint32_t)(128 - r % BIN_MAX_BORDERS - 1);
     }
   }
-  TC_TRY(d_bsplits.alloc(ctx, std::max<size_t>(1, bs.size()), "binned model splits"));
+  TC_TRY(d_bsplits.alloc(ctx, std::max<size_t>(2, bs.size()), "binned model splits"));
+  if (K > 1) {
+    std::vector<float> bl(lv.size());
+    for (int q = 0; q < T; ++q) std::memcpy(&bl[(size_t)q * L], &lv[(size_t)order[q] * L], L * sizeof(float));
+    TC_TRY(d_bleaves.alloc(ctx, bl.size(), "binned model leaves"));
+    TC_CUDA(ctx, cudaMemcpy(d_bleaves.p, bl.data(), bl.size() * sizeof(float), cudaMemcpyHostToDevice));
+  }
   TC_TRY(d_bord.alloc(ctx, bord.size(), "model borders"));
   TC_TRY(d_vdesc.alloc(ctx, vd.size(), "model virtual features"));
   if (!bs.empty())
-    TC_CUDA(ctx, cudaMemcpy(d_bsplits.p, bs.data(), bs.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+    TC_CUDA(ctx, cudaMemcpy(d_bsplits.p, bs.data(), bs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
   TC_CUDA(ctx, cudaMemcpy(d_bord.p, bord.data(), bord.size() * sizeof(float), cudaMemcpyHostToDevice));
   TC_CUDA(ctx, cudaMemcpy(d_vdesc.p, vd.data(), vd.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  bin_stride = stride;
   n_virtual = V;
   n_bord = B;
   return TC_OK;
@@ -1046,10 +1167,12 @@ ModelDesc model_desc(const tc_model* m) {
   d.splits = m->d_splits.p;
   d.leaves = m->d_leaves.p;
   d.bsplits = m->d_bsplits.p;
+  d.bleaves = m->d_bleaves.p ? m->d_bleaves.p : m->d_leaves.p;
   d.bord = m->d_bord.p;
   d.vdesc = m->d_vdesc.p;
   d.n_virtual = m->n_virtual;
   d.n_bord = m->n_bord;
+  d.bin_stride = m->bin_stride;
   d.n_trees = m->info.n_trees;
   d.max_depth = m->info.max_depth;
   d.n_classes = m->info.n_classes;
@@ -1091,7 +1214,9 @@ tc_status predict_device(tc_ctx* ctx, const tc_model* m, const float* X, uint32_
   jt.n_jobs = 1;
   jt.one_model = model_desc(m);
   jt.one_req = ReqDesc{X, out, n, 0, 0, transform};
-  return launch_predict(ctx, jt, predict_plan(&m, 1), predict_tiles(n), stream);
+  const PredictPlan plan = predict_plan(&m, 1);
+  const int rows = predict_tile_rows(ctx, plan, predict_tiles(n, PRED_HALF));
+  return launch_predict(ctx, jt, plan, rows, predict_tiles(n, rows), stream);
 }
 
 }  // namespace tc

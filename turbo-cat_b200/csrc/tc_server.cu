@@ -103,6 +103,9 @@ static bool is_pinned(const void* p) {
 bool tc_server::launch(Slot& s, std::vector<Request*>& batch) {
   uint32_t row = 0, tile = 0;
   int j = 0;
+  uint64_t half_tiles = 0;
+  for (Request* r : batch) half_tiles += predict_tiles(r->n, 128);
+  const int tile_rows = predict_tile_rows(ctx, plan, half_tiles);
   for (Request* r : batch) {
     float* din = s.d_in.p + (size_t)row * max_f;
     const size_t bytes = (size_t)r->n * r->f * sizeof(float);
@@ -114,14 +117,14 @@ bool tc_server::launch(Slot& s, std::vector<Request*>& batch) {
     }
     s.h_reqs[j] = ReqDesc{din, s.d_out.p + (size_t)row * 16, r->n, row, r->model, r->transform};
     s.h_tiles[j] = tile;
-    tile += predict_tiles(r->n);
+    tile += predict_tiles(r->n, tile_rows);
     row += r->n;
     ++j;
   }
   s.h_tiles[j] = tile;
   cudaMemcpyAsync(s.d_reqs.p, s.h_reqs, j * sizeof(ReqDesc), cudaMemcpyHostToDevice, s.stream);
   cudaMemcpyAsync(s.d_tiles.p, s.h_tiles, (j + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s.stream);
-  if (predict_batched(ctx, d_models.p, s.d_reqs.p, j, s.d_tiles.p, tile, plan, s.stream) != TC_OK)
+  if (predict_batched(ctx, d_models.p, s.d_reqs.p, j, s.d_tiles.p, tile_rows, tile, plan, s.stream) != TC_OK)
     return false;
   for (int q = 0; q < j; ++q) {
     Request* r = batch[q];
