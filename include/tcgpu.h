@@ -70,7 +70,10 @@ tc_status tc_ctx_create(int device, size_t mem_budget, tc_ctx** out);
 void tc_ctx_destroy(tc_ctx* ctx);
 /* Message of the last failed call on this context (never NULL). */
 const char* tc_last_error(const tc_ctx* ctx);
-/* Bytes currently allocated by the context and its objects, and the peak. */
+/* Bytes currently allocated by the context and its objects, and the peak.
+ * Buffers that a destroyed object gave back and the context keeps for its next
+ * one (at most 4 GiB; they count against the budget and are given back to the
+ * device when an allocation needs the room) are not among them. */
 tc_status tc_ctx_memory(const tc_ctx* ctx, size_t* in_use, size_t* peak);
 /* Fault-injection hook for host-side tests: the next `count` device
  * allocations made through this context fail with TC_ERR_OOM. */

@@ -4,7 +4,8 @@
 
 #include "tc_internal.h"
 
-tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what) {
+tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
+  bool trim = false;
   {
     std::lock_guard<std::mutex> g(mu);
     if (fail_next > 0) {
@@ -19,8 +20,29 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what) {
       err = buf;
       return TC_ERR_OOM;
     }
+    if (pooled) {
+      // the smallest kept block that holds `bytes` with at most a quarter to spare
+      const auto it = pool.lower_bound(bytes);
+      if (it != pool.end() && it->first <= bytes + bytes / 4 + 4096 && (!budget || in_use + it->first <= budget)) {
+        *p = it->second;
+        const size_t size = it->first;
+        pool_bytes -= size;
+        pool.erase(it);
+        allocs[*p] = size;
+        in_use += size;
+        if (in_use > peak) peak = in_use;
+        return TC_OK;
+      }
+    }
+    trim = budget && pool_bytes && in_use + pool_bytes + bytes > budget;
   }
+  if (trim) trim_pool();
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pool();
+    e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(TC_ERR_OOM, "cudaMalloc(%zu) for %s: %s", bytes, what, cudaGetErrorString(e));
@@ -32,19 +54,37 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what) {
   return TC_OK;
 }
 
-void tc_ctx::release(void* p) {
+void tc_ctx::release(void* p, bool pooled) {
   if (!p) return;
-  size_t bytes = 0;
+  // a kept block may go to work on another stream (or a synchronous call) next:
+  // wait for what the context's stream still does with it, as cudaFree would
+  const bool idle = pooled && cudaStreamSynchronize(stream) == cudaSuccess;
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = allocs.find(p);
     if (it != allocs.end()) {
-      bytes = it->second;
+      const size_t bytes = it->second;
       allocs.erase(it);
       in_use -= bytes;
+      if (idle && bytes <= tc::kPoolBlockMax && pool_bytes + bytes <= tc::kPoolMax &&
+          (!budget || in_use + pool_bytes + bytes <= budget)) {
+        pool.emplace(bytes, p);
+        pool_bytes += bytes;
+        return;
+      }
     }
   }
   cudaFree(p);
+}
+
+void tc_ctx::trim_pool() {
+  std::multimap<size_t, void*> blocks;
+  {
+    std::lock_guard<std::mutex> g(mu);
+    blocks.swap(pool);
+    pool_bytes = 0;
+  }
+  for (auto& kv : blocks) cudaFree(kv.second);
 }
 
 extern "C" {
@@ -88,6 +128,7 @@ void tc_ctx_destroy(tc_ctx* ctx) {
   }
   cudaStreamSynchronize(ctx->stream);
   cudaStreamSynchronize(ctx->pred_stream);
+  ctx->trim_pool();
   for (auto& kv : ctx->allocs) cudaFree(kv.first);
   ctx->allocs.clear();
   if (ctx->pin_io) cudaFreeHost(ctx->pin_io);

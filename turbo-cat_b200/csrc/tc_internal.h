@@ -82,9 +82,25 @@ struct tc_ctx {
     return fail(TC_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
   }
   // Device allocation with budget accounting and test fault injection.
-  tc_status alloc(void** p, size_t bytes, const char* what);
-  void release(void* p);
+  // `pooled` memory is used by work on `stream` only (and by synchronous calls);
+  // release waits for that stream and keeps the block for the next pooled
+  // allocation of about its size, so that a fit, a binning or an encoding does
+  // not map and unmap its buffers every time (1M x 100: tc_quantize 10.7 -> 7.0
+  // ms, a 20-tree regression fit 23.8 -> 14.7 ms; 1M x 20 with four categorical
+  // columns, upload to binning 13.5 -> 4.3 ms; the calls' spread went with it).  At most kPoolMax bytes in
+  // blocks of at most kPoolBlockMax are kept, all of them are given back when an
+  // allocation fails or would pass the budget, and with the context.
+  tc_status alloc(void** p, size_t bytes, const char* what, bool pooled = false);
+  void release(void* p, bool pooled = false);
+  void trim_pool();                         // gives every kept block back to the device
+  std::multimap<size_t, void*> pool;        // kept blocks by size (guarded by mu)
+  size_t pool_bytes = 0;
 };
+
+namespace tc {
+constexpr size_t kPoolMax = (size_t)4 << 30;
+constexpr size_t kPoolBlockMax = (size_t)1 << 30;
+}  // namespace tc
 
 #define TC_CUDA(ctx, call)                                         \
   do {                                                             \
@@ -98,8 +114,10 @@ struct tc_ctx {
     if (s_ != TC_OK) return s_;         \
   } while (0)
 
-// A device buffer owned by a context.
-template <class T>
+// A device buffer owned by a context.  Pooled buffers are touched by work on
+// the context's stream and by synchronous calls only; buffers of models and
+// servers, which kernels on any stream read, are not pooled (AnyStreamBuf).
+template <class T, bool Pooled = true>
 struct DevBuf {
   tc_ctx* ctx = nullptr;
   T* p = nullptr;
@@ -112,19 +130,21 @@ struct DevBuf {
     reset();
     ctx = c;
     void* q = nullptr;
-    tc_status s = c->alloc(&q, count * sizeof(T) > 0 ? count * sizeof(T) : 16, what);
+    tc_status s = c->alloc(&q, count * sizeof(T) > 0 ? count * sizeof(T) : 16, what, Pooled);
     if (s != TC_OK) return s;
     p = static_cast<T*>(q);
     n = count;
     return TC_OK;
   }
   void reset() {
-    if (p && ctx) ctx->release(p);
+    if (p && ctx) ctx->release(p, Pooled);
     p = nullptr;
     n = 0;
   }
   size_t bytes() const { return n * sizeof(T); }
 };
+template <class T>
+using AnyStreamBuf = DevBuf<T, false>;
 
 struct tc_dataset {
   tc_ctx* ctx = nullptr;
@@ -182,23 +202,23 @@ struct tc_model {
   std::vector<float> edges;         // [f][255]
   std::vector<uint16_t> n_edges;    // [f]
   // device copies used by the predict kernels
-  DevBuf<uint2> d_splits;           // [T][D] (feature, threshold bits), padded to depth D
-  DevBuf<float> d_leaves;           // [T][2^D] (weights folded in, padded trees' leaves spread)
-  DevBuf<uint32_t> d_bsplits;       // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class
-  DevBuf<float> d_bleaves;          // binned form, several classes: leaves in the order of d_bsplits
-  DevBuf<float> d_bord;             // binned form: borders of every virtual feature, Eytzinger order
-  DevBuf<uint2> d_vdesc;            // binned form: (feature, border offset | search steps << 24)
+  AnyStreamBuf<uint2> d_splits;           // [T][D] (feature, threshold bits), padded to depth D
+  AnyStreamBuf<float> d_leaves;           // [T][2^D] (weights folded in, padded trees' leaves spread)
+  AnyStreamBuf<uint32_t> d_bsplits;       // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class
+  AnyStreamBuf<float> d_bleaves;          // binned form, several classes: leaves in the order of d_bsplits
+  AnyStreamBuf<float> d_bord;             // binned form: borders of every virtual feature, Eytzinger order
+  AnyStreamBuf<uint2> d_vdesc;            // binned form: (feature, border offset | search steps << 24)
   int n_virtual = 0, n_bord = 0;
   int bin_stride = 0;               // bytes of a bin column: 256 or 128 rows (0: no binned form)
   // regular (depth-wise) trees of a model the reference trained with
   // mode="small" (served for prediction only; tc_predict.cu)
   bool regular = false;
   std::vector<uint8_t> tcat;        // the stream as loaded (saved back byte for byte)
-  DevBuf<uint4> d_rnodes;           // (feature | bin << 16 | leaf << 24, left, right, value bits), global indices
-  DevBuf<uint32_t> d_rroots;        // [T] first node of each tree
-  DevBuf<float> d_rweights;         // [T]
-  DevBuf<float> d_redges;           // [f][255] bin edges
-  DevBuf<int32_t> d_rnedges;        // [f]
+  AnyStreamBuf<uint4> d_rnodes;           // (feature | bin << 16 | leaf << 24, left, right, value bits), global indices
+  AnyStreamBuf<uint32_t> d_rroots;        // [T] first node of each tree
+  AnyStreamBuf<float> d_rweights;         // [T]
+  AnyStreamBuf<float> d_redges;           // [f][255] bin edges
+  AnyStreamBuf<int32_t> d_rnedges;        // [f]
   tc_status upload();
 };
 

@@ -49,10 +49,10 @@ struct Request {
 struct Slot {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
-  DevBuf<float> d_in;        // [rows_cap][max_f]
-  DevBuf<float> d_out;       // [rows_cap][16]
-  DevBuf<ReqDesc> d_reqs;    // [req_cap]
-  DevBuf<uint32_t> d_tiles;  // [req_cap + 1]
+  AnyStreamBuf<float> d_in;        // [rows_cap][max_f]
+  AnyStreamBuf<float> d_out;       // [rows_cap][16]
+  AnyStreamBuf<ReqDesc> d_reqs;    // [req_cap]
+  AnyStreamBuf<uint32_t> d_tiles;  // [req_cap + 1]
   float* h_in = nullptr;     // pinned staging for pageable inputs
   float* h_out = nullptr;    // pinned staging for pageable outputs
   ReqDesc* h_reqs = nullptr;
@@ -74,7 +74,7 @@ struct tc_server {
   std::vector<std::unique_ptr<Slot>> slots;
   std::vector<ModelDesc> models;
   std::vector<const tc_model*> model_ptrs;
-  DevBuf<ModelDesc> d_models;
+  AnyStreamBuf<ModelDesc> d_models;
   std::mutex mu;
   std::condition_variable cv_work;   // worker wake-up
   std::condition_variable cv_done;   // completion notifications
