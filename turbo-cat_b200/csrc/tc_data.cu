@@ -46,142 +46,274 @@ __device__ __forceinline__ float key_float(uint32_t k) {
   return __uint_as_float(u);
 }
 
-// X [n][f] row-major -> keys [f][n] via 32x32 shared-memory tiles.
-__global__ void k_make_keys(const float* __restrict__ X, uint32_t n, uint32_t f,
-                            uint32_t* __restrict__ keys) {
-  __shared__ uint32_t t[32][33];
-  const uint32_t r0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t r = r0 + i, c = c0 + threadIdx.x;
-    if (r < n && c < f) t[i][threadIdx.x] = float_key(X[(size_t)r * f + c]);
+// X [n][f] row-major -> keys [f][n] via shared-memory tiles of 128 rows x 32
+// features, 16 loads of a thread in flight (32 x 32 tiles with four: 390 us on
+// 100M values, 320 here).
+constexpr int MK_ROWS = 128;
+__global__ void __launch_bounds__(256) k_make_keys(const float* __restrict__ X, uint32_t n, uint32_t f,
+                                                   uint32_t* __restrict__ keys) {
+  __shared__ uint32_t t[MK_ROWS][33];
+  const uint32_t r0 = blockIdx.x * MK_ROWS, c0 = blockIdx.y * 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float v[MK_ROWS / 8];
+#pragma unroll
+  for (int i = 0; i < MK_ROWS / 8; ++i) {
+    const uint32_t r = r0 + warp + 8 * i, c = c0 + lane;
+    v[i] = r < n && c < f ? X[(size_t)r * f + c] : 0.0f;
   }
+#pragma unroll
+  for (int i = 0; i < MK_ROWS / 8; ++i) t[warp + 8 * i][lane] = float_key(v[i]);
   __syncthreads();
-  for (int i = threadIdx.y; i < 32; i += blockDim.y) {
-    const uint32_t c = c0 + i, r = r0 + threadIdx.x;
-    if (r < n && c < f) keys[(size_t)c * n + r] = t[threadIdx.x][i];
+#pragma unroll
+  for (int i = 0; i < MK_ROWS / 8; ++i) {
+    const uint32_t c = c0 + warp + 8 * (i & 3), q = 32 * (i >> 2) + lane, r = r0 + q;
+    if (r < n && c < f) keys[(size_t)c * n + r] = t[q][warp + 8 * (i & 3)];
   }
 }
 
-__global__ void k_radix_count(const uint32_t* __restrict__ keys, uint32_t n, uint32_t n_tiles,
-                              int shift, uint32_t* __restrict__ counts) {
+// counts[j][digit][tile] of one radix pass (all of a thread's loads in flight:
+// 186 us on 100M keys with a load per iteration, 82 here).
+__global__ void __launch_bounds__(RS_THREADS) k_radix_count(const uint32_t* __restrict__ keys, uint32_t n,
+                                                            uint32_t n_tiles, int shift,
+                                                            uint32_t* __restrict__ counts) {
   __shared__ uint32_t h[256];
   const uint32_t j = blockIdx.y, tile = blockIdx.x;
+  const uint32_t* kj = keys + (size_t)j * n + tile * RS_TILE;
+  const uint32_t cnt = min((uint32_t)RS_TILE, n - tile * RS_TILE);
+  uint32_t k[RS_ITEMS];
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t q = i * RS_THREADS + threadIdx.x;
+    k[i] = q < cnt ? kj[q] : 0u;
+  }
   h[threadIdx.x] = 0;
   __syncthreads();
-  const uint32_t* kj = keys + (size_t)j * n;
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    const uint32_t idx = tile * RS_TILE + it * RS_THREADS + threadIdx.x;
-    if (idx < n) atomicAdd(&h[(kj[idx] >> shift) & 255u], 1u);
-  }
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i)
+    if (i * RS_THREADS + threadIdx.x < cnt) atomicAdd(&h[(k[i] >> shift) & 255u], 1u);
   __syncthreads();
   counts[((size_t)j * 256 + threadIdx.x) * n_tiles + tile] = h[threadIdx.x];
 }
 
+// Exclusive scan over the tiles of each digit of each column, in place, and the
+// digit totals: a warp per (column, digit).  (One block per column over all
+// digits took 40-50 us at 1M rows, a serial chain of block-wide rounds.)
+__global__ void __launch_bounds__(256) k_digit_scan(uint32_t* __restrict__ counts, uint32_t n_tiles,
+                                                    uint32_t* __restrict__ totals) {
+  const uint32_t jd = blockIdx.x * 8 + (threadIdx.x >> 5);  // column * 256 + digit
+  const int lane = threadIdx.x & 31;
+  uint32_t* s = counts + (size_t)jd * n_tiles;
+  uint32_t carry = 0;
+  for (uint32_t base = 0; base < n_tiles; base += 32 * 8) {
+    uint32_t v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const uint32_t i = base + 32 * q + lane;
+      v[q] = i < n_tiles ? s[i] : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      uint32_t x = v[q];
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      const uint32_t i = base + 32 * q + lane;
+      if (i < n_tiles) s[i] = carry + x - v[q];
+      carry += __shfl_sync(0xffffffffu, x, 31);
+    }
+  }
+  if (lane == 0) totals[jd] = carry;
+}
+
 // Exclusive scan, in place, of each segment a[j*m .. j*m+m); totals[j] = sum.
-__global__ void k_segment_scan(uint32_t* __restrict__ a, uint32_t m, uint32_t* __restrict__ totals) {
-  __shared__ uint32_t warp_sums[32];
-  __shared__ uint32_t carry_s;
+// A block per segment, SCAN_PER consecutive entries per thread and round, one
+// barrier a round.
+constexpr int SCAN_PER = 8;
+__global__ void __launch_bounds__(1024) k_segment_scan(uint32_t* __restrict__ a, uint32_t m, uint32_t* __restrict__ totals) {
+  __shared__ uint32_t warp_sums[2][32];
   uint32_t* s = a + (size_t)blockIdx.x * m;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  if (threadIdx.x == 0) carry_s = 0;
-  __syncthreads();
-  for (uint32_t base = 0; base < m; base += blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < m ? s[i] : 0u;
-    uint32_t x = v;
+  uint32_t carry = 0;
+  int ph = 0;
+  for (uint32_t base = 0; base < m; base += blockDim.x * SCAN_PER, ph ^= 1) {
+    const uint32_t i0 = base + threadIdx.x * SCAN_PER;
+    uint32_t v[SCAN_PER], sum = 0;
+#pragma unroll
+    for (int q = 0; q < SCAN_PER; ++q) {
+      v[q] = i0 + q < m ? s[i0 + q] : 0u;
+      sum += v[q];
+    }
+    uint32_t x = sum;
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-      uint32_t w = lane < nw ? warp_sums[lane] : 0u;
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
-      }
-      if (lane < nw) warp_sums[lane] = w;  // inclusive
+    if (lane == 31) warp_sums[ph][warp] = x;
+    __syncthreads();  // (the other half is read by the round before only)
+    uint32_t before = 0, all = 0;
+    {
+      const uint32_t w = lane < nw ? warp_sums[ph][lane] : 0u;
+      before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+      all = __reduce_add_sync(0xffffffffu, w);
     }
-    __syncthreads();
-    const uint32_t carry = carry_s;
-    const uint32_t excl = carry + (warp ? warp_sums[warp - 1] : 0u) + x - v;
-    if (i < m) s[i] = excl;
-    __syncthreads();
-    if (threadIdx.x == 0) carry_s = carry + warp_sums[nw - 1];
-    __syncthreads();
+    uint32_t run = carry + before + x - sum;
+#pragma unroll
+    for (int q = 0; q < SCAN_PER; ++q) {
+      if (i0 + q < m) s[i0 + q] = run;
+      run += v[q];
+    }
+    carry += all;
   }
-  if (threadIdx.x == 0 && totals) totals[blockIdx.x] = carry_s;
+  if (threadIdx.x == 0 && totals) totals[blockIdx.x] = carry;
 }
 
-// Stable scatter of one radix pass.  Keys of a tile are visited in index
-// order (round-major, then thread order); a key's slot is its digit's global
-// offset for the tile + the count of equal digits before it in the tile.
-__global__ void k_radix_scatter(const uint32_t* __restrict__ kin, uint32_t* __restrict__ kout,
-                                uint32_t n, uint32_t n_tiles, int shift,
-                                const uint32_t* __restrict__ offsets,
-                                const uint32_t* __restrict__ vin = nullptr, uint32_t* __restrict__ vout = nullptr) {
-  __shared__ uint32_t s_base[256];
-  __shared__ uint32_t s_run[256];
-  __shared__ uint32_t s_w[RS_THREADS / 32][256];
+// Stable scatter of one radix pass over tiles of 4096 keys: warp w takes keys
+// [512 w, 512 w + 512) of the tile, 32 at a time, so a tile's keys are in index
+// order warp by warp.  A key's place among its tile's equal digits is its
+// warp's count of the digit so far plus the equal digits of lower lanes
+// (registers and a warp's own counters: no block barrier per 32 keys); the
+// tile is then put in digit order in shared memory and written out from
+// there, so a digit's run is one contiguous write.  What bounds it: the ranking's
+// instructions (eight ballots a key; the match instruction instead was 130 us
+// slower), then memory: 100M keys a pass 790 us with the scatter straight from
+// registers and four barriers per 256 keys, 460 here (1.7 TB/s).
+template <bool VALS>
+__global__ void __launch_bounds__(RS_THREADS) k_radix_scatter(const uint32_t* __restrict__ kin,
+                                                              uint32_t* __restrict__ kout, uint32_t n,
+                                                              uint32_t n_tiles, int shift,
+                                                              const uint32_t* __restrict__ offsets,
+                                                              const uint32_t* __restrict__ totals,
+                                                              const uint32_t* __restrict__ vin,
+                                                              uint32_t* __restrict__ vout) {
+  constexpr int NW = RS_THREADS / 32;
+  __shared__ uint32_t s_key[RS_TILE];
+  __shared__ uint32_t s_val[VALS ? RS_TILE : 1];
+  __shared__ uint16_t s_cnt[NW][256];  // the warps' digit counts, then their starts in the tile's order
+  __shared__ uint32_t s_goff[256];     // a digit's global offset minus its start in the tile's order
+  __shared__ uint32_t s_sum[NW], s_tot[NW];
   const uint32_t j = blockIdx.y, tile = blockIdx.x;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  s_base[tid] = offsets[((size_t)j * 256 + tid) * n_tiles + tile];
-  s_run[tid] = 0;
-  for (int w = 0; w < RS_THREADS / 32; ++w) s_w[w][tid] = 0;
+  const uint32_t tbase = tile * RS_TILE, cnt = min((uint32_t)RS_TILE, n - tbase);
+  // digit tid: its keys of the tiles before, and its keys in all
+  const uint32_t goff = offsets[((size_t)j * 256 + tid) * n_tiles + tile];
+  const uint32_t total = totals[(size_t)j * 256 + tid];
+  const uint32_t* ki = kin + (size_t)j * n + tbase;
+  uint32_t key[RS_ITEMS], val[VALS ? RS_ITEMS : 1];
+  uint16_t rank[RS_ITEMS];
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t q = warp * (32 * RS_ITEMS) + i * 32 + lane;
+    key[i] = q < cnt ? ki[q] : 0xffffffffu;  // past the end: last of the tile
+    if (VALS) val[i] = q < cnt ? vin[(size_t)j * n + tbase + q] : 0u;
+  }
+#pragma unroll
+  for (int w = 0; w < NW; ++w) s_cnt[w][tid] = 0;
   __syncthreads();
-  const uint32_t* ki = kin + (size_t)j * n;
-  uint32_t* ko = kout + (size_t)j * n;
   const uint32_t lt = (1u << lane) - 1u;
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    const uint32_t idx = tile * RS_TILE + it * RS_THREADS + tid;
-    const bool valid = idx < n;
-    const uint32_t key = valid ? ki[idx] : 0u;
-    const uint32_t d = valid ? ((key >> shift) & 255u) : 256u;
-    const uint32_t mask = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank = __popc(mask & lt);
-    if (valid && rank == 0) s_w[warp][d] = __popc(mask);
-    __syncthreads();
-    {
-      uint32_t run = s_run[tid];
-      for (int w = 0; w < RS_THREADS / 32; ++w) {
-        const uint32_t c = s_w[w][tid];
-        s_w[w][tid] = run;
-        run += c;
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t d = (key[i] >> shift) & 255u;
+    uint32_t m = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const uint32_t v = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+      m &= ((d >> b) & 1u) ? v : ~v;
+    }
+    const uint32_t before = s_cnt[warp][d];
+    rank[i] = (uint16_t)(before + __popc(m & lt));
+    __syncwarp();
+    if ((m & lt) == 0) s_cnt[warp][d] = (uint16_t)(before + __popc(m));
+    __syncwarp();
+  }
+  __syncthreads();
+  {
+    // digit tid: the warps' starts, and the digit's start in the tile's order
+    uint32_t run = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) run += s_cnt[w][tid];
+    uint32_t x = run, g = total;
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o), z = __shfl_up_sync(0xffffffffu, g, o);
+      if (lane >= o) {
+        x += y;
+        g += z;
       }
-      s_run[tid] = run;
+    }
+    if (lane == 31) {
+      s_sum[warp] = x;
+      s_tot[warp] = g;
     }
     __syncthreads();
-    if (valid) {
-      const uint32_t slot = s_base[d] + s_w[warp][d] + rank;
-      ko[slot] = key;
-      if (vout) vout[(size_t)j * n + slot] = vin[(size_t)j * n + idx];  // payload rides along
+    uint32_t start = x - run, gbase = g - total;
+    for (int w = 0; w < warp; ++w) {
+      start += s_sum[w];
+      gbase += s_tot[w];
     }
-    __syncthreads();
-    for (int w = 0; w < RS_THREADS / 32; ++w) s_w[w][tid] = 0;
-    __syncthreads();
+    s_goff[tid] = gbase + goff - start;
+    for (int w = 0; w < NW; ++w) {
+      const uint32_t c = s_cnt[w][tid];
+      s_cnt[w][tid] = (uint16_t)start;
+      start += c;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t at = s_cnt[warp][(key[i] >> shift) & 255u] + rank[i];
+    s_key[at] = key[i];
+    if (VALS) s_val[at] = val[i];
+  }
+  __syncthreads();
+  uint32_t* ko = kout + (size_t)j * n;
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t q = i * RS_THREADS + tid;
+    if (q < cnt) {  // (the keys past the end took the last places)
+      const uint32_t k = s_key[q];
+      const uint32_t at = s_goff[(k >> shift) & 255u] + q;
+      ko[at] = k;
+      if (VALS) vout[(size_t)j * n + at] = s_val[q];
+    }
   }
 }
 
-__device__ __forceinline__ bool uniq_flag(const uint32_t* kj, uint32_t idx, uint32_t n) {
-  if (idx >= n) return false;
-  const uint32_t k = kj[idx];
-  return k != NAN_KEY && (idx == 0 || kj[idx - 1] != k);
+// First occurrences (not NaN) among a warp's 32 * RS_ITEMS consecutive sorted
+// keys from k0: key[i] is key k0 + 32 i + lane, the result its bit masks.  The
+// key before comes from the lane below, so every key is loaded once and all
+// loads are in flight.
+__device__ __forceinline__ void first_masks(const uint32_t* kj, uint32_t k0, uint32_t n, uint32_t (&key)[RS_ITEMS],
+                                            uint32_t (&mask)[RS_ITEMS]) {
+  const int lane = threadIdx.x & 31;
+  uint32_t prev = 0;  // lane 31: the key before the group
+  if (lane == 31 && k0 > 0 && k0 - 1 < n) prev = kj[k0 - 1];
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) key[i] = k0 + 32 * i + lane < n ? kj[k0 + 32 * i + lane] : NAN_KEY;
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    const uint32_t below = __shfl_sync(0xffffffffu, lane == 31 ? prev : key[i], (lane + 31) & 31);
+    const bool first = key[i] != NAN_KEY && (k0 + 32 * i + lane == 0 || below != key[i]);
+    mask[i] = __ballot_sync(0xffffffffu, first);
+    prev = key[i];
+  }
 }
 
-__global__ void k_unique_count(const uint32_t* __restrict__ keys, uint32_t n, uint32_t n_tiles,
-                               uint32_t* __restrict__ tile_cnt) {
-  __shared__ uint32_t s;
-  if (threadIdx.x == 0) s = 0;
-  __syncthreads();
+__global__ void __launch_bounds__(RS_THREADS) k_unique_count(const uint32_t* __restrict__ keys, uint32_t n,
+                                                             uint32_t n_tiles, uint32_t* __restrict__ tile_cnt) {
+  __shared__ uint32_t s[RS_THREADS / 32];
   const uint32_t j = blockIdx.y, tile = blockIdx.x;
-  const uint32_t* kj = keys + (size_t)j * n;
-  uint32_t c = 0;
-  for (int it = 0; it < RS_ITEMS; ++it) c += uniq_flag(kj, tile * RS_TILE + it * RS_THREADS + threadIdx.x, n);
-  for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(&s, c);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t key[RS_ITEMS], mask[RS_ITEMS], c = 0;
+  first_masks(keys + (size_t)j * n, tile * RS_TILE + warp * (32 * RS_ITEMS), n, key, mask);
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) c += __popc(mask[i]);
+  if (lane == 0) s[warp] = c;
   __syncthreads();
-  if (threadIdx.x == 0) tile_cnt[(size_t)j * n_tiles + tile] = s;
+  if (threadIdx.x == 0) {
+    c = 0;
+    for (int w = 0; w < RS_THREADS / 32; ++w) c += s[w];
+    tile_cnt[(size_t)j * n_tiles + tile] = c;
+  }
 }
 
 __device__ __forceinline__ uint32_t actual_bins(uint32_t U, int max_bins, int compat_u8) {
@@ -189,13 +321,17 @@ __device__ __forceinline__ uint32_t actual_bins(uint32_t U, int max_bins, int co
   return a < (uint32_t)max_bins ? a : (uint32_t)max_bins;
 }
 
-// Picks edge b-1 = distinct value of rank floor(b*U/A) for b = 1 .. A-1.
-__global__ void k_unique_pick(const uint32_t* __restrict__ keys, uint32_t n, uint32_t n_tiles,
+// Picks edge b-1 = distinct value of rank floor(b*U/A) for b = 1 .. A-1: the
+// ranks that fall into the block's tile are marked in a table over the tile's
+// distinct values (a division per edge; one per key made this 570 us on 100M
+// keys, 186 here), then every first occurrence looks its rank up.
+__global__ void __launch_bounds__(RS_THREADS) k_unique_pick(const uint32_t* __restrict__ keys, uint32_t n, uint32_t n_tiles,
                               const uint32_t* __restrict__ tile_off, const uint32_t* __restrict__ U_,
                               int max_bins, int compat_u8, const uint8_t* __restrict__ ts,
                               float* __restrict__ edges) {
-  __shared__ uint32_t warp_sums[RS_THREADS / 32];
-  __shared__ uint32_t run_s;
+  __shared__ uint16_t s_edge[RS_TILE];  // b of the tile's q-th distinct value, 0: no edge
+  __shared__ uint32_t s_warp[RS_THREADS / 32];
+  __shared__ int s_any;
   const uint32_t j = blockIdx.y, tile = blockIdx.x;
   const uint32_t* kj = keys + (size_t)j * n;
   const uint64_t U = U_[j];
@@ -203,35 +339,38 @@ __global__ void k_unique_pick(const uint32_t* __restrict__ keys, uint32_t n, uin
   // edge b-1 = rank floor(b*U/(A+1)), b = 1 .. A (src/core/dataset.cpp:221-224)
   const uint64_t A = actual_bins((uint32_t)U, max_bins, compat_u8) + (ts && ts[j] ? 1 : 0);
   if (A < 2) return;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) run_s = tile_off[(size_t)j * n_tiles + tile];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t first = tile_off[(size_t)j * n_tiles + tile];
+  if (tid == 0) s_any = 0;
+  for (int q = tid; q < RS_TILE / 2; q += RS_THREADS) reinterpret_cast<uint32_t*>(s_edge)[q] = 0u;
   __syncthreads();
-  for (int it = 0; it < RS_ITEMS; ++it) {
-    const uint32_t idx = tile * RS_TILE + it * RS_THREADS + threadIdx.x;
-    const uint32_t fl = uniq_flag(kj, idx, n);
-    uint32_t x = fl;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+  for (uint64_t b = 1 + tid; b < A; b += RS_THREADS) {  // ranks grow with b, no two alike
+    const uint64_t r = b * U / A;
+    if (r >= first && r - first < RS_TILE) {
+      s_edge[r - first] = (uint16_t)b;
+      s_any = 1;
     }
-    if (lane == 31) warp_sums[warp] = x;
-    __syncthreads();
-    uint32_t before = run_s;
-    for (int w = 0; w < warp; ++w) before += warp_sums[w];
-    if (fl) {
-      const uint64_t r = before + x - 1;  // distinct-value rank
-      // the smallest b with floor(b*U/A) >= r; b >= 1 (with A > U, as the
-      // target-statistics rule has for A = U, rank 0 is edge 0)
-      const uint64_t b = max((r * A + U - 1) / U, (uint64_t)1);
-      if (b >= 1 && b <= A - 1 && (b * U) / A == r) edges[(size_t)j * kSlots + (b - 1)] = key_float(kj[idx]);
+  }
+  __syncthreads();
+  if (!s_any) return;
+  // warp w: keys [512 w, 512 w + 512) of the tile
+  const uint32_t k0 = tile * RS_TILE + warp * (32 * RS_ITEMS);
+  uint32_t key[RS_ITEMS], mask[RS_ITEMS], mine = 0;
+  first_masks(kj, k0, n, key, mask);
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) mine += __popc(mask[i]);
+  if (lane == 0) s_warp[warp] = mine;
+  __syncthreads();
+  uint32_t run = 0;
+  for (int w = 0; w < warp; ++w) run += s_warp[w];
+  const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+  for (int i = 0; i < RS_ITEMS; ++i) {
+    if ((mask[i] >> lane) & 1u) {
+      const uint32_t b = s_edge[run + __popc(mask[i] & lt)];
+      if (b) edges[(size_t)j * kSlots + (b - 1)] = key_float(key[i]);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      uint32_t t = 0;
-      for (int w = 0; w < RS_THREADS / 32; ++w) t += warp_sums[w];
-      run_s += t;
-    }
-    __syncthreads();
+    run += __popc(mask[i]);
   }
 }
 
@@ -250,73 +389,128 @@ __global__ void k_edge_meta(const uint32_t* __restrict__ U_, uint32_t f, int max
   n_edges[j] = (uint16_t)((ts && ts[j]) ? A : (A >= 2 ? A - 1 : 0));
 }
 
-constexpr int AB_ROWS = 256;
+constexpr int AB_THREADS = 256;
+constexpr int AB_MAX_ROWS = 1024;
+
+// The edges of each group of 32 features as k_assign_bins searches them:
+// table[group][slot][feature], slots past a feature's edges NaN.  Grid (8,
+// groups), 32 x 8 threads: 32 slots of a group, turned through shared memory
+// once here instead of with 32-way conflicts in every block of the assignment.
+__global__ void k_edge_table(const float* __restrict__ edges, const uint16_t* __restrict__ n_edges, uint32_t f,
+                             float* __restrict__ table) {
+  __shared__ float t[32][33];
+  const uint32_t j0 = blockIdx.y * 32, e0 = blockIdx.x * 32;
+  for (uint32_t i = threadIdx.y; i < 32; i += 8) {
+    const uint32_t j = j0 + i, e = e0 + threadIdx.x;
+    t[i][threadIdx.x] = j < f && e < n_edges[j] ? edges[(size_t)j * kSlots + e] : __int_as_float(0x7fc00000);
+  }
+  __syncthreads();
+  for (uint32_t i = threadIdx.y; i < 32; i += 8)
+    table[((size_t)blockIdx.y * kSlots + e0 + i) * 32 + threadIdx.x] = t[threadIdx.x][i];
+}
 
 // bin = #edges <= x (upper_bound), NaN -> 255; target-statistics columns
 // (ts[j]) take #edges < x (lower_bound, src/core/dataset.cpp:226-235); writes
-// both bin layouts.  Block (row tile, group): 256 rows of the 32 features of
-// group blockIdx.y.
-__global__ void k_assign_bins(const float* __restrict__ X, uint32_t n, uint32_t f,
-                              const float* __restrict__ edges, const uint16_t* __restrict__ n_edges,
-                              const uint8_t* __restrict__ ts,
-                              uint8_t* __restrict__ bins_t, uint64_t gstride, uint32_t nt, uint32_t wlast,
-                              uint8_t* __restrict__ bins_cm, uint32_t np, uint32_t* __restrict__ nan_any) {
-  __shared__ float s_e[32][kSlots + 1];
-  __shared__ int s_ne[32];
-  __shared__ uint8_t s_b[32][AB_ROWS + 4];
-  __shared__ int s_nan[32];
-  __shared__ int s_ts[32];
-  const uint32_t j0 = blockIdx.y * 32, r0 = blockIdx.x * AB_ROWS;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  for (int q = tid; q < 32 * kSlots; q += blockDim.x) {
-    const int jj = q / kSlots, e = q % kSlots;
-    s_e[jj][e] = (j0 + jj < f) ? edges[(size_t)(j0 + jj) * kSlots + e] : 0.0f;
-  }
-  if (tid < 32) {
-    s_ne[tid] = (j0 + tid < f) ? (int)n_edges[j0 + tid] : 0;
-    s_ts[tid] = (ts && j0 + tid < f) ? (int)ts[j0 + tid] : 0;
-    s_nan[tid] = 0;
-  }
-  __syncthreads();
+// both bin layouts.  Block (row tile, group): `rows` rows of the 32 features of
+// group blockIdx.y, lane = feature.  Edges lie [node][feature] in shared memory
+// (a feature = a bank, so no search step conflicts), padded with NaN, which no
+// value reaches; a search is eight halvings of four rows at a time.  A row's
+// bins are 32 consecutive bytes of the group's tile block, written from the
+// lanes; the column-major copy goes through shared memory.
+//
+// What bounds it: the instructions of the searches (about 30 per row and
+// feature).  With [feature][edge] in shared memory, 256 rows per 32 KB of
+// edges and one-byte stores of both layouts: 1.17 ms on 1M x 100, 0.47 here.
+__global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
+    const float* __restrict__ X, uint32_t n, uint32_t f, const float* __restrict__ table,
+    const uint8_t* __restrict__ ts, uint8_t* __restrict__ bins_t,
+    uint64_t gstride, uint32_t nt, uint32_t wlast, uint8_t* __restrict__ bins_cm, uint32_t np,
+    uint32_t* __restrict__ nan_any, int rows) {
+  extern __shared__ __align__(16) float s_ab[];
+  float* s_e = s_ab;                                            // [256][32]
+  uint32_t* s_b = reinterpret_cast<uint32_t*>(s_ab + 256 * 32);  // [32][rows / 4 + 1] four rows' bins a word
+  const int bs = rows / 4 + 1;
+  const uint32_t j0 = blockIdx.y * 32, r0 = blockIdx.x * (uint32_t)rows;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = AB_THREADS / 32;
   const uint32_t j = j0 + lane;
-  for (int i = warp; i < AB_ROWS; i += nw) {
-    const uint32_t r = r0 + i;
-    uint8_t b = 0;
-    if (r < n && j < f) {
-      const float x = X[(size_t)r * f + j];
-      if (isnan(x)) {
-        b = (uint8_t)kNanBin;
-        s_nan[lane] = 1;
-      } else {
-        int lo = 0, hi = s_ne[lane];
-        const bool lower = s_ts[lane] != 0;
-        while (lo < hi) {
-          const int mid = (lo + hi) >> 1;
-          const float e = s_e[lane][mid];
-          if (lower ? (x <= e) : (x < e)) hi = mid; else lo = mid + 1;
-        }
-        b = (uint8_t)lo;
-        if (lo == kNanBin) s_nan[lane] = 1;  // a target-statistics column's top bin shares the NaN slot
-      }
-    }
-    s_b[lane][i] = b;
+  const bool live = j < f;
+  {
+    const float4* src = reinterpret_cast<const float4*>(table) + (size_t)blockIdx.y * (kSlots * 8);
+    float4* dst = reinterpret_cast<float4*>(s_e);
+#pragma unroll
+    for (int q = 0; q < kSlots * 8 / AB_THREADS; ++q) dst[q * AB_THREADS + tid] = src[q * AB_THREADS + tid];
   }
+  const bool lower = ts && live && ts[j];
+  const bool any_lower = __any_sync(0xffffffffu, lower);
   __syncthreads();
-  if (tid < 32 && s_nan[tid] && j0 + tid < f) atomicOr(&nan_any[j0 + tid], 1u);
-  // column-major rows of this tile
-  for (int q = tid; q < 32 * AB_ROWS; q += blockDim.x) {
-    const int jj = q / AB_ROWS, i = q % AB_ROWS;
-    const uint32_t r = r0 + i;
-    if (j0 + jj < f && r < np) bins_cm[(size_t)(j0 + jj) * np + r] = (r < n) ? s_b[jj][i] : (uint8_t)0;
-  }
-  // the group's tile block: rows r0.. at a stride of the group's width
-  const uint32_t w = (blockIdx.y == gridDim.y - 1) ? wlast : 32u;
+  const uint32_t w = (blockIdx.y == gridDim.y - 1) ? wlast : 32u;  // the group's bytes per row
   uint8_t* blk = bins_t + (uint64_t)blockIdx.y * gstride;
-  for (int q = tid; q < 32 * AB_ROWS; q += blockDim.x) {
-    const int i = q / 32, jj = q % 32;
-    const uint32_t r = r0 + i;
-    if (r < nt && (uint32_t)jj < w) blk[(size_t)r * w + jj] = (r < n && j0 + jj < f) ? s_b[jj][i] : (uint8_t)0;
+  const float* se = s_e + lane;
+  bool nan = false;
+  for (int i = warp * 4; i < rows; i += NW * 4) {
+    float x[4];
+    int pos[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t r = r0 + i + u;
+      x[u] = (live && r < n) ? X[(size_t)r * f + j] : 0.0f;
+      pos[u] = 0;
+    }
+    if (!any_lower) {
+#pragma unroll
+      for (int h = 128; h > 0; h >>= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (se[(pos[u] + h - 1) * 32] <= x[u]) pos[u] += h;
+    } else {
+#pragma unroll
+      for (int h = 128; h > 0; h >>= 1)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float e = se[(pos[u] + h - 1) * 32];
+          if (e < x[u] || (!lower && e == x[u])) pos[u] += h;
+        }
+    }
+    uint32_t four = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t r = r0 + i + u;
+      uint32_t b = (uint32_t)pos[u];
+      if (x[u] != x[u]) b = kNanBin;
+      if (!live || r >= n) b = 0;
+      else if (b == kNanBin) nan = true;  // NaN, or a target-statistics column's top bin, which shares the slot
+      four |= b << (8 * u);
+      if (r < nt && (uint32_t)lane < w) blk[(size_t)r * w + lane] = (uint8_t)b;
+    }
+    s_b[lane * bs + (i >> 2)] = four;
   }
+  if (nan) atomicOr(&nan_any[j], 1u);
+  __syncthreads();
+  // column-major rows of this tile (np is a multiple of 16, r0 of 32)
+  for (int jj = warp; jj < 32 && j0 + jj < f; jj += NW)
+    for (int q = lane; q < rows / 4; q += 32)
+      if (r0 + 4 * q < np)
+        *reinterpret_cast<uint32_t*>(bins_cm + (size_t)(j0 + jj) * np + r0 + 4 * q) = s_b[jj * bs + q];
+}
+
+// Rows per block of k_assign_bins: 1024 amortise the block's 32 KB of edges;
+// fewer while the grid would not give every SM three blocks (50k x 20: 40 us in
+// 196 blocks before, 14 here).
+tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, DevBuf<float>& table, cudaStream_t st) {
+  int rows = AB_MAX_ROWS;
+  while (rows > 64 && (ds->n + rows - 1) / rows * ds->groups < 3u * (uint32_t)ds->ctx->sm_count) rows /= 2;
+  const size_t smem = 256 * 32 * 4 + (size_t)32 * (rows / 4 + 1) * 4;
+  TC_CUDA(ds->ctx, cudaFuncSetAttribute(k_assign_bins, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        256 * 32 * 4 + 32 * (AB_MAX_ROWS / 4 + 1) * 4));
+  // blocks cover the tiles' padding rows (nt: n rounded up to 32) too
+  const dim3 grid((ds->nt + rows - 1) / rows, ds->groups);
+  TC_TRY(table.alloc(ds->ctx, (size_t)ds->groups * kSlots * 32, "edge table"));
+  k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(ds->edges.p, ds->n_edges.p, ds->f, table.p);
+  k_assign_bins<<<grid, AB_THREADS, smem, st>>>(ds->X.p, ds->n, ds->f, table.p, ts, ds->bins_t.p,
+                                                ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p,
+                                                rows);
+  return TC_OK;
 }
 
 // ------------------------------------------- categorical target statistics
@@ -849,10 +1043,11 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   cudaStream_t st = ctx->stream;
   const uint32_t n_tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
   const uint8_t* ts = ds->h_cat_feats.empty() ? nullptr : ds->ts.p;
-  DevBuf<uint32_t> ka, kb, counts, tcnt, U;
+  DevBuf<uint32_t> ka, kb, counts, totals, tcnt, U;
   TC_TRY(ka.alloc(ctx, (size_t)n * f, "sort keys"));
   TC_TRY(kb.alloc(ctx, (size_t)n * f, "sort keys (alt)"));
   TC_TRY(counts.alloc(ctx, (size_t)f * 256 * n_tiles, "radix counts"));
+  TC_TRY(totals.alloc(ctx, (size_t)f * 256, "digit totals"));
   TC_TRY(tcnt.alloc(ctx, (size_t)f * n_tiles, "unique tile counts"));
   TC_TRY(U.alloc(ctx, f, "unique counts"));
   TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
@@ -865,14 +1060,14 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   TC_CUDA(ctx, cudaMemsetAsync(ds->edges.p, 0, ds->edges.bytes(), st));
 
   if (n > 0) {
-    dim3 tg((n + 31) / 32, (f + 31) / 32);
-    k_make_keys<<<tg, dim3(32, 8), 0, st>>>(ds->X.p, n, f, ka.p);
+    k_make_keys<<<dim3((n + MK_ROWS - 1) / MK_ROWS, (f + 31) / 32), 256, 0, st>>>(ds->X.p, n, f, ka.p);
     uint32_t* src = ka.p;
     uint32_t* dst = kb.p;
     for (int shift = 0; shift < 32; shift += 8) {
       k_radix_count<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, n, n_tiles, shift, counts.p);
-      k_segment_scan<<<f, 1024, 0, st>>>(counts.p, 256 * n_tiles, nullptr);
-      k_radix_scatter<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, dst, n, n_tiles, shift, counts.p);
+      k_digit_scan<<<32 * f, 256, 0, st>>>(counts.p, n_tiles, totals.p);
+      k_radix_scatter<false><<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, dst, n, n_tiles, shift, counts.p, totals.p,
+                                                                       nullptr, nullptr);
       std::swap(src, dst);
     }
     k_unique_count<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, n, n_tiles, tcnt.p);
@@ -883,12 +1078,9 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
     TC_CUDA(ctx, cudaMemsetAsync(U.p, 0, U.bytes(), st));
   }
   k_edge_meta<<<(f + 127) / 128, 128, 0, st>>>(U.p, f, max_bins, compat_u8, ts, ds->edges.p, ds->n_edges.p);
-  TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
-  if (n > 0) {
-    dim3 ag((n + AB_ROWS - 1) / AB_ROWS, ds->groups);
-    k_assign_bins<<<ag, 256, 0, st>>>(ds->X.p, n, f, ds->edges.p, ds->n_edges.p, ts, ds->bins_t.p,
-                                      ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p);
-  }
+  DevBuf<float> table;
+  if (n > 0) TC_TRY(launch_assign(ds, ts, table, st));
+  else TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   TC_CUDA(ctx, cudaGetLastError());
   // host copy of the edges for model export / thresholds
   std::vector<float> e((size_t)f * kSlots);
@@ -914,6 +1106,7 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
   if (ref == ds) return TC_OK;  // already binned with its own edges
   cudaStream_t st = ctx->stream;
   const uint32_t n = ds->n, f = ds->f;
+  DevBuf<float> table;
   if (!ref->h_cat_feats.empty() && ds->encoded_by != ref->id) {
     if (!ds->h_cat_feats.empty() || ds->encoded_by)
       return ctx->fail(TC_ERR_INVALID_ARG, "the dataset's categorical columns are already encoded");
@@ -934,12 +1127,11 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
   TC_CUDA(ctx, cudaMemcpyAsync(ds->edges.p, ref->edges.p, ds->edges.bytes(), cudaMemcpyDeviceToDevice, st));
   TC_CUDA(ctx, cudaMemcpyAsync(ds->n_edges.p, ref->n_edges.p, ds->n_edges.bytes(), cudaMemcpyDeviceToDevice, st));
   TC_CUDA(ctx, cudaMemsetAsync(ds->nan_any.p, 0, ds->nan_any.bytes(), st));
-  TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   if (n > 0) {
-    dim3 ag((n + AB_ROWS - 1) / AB_ROWS, ds->groups);
-    k_assign_bins<<<ag, 256, 0, st>>>(ds->X.p, n, f, ds->edges.p, ds->n_edges.p, nullptr, ds->bins_t.p,
-                                      ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p);
+    TC_TRY(launch_assign(ds, nullptr, table, st));
     TC_CUDA(ctx, cudaGetLastError());
+  } else {
+    TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   }
   TC_CUDA(ctx, cudaStreamSynchronize(st));
   ds->h_edges = ref->h_edges;
@@ -991,7 +1183,7 @@ tc_status encode_categorical(tc_dataset* ds, const uint16_t* feats, uint16_t nc,
   }
   cudaStream_t st = ctx->stream;
   const uint32_t n_tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
-  DevBuf<uint32_t> ka, kb, ra, rb, counts, tcnt, nseg, starts, segid, given, lab_flag;
+  DevBuf<uint32_t> ka, kb, ra, rb, counts, totals, tcnt, nseg, starts, segid, given, lab_flag;
   DevBuf<unsigned long long> lab_sum;
   DevBuf<float> prior;
   TC_TRY(ka.alloc(ctx, (size_t)nc * n, "category keys"));
@@ -999,6 +1191,7 @@ tc_status encode_categorical(tc_dataset* ds, const uint16_t* feats, uint16_t nc,
   TC_TRY(ra.alloc(ctx, (size_t)nc * n, "category rows"));
   TC_TRY(rb.alloc(ctx, (size_t)nc * n, "category rows (alt)"));
   TC_TRY(counts.alloc(ctx, (size_t)nc * 256 * n_tiles, "radix counts"));
+  TC_TRY(totals.alloc(ctx, (size_t)nc * 256, "digit totals"));
   TC_TRY(tcnt.alloc(ctx, (size_t)nc * n_tiles, "segment tile counts"));
   TC_TRY(nseg.alloc(ctx, nc, "segment counts"));
   TC_TRY(starts.alloc(ctx, (size_t)nc * n, "segment starts"));
@@ -1032,8 +1225,9 @@ tc_status encode_categorical(tc_dataset* ds, const uint16_t* feats, uint16_t nc,
   uint32_t *ks = ka.p, *kd = kb.p, *rs = ra.p, *rd = rb.p;
   for (int shift = 0; shift < 32; shift += 8) {
     k_radix_count<<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, n, n_tiles, shift, counts.p);
-    k_segment_scan<<<nc, 1024, 0, st>>>(counts.p, 256 * n_tiles, nullptr);
-    k_radix_scatter<<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, kd, n, n_tiles, shift, counts.p, rs, rd);
+    k_digit_scan<<<32 * nc, 256, 0, st>>>(counts.p, n_tiles, totals.p);
+    k_radix_scatter<true><<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, kd, n, n_tiles, shift, counts.p, totals.p, rs,
+                                                                     rd);
     std::swap(ks, kd);
     std::swap(rs, rd);
   }
