@@ -6,23 +6,22 @@
 //   grad       pred += lr * leaf(prev tree) (fused), loss gradients/hessians,
 //              leaf ids reset, per-block root sums            [one pass over rows]
 //   per level d = 0 .. D-1, for all classes k at once:
-//     hist     FP32 shared-memory histograms of the level's build set -- the
-//              root at d = 0, the smaller child of every sibling pair after --
-//              over row-major uint8 bins gathered through the node-grouped row
-//              list; one FP32 partial per (segment chunk, feature group)
-//     merge    FP64 sum of the partials (the cross-block merge) and the FP64
-//              sibling subtraction larger = parent - smaller
-//     scan     per (feature, node group): FP64 prefix (left, NaN slot
-//              included: NaN routes left) and suffix (right) sums and the
-//              Newton gain of every bin for every node, summed over nodes
-//     pick     per class: argmax over (feature, bin), lowest feature then
+//     hist     exact 48-bit fixed-point shared-memory histograms of the level's
+//              build set -- the root at d = 0, the smaller child of every
+//              sibling pair after -- over row-major uint8 bins gathered through
+//              the node-grouped row list, added to FP64 accumulators
+//     scan     per (feature, sibling pair): the FP64 subtraction larger =
+//              parent - smaller, FP64 prefix (left, NaN slot included: NaN
+//              routes left) and suffix (right) sums and the Newton gain of
+//              every bin for both nodes, summed over nodes; its last blocks
+//              pick, per class: argmax over (feature, bin), lowest feature then
 //              lowest bin on ties (the reference keeps the first strictly
 //              greater gain), stop rules, the split goes into the model
 //     part     leaf = 2*leaf + go_right, go_right = bin != 255 && bin > t;
-//              per-block child counts and FP64 child sums
+//              per-block child counts
 //     reduce   child totals, smaller child per pair, scatter offsets
-//     plan     (one block) segment starts, rows per chunk and the chunk counts
-//              the histogram kernel decodes into work items,
+//     plan     (the reduce's last block) segment starts, rows per chunk and the
+//              chunk counts the histogram kernel decodes into work items,
 //              the stop pre-check, leaf values when the tree is complete
 //     scatter  node-grouped row list of the smaller children
 //
@@ -56,7 +55,6 @@ constexpr int PART_THREADS = 512;
 constexpr int GRAD_UNROLL = 4;    // rows per thread with their loads in flight together (one class)
 constexpr int kSoftmaxMaxK = 16;  // softmax classes at most (checked when a trainer is created)
 constexpr int SCAN_WARPS = 8;     // warps per scan block
-constexpr int SCAN_NODES = 16;    // nodes per scan block (2 per warp; measured: 32 per block 4% slower on 1M x 100 depth 8)
 static_assert(SCAN_WARPS * 32 == 256, "a scan block also runs the 256-thread pick");
 constexpr int PLAN_THREADS = 1024;
 constexpr int kHistItemRows = 2048;   // an item's fixed cost in rows of a full group
@@ -92,7 +90,7 @@ struct EsState {
 // Per-(class, feature) best candidate of a level.
 struct FeatBest {
   double gain, second;
-  int32_t b, valid;
+  int32_t key, pad;  // feature << 8 | bin (0x7fffffff: no candidate)
 };
 
 struct DevCfg {
@@ -139,11 +137,10 @@ struct DevPtrs {
   int32_t* seg_len;              // [K][2^(D-1)]
   int32_t* small;                // [K][2^(D-1)] child index of the smaller sibling
   NodeStat* nstat;               // [K][D+1][2^D]
-  uint32_t* pcnt;                // [K][PB][2^D]
-  double2* psum;                 // [K][PB][2^D]
+  uint32_t* pcnt;                // [K][2^D][PB] rows of a node in each partition block
+  double2* psum;                 // [K][PB] root sums of the gradient blocks
   uint32_t* blk_off;             // [K][PB][2^(D-1)]
   double* gpart;                 // [K][F][NG][256]
-  uint8_t* gany;                 // [K][F][NG][256]
   FeatBest* fbest;               // [K][F]
   uint32_t* counters;            // [K] completion counters of the pick blocks
   uint32_t* fcnt;                // [K][F] completion counters of a feature's scan blocks
@@ -180,14 +177,14 @@ __device__ __forceinline__ size_t hist_index(const DevCfg& c, int k, int node, i
   return (((size_t)k * (1u << (c.D > 0 ? c.D - 1 : 0)) + node) * c.f + f) * kSlots + b;
 }
 
-__device__ __forceinline__ int pairs_at(int d) { return d == 0 ? 1 : (1 << (d - 1)); }
+__host__ __device__ __forceinline__ int pairs_at(int d) { return d == 0 ? 1 : (1 << (d - 1)); }
 
 // ------------------------------------------------------------------ grad --
 
 // One thread per row: applies the previous tree of every class
 // (preds += lr * leaf, fused multiply-add as in src/boosting/booster.cpp:458-463),
 // computes the gradients and resets the leaf ids; then per-block root sums
-// (FP64, fixed order) go to psum[k][block][0] / pcnt.
+// (FP64, fixed order) go to psum[k][block] / pcnt.
 // One class's root sums: per-thread FP64 partials (rows in increasing
 // order), reduced in a fixed order (warp shuffles, then the warps in order)
 // into the block's slot of the partition sums, which the level -1 reduce
@@ -207,9 +204,8 @@ __device__ void store_root_partials(const DevCfg& c, const DevPtrs& P, int k, do
     double tg = 0.0, th = 0.0;
     uint32_t tc = 0;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { tg += sG[w]; th += sH[w]; tc += sCnt[w]; }
-    const size_t o = ((size_t)k * c.PB + blockIdx.x) * (1 << c.D);
-    P.psum[o] = make_double2(tg, th);
-    P.pcnt[o] = tc;
+    P.psum[(size_t)k * c.PB + blockIdx.x] = make_double2(tg, th);
+    P.pcnt[((size_t)k << c.D) * c.PB + blockIdx.x] = tc;
   }
   __syncthreads();
 }
@@ -732,138 +728,217 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
 
 // ------------------------------------------------------------------ scan --
 
-__device__ void pick_body(const DevCfg& c, const DevPtrs& P, int d, int f, int k, bool direct, double s_in,
-                          uint8_t any_in);
+__device__ __forceinline__ bool better(double ga, int ka, double gb, int kb) {
+  return ga != gb ? ga > gb : ka < kb;
+}
 
-// grid (F, node groups, K), SCAN_WARPS warps.  A warp scores one node at a
-// time: lane l holds bins 8l .. 8l+7 (bin 255 = NaN rows, added to the left
-// side); left sums are NaN + prefix, right sums an independent suffix, so an
-// empty side is exactly zero.  Per-bin gains (the reference's formula,
-// src/tree/symmetric_tree.cpp:161-178 and 221-236) accumulate in FP64 over
-// the warp's nodes; the block then sums its warps in a fixed order.
-__global__ void __launch_bounds__(SCAN_WARPS * 32) k_scan(DevCfg c, DevPtrs P, int d) {
-  __shared__ double s_acc[SCAN_WARPS][kSlots];
-  __shared__ uint8_t s_any[SCAN_WARPS][kSlots];
-  const int f = blockIdx.x, ng = blockIdx.y, k = blockIdx.z;
-  if (P.cs[k].done) return;
+// A candidate of the pick: gain, runner-up gain and key (feature << 8 | bin;
+// no candidate: 0x7fffffff).  Equal gains go to the lower key: the lowest
+// feature, then the lowest bin (the reference keeps the first strictly greater
+// gain).
+struct PickCand {
+  double g, second;
+  int key;
+};
+__device__ __forceinline__ void pick_merge(PickCand& a, const PickCand& b) {
+  const double rest = fmax(a.second, b.second);
+  if (better(b.g, b.key, a.g, a.key)) {
+    a.second = fmax(a.g, rest);
+    a.g = b.g;
+    a.key = b.key;
+  } else {
+    a.second = fmax(b.g, rest);
+  }
+}
+// Best candidate of a 256-thread block, valid in warp 0; s: 8 entries.
+__device__ __forceinline__ PickCand block_pick(PickCand c, PickCand* s) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int nn = 1 << d;
-  const double lam = (double)c.lam;
-  double2* cur = P.hist[d & 1];
-  const double2* par = P.hist[(d & 1) ^ 1];
+  for (int o = 16; o; o >>= 1) {
+    PickCand b;
+    b.g = __shfl_xor_sync(0xffffffffu, c.g, o);
+    b.second = __shfl_xor_sync(0xffffffffu, c.second, o);
+    b.key = __shfl_xor_sync(0xffffffffu, c.key, o);
+    pick_merge(c, b);
+  }
+  if (lane == 0) s[warp] = c;
+  __syncthreads();
+  if (warp == 0) {
+    c = lane < SCAN_WARPS ? s[lane] : PickCand{-1e300, -1e300, 0x7fffffff};
+    for (int o = SCAN_WARPS / 2; o; o >>= 1) {
+      PickCand b;
+      b.g = __shfl_xor_sync(0xffffffffu, c.g, o);
+      b.second = __shfl_xor_sync(0xffffffffu, c.second, o);
+      b.key = __shfl_xor_sync(0xffffffffu, c.key, o);
+      pick_merge(c, b);
+    }
+  }
+  return c;
+}
+
+__device__ void pick_body(const DevCfg& c, const DevPtrs& P, int d, int f, int k, bool direct, double s_in,
+                          bool any_in, PickCand* s_pick);
+
+// A histogram tile (256 slots of (grad, hess)) between the two layouts of a
+// warp: coalesced, lane l holding slots 32i + l, and by bins, lane l holding
+// slots 8l .. 8l+7; 16-byte units padded by one per 8, so both sides are free
+// of conflicts.
+constexpr int TILE_UNITS = 32 * 9;
+__device__ __forceinline__ int tile_unit(int slot) { return (slot >> 3) * 9 + (slot & 7); }
+
+// Adds one node's gains per bin (lane l: bins 8l .. 8l+7; slot 255 = NaN rows,
+// added to the left side) to acc: left sums are NaN + prefix, right sums an
+// independent suffix, so an empty side is exactly zero.  The reference's
+// formula (src/tree/symmetric_tree.cpp:161-178 and 221-236).
+__device__ __forceinline__ void node_gains(const double2* tile, double lam, int nb_scan, double (&acc)[8],
+                                           uint32_t& anyb) {
+  const int lane = threadIdx.x & 31;
+  double hg[8], hh[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const double2 v = tile[lane * 9 + i];
+    hg[i] = v.x;
+    hh[i] = v.y;
+  }
+  const double nan_g = __shfl_sync(0xffffffffu, hg[7], 31);
+  const double nan_h = __shfl_sync(0xffffffffu, hh[7], 31);
+  if (lane == 31) { hg[7] = 0.0; hh[7] = 0.0; }  // NaN slot is not a regular bin
+  double tg = 0.0, th = 0.0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { tg += hg[i]; th += hh[i]; }
+  // exclusive prefix and suffix of the lane totals
+  double pg = tg, ph = th, sg = tg, sh = th;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double ug = __shfl_up_sync(0xffffffffu, pg, o), uh = __shfl_up_sync(0xffffffffu, ph, o);
+    const double dg = __shfl_down_sync(0xffffffffu, sg, o), dh = __shfl_down_sync(0xffffffffu, sh, o);
+    if (lane >= o) { pg += ug; ph += uh; }
+    if (lane + o < 32) { sg += dg; sh += dh; }
+  }
+  // the node's totals from its own histogram (lane 31's inclusive prefix
+  // plus the NaN slot: one value for the whole warp), so that the parent
+  // term of every bin's gain is consistent with its left and right sums
+  const double Gn = __shfl_sync(0xffffffffu, pg, 31) + nan_g;
+  const double Hn = __shfl_sync(0xffffffffu, ph, 31) + nan_h;
+  pg -= tg; ph -= th;  // exclusive prefix
+  sg -= tg; sh -= th;  // exclusive suffix
+  const double pgain = (Hn > 1e-10) ? (Gn * Gn) / (Hn + lam) : 0.0;
+  // right side of bin 8l+i: this lane's bins above i plus all lanes above
+  double rsg[8], rsh[8];
+  {
+    double ag = sg, ah = sh;
+#pragma unroll
+    for (int i = 7; i >= 0; --i) {
+      rsg[i] = ag;
+      rsh[i] = ah;
+      ag += hg[i];
+      ah += hh[i];
+    }
+  }
+  double lg = nan_g + pg, lh = nan_h + ph;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    lg += hg[i];
+    lh += hh[i];
+    const int b = lane * 8 + i;
+    if (b < nb_scan && lh >= 1e-10 && rsh[i] >= 1e-10) {
+      // GL^2/(HL+lam) + GR^2/(HR+lam) over one FP64 division
+      const double dl = lh + lam, dr = rsh[i] + lam;
+      acc[i] += 0.5 * ((lg * lg * dr + rsg[i] * rsg[i] * dl) / (dl * dr) - pgain);
+      anyb |= 1u << i;
+    }
+  }
+}
+
+// grid (F, pair groups, K), SCAN_WARPS warps, a sibling pair per warp (the
+// root alone at d = 0).  The smaller child (and the root) is the items' FP64
+// sum, the larger one parent - smaller (FP64); both are read and written in
+// whole lines, the accumulators cleared behind the read, and turned to the
+// by-bins layout in shared memory.  Per-bin gains accumulate in FP64 over the
+// pair's nodes; the block then sums its warps in a fixed order, and the last
+// block of a feature picks.
+//
+// What bounds it: memory on wide, deep levels, latency on small ones.  With a
+// node per warp (the pair's accumulators read twice), 16-byte accesses at a
+// 128-byte stride and a pick of two 8-step trees with block barriers, the
+// scans of an iteration took 163 us on 2.5M x 200 (depth 8), here 122; 215 and
+// 150 on 1M x 50, ten classes; 79 and 60 on 50k x 20.
+__global__ void __launch_bounds__(SCAN_WARPS * 32) k_scan(DevCfg c, DevPtrs P, int d) {
+  __shared__ __align__(16) double2 s_tile[SCAN_WARPS][TILE_UNITS];
+  __shared__ PickCand s_pick[SCAN_WARPS];
+  const int f = blockIdx.x, ng = blockIdx.y, k = blockIdx.z;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int np = pairs_at(d), pr = ng * SCAN_WARPS + warp;
   const int Pmax = 1 << (c.D - 1);
-  // the next level reads this level's histograms as parents, the reduce
-  // kernel reads the split feature's row for the children's sums (and the
-  // root's is the tree builder's root-histogram output)
-  const NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + d) * (1 << c.D);
+  const int done = P.cs[k].done;
   double acc[8];
   uint32_t anyb = 0;
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.0;
-  const int n0 = ng * SCAN_NODES, n1 = min(nn, n0 + SCAN_NODES);
-  for (int node = n0 + warp; node < n1; node += SCAN_WARPS) {
-    const NodeStat st = ns[node];
-    if (st.cnt == 0) continue;
-    // the smaller child of a pair (and the root) is the items' FP64 sum; the
-    // larger one is parent - smaller (FP64)
-    const int pr = d == 0 ? 0 : node >> 1;
-    const double2* ap = P.acc + (((size_t)k * Pmax + pr) * c.f + f) * kSlots + lane * 8;
-    double hg[8], hh[8];
+  if (pr < np && !done) {
+    const NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + d) * (1 << c.D);
+    const int n0 = d == 0 ? 0 : 2 * pr;
+    const uint32_t c0 = ns[n0].cnt, c1 = d == 0 ? 0u : ns[n0 + 1].cnt;
+    const int small = d == 0 ? 0 : P.small[k * Pmax + pr];
+    double2* ap = P.acc + (((size_t)k * Pmax + pr) * c.f + f) * kSlots + lane;
+    if (c0 + c1 > 0) {
+      double2 a[8], larger[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const double2 v = ap[i];
-      hg[i] = v.x;
-      hh[i] = v.y;
-    }
-    if (d > 0 && node != P.small[k * Pmax + pr]) {
-      const double2* pp = par + hist_index(c, k, pr, f, 0) + lane * 8;
+      for (int i = 0; i < 8; ++i) a[i] = ap[32 * i];
+      if (d > 0) {
+        const double2* pp = P.hist[(d & 1) ^ 1] + hist_index(c, k, pr, f, 0) + lane;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) larger[i] = pp[32 * i];
+      }
+      double2* tile = s_tile[warp];
+      double2* cur = P.hist[d & 1] + hist_index(c, k, small, f, 0) + lane;
+      // the next level reads this level's histograms as parents, the reduce
+      // kernel reads the split feature's row for the children's sums (and the
+      // root's is the tree builder's root-histogram output)
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        const double2 v = pp[i];
-        hg[i] = v.x - hg[i];
-        hh[i] = v.y - hh[i];
+        ap[32 * i] = make_double2(0.0, 0.0);
+        cur[32 * i] = a[i];
+        tile[tile_unit(32 * i + lane)] = a[i];
       }
-    }
-    {
-      double2* hp = cur + hist_index(c, k, node, f, 0) + lane * 8;
+      __syncwarp();
+      if ((small == n0 ? c0 : c1) > 0) node_gains(tile, (double)c.lam, c.nb_scan, acc, anyb);
+      if (d > 0) {
+        __syncwarp();
+        cur = P.hist[d & 1] + hist_index(c, k, small ^ 1, f, 0) + lane;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) hp[i] = make_double2(hg[i], hh[i]);
-    }
-    const double nan_g = __shfl_sync(0xffffffffu, hg[7], 31);
-    const double nan_h = __shfl_sync(0xffffffffu, hh[7], 31);
-    if (lane == 31) { hg[7] = 0.0; hh[7] = 0.0; }  // NaN slot is not a regular bin
-    double tg = 0.0, th = 0.0;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) { tg += hg[i]; th += hh[i]; }
-    // exclusive prefix and suffix of the lane totals
-    double pg = tg, ph = th, sg = tg, sh = th;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double ug = __shfl_up_sync(0xffffffffu, pg, o), uh = __shfl_up_sync(0xffffffffu, ph, o);
-      const double dg = __shfl_down_sync(0xffffffffu, sg, o), dh = __shfl_down_sync(0xffffffffu, sh, o);
-      if (lane >= o) { pg += ug; ph += uh; }
-      if (lane + o < 32) { sg += dg; sh += dh; }
-    }
-    // the node's totals from its own histogram (lane 31's inclusive prefix
-    // plus the NaN slot: one value for the whole warp), so that the parent
-    // term of every bin's gain is consistent with its left and right sums
-    const double Gn = __shfl_sync(0xffffffffu, pg, 31) + nan_g;
-    const double Hn = __shfl_sync(0xffffffffu, ph, 31) + nan_h;
-    pg -= tg; ph -= th;  // exclusive prefix
-    sg -= tg; sh -= th;  // exclusive suffix
-    const double pgain = (Hn > 1e-10) ? (Gn * Gn) / (Hn + lam) : 0.0;
-    // right side of bin 8l+i: this lane's bins above i plus all lanes above
-    double rsg[8], rsh[8];
-    {
-      double ag = sg, ah = sh;
-#pragma unroll
-      for (int i = 7; i >= 0; --i) {
-        rsg[i] = ag;
-        rsh[i] = ah;
-        ag += hg[i];
-        ah += hh[i];
+        for (int i = 0; i < 8; ++i) {
+          larger[i].x -= a[i].x;
+          larger[i].y -= a[i].y;
+          cur[32 * i] = larger[i];
+          tile[tile_unit(32 * i + lane)] = larger[i];
+        }
+        __syncwarp();
+        if ((small == n0 ? c1 : c0) > 0) node_gains(tile, (double)c.lam, c.nb_scan, acc, anyb);
       }
-    }
-    double lg = nan_g + pg, lh = nan_h + ph;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      lg += hg[i];
-      lh += hh[i];
-      const int b = lane * 8 + i;
-      if (b < c.nb_scan && lh >= 1e-10 && rsh[i] >= 1e-10) {
-        // GL^2/(HL+lam) + GR^2/(HR+lam) over one FP64 division
-        const double dl = lh + lam, dr = rsh[i] + lam;
-        acc[i] += 0.5 * ((lg * lg * dr + rsg[i] * rsg[i] * dl) / (dl * dr) - pgain);
-        anyb |= 1u << i;
-      }
+      __syncwarp();
     }
   }
+  if (done) return;
+  // thread b sums bin b over the warps (their tiles' space, unit per lane and bin)
+  double* s_acc = reinterpret_cast<double*>(s_tile[warp]);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    s_acc[warp][lane * 8 + i] = acc[i];
-    s_any[warp][lane * 8 + i] = (anyb >> i) & 1u;
-  }
+  for (int i = 0; i < 8; ++i) s_acc[lane * 9 + i] = acc[i];
+  // (candidates of the root need a node that allows the bin; only one warp has it)
+  __shared__ uint32_t s_any[32];
+  if (d == 0 && warp == 0) s_any[lane] = anyb;
   __syncthreads();
-  // blockDim.x == kSlots: thread b sums bin b over the warps
   const int b = threadIdx.x;
-  // the accumulators of this block's pairs (this feature) start the next level at zero
-  for (int pr = (d == 0 ? 0 : n0 >> 1); pr < (d == 0 ? 1 : (n1 + 1) >> 1); ++pr)
-    P.acc[(((size_t)k * Pmax + pr) * c.f + f) * kSlots + b] = make_double2(0.0, 0.0);
   double sb = 0.0;
-  uint8_t ab = 0;
-  for (int w = 0; w < SCAN_WARPS; ++w) {
-    sb += s_acc[w][b];
-    ab |= s_any[w][b];
-  }
+#pragma unroll
+  for (int w = 0; w < SCAN_WARPS; ++w) sb += reinterpret_cast<const double*>(s_tile[w])[tile_unit(b)];
+  const bool any = d > 0 || ((s_any[b >> 3] >> (b & 7)) & 1u);
   if (gridDim.y == 1) {  // the only block of its feature: its sums go straight to the pick
-    pick_body(c, P, d, f, k, true, sb, ab);
+    pick_body(c, P, d, f, k, true, sb, any, s_pick);
     return;
   }
-  const size_t o = (((size_t)k * c.f + f) * c.n_scan_groups_max + ng) * kSlots + b;
-  P.gpart[o] = sb;
-  P.gany[o] = ab;
-  // the last node-group block of feature f (completion counter; nobody
-  // waits) picks the feature's best bin, and the class's last feature its split
+  P.gpart[(((size_t)k * c.f + f) * c.n_scan_groups_max + ng) * kSlots + b] = sb;
+  // the last block of feature f (completion counter; nobody waits) picks the
+  // feature's best bin, and the class's last feature its split
   __shared__ bool s_fdone;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -875,67 +950,32 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32) k_scan(DevCfg c, DevPtrs P, i
   if (!s_fdone) return;
   __threadfence();
   if (threadIdx.x == 0) P.fcnt[(size_t)k * c.f + f] = 0;  // re-armed for the next level / graph replay
-  pick_body(c, P, d, f, k, false, 0.0, 0);
+  pick_body(c, P, d, f, k, false, 0.0, true, s_pick);
 }
 
 // ------------------------------------------------------------------ pick --
 
-__device__ __forceinline__ bool better(double ga, int fa, int ba, double gb, int fb, int bb) {
-  if (ga != gb) return ga > gb;
-  if (fa != fb) return fa < fb;
-  return ba < bb;
-}
-
 // Called by the 256 threads (= bins) of the scan block that completes feature
-// f of class k: sums the node-group partials of every bin (or takes the
-// block's own sums, `direct`), keeps the best bin (lowest bin on equal gain)
-// and the runner-up; the last feature block of the class (completion
-// counter, no waiting) reduces the features in ascending order -- the
-// reference keeps the first strictly greater gain, i.e. lowest feature then
-// lowest bin -- applies the stop rule and records the split.
+// f of class k: sums the pair-group partials of every bin (or takes the
+// block's own sums, `direct`), keeps the best bin and the runner-up; the last
+// feature block of the class (completion counter, no waiting) reduces the
+// features, applies the stop rule and records the split.
 __device__ void pick_body(const DevCfg& c, const DevPtrs& P, int d, int f, int k, bool direct, double s_in,
-                          uint8_t any_in) {
-  __shared__ double s_g[256], s_2[256];
-  __shared__ int s_b[256];
+                          bool any_in, PickCand* s_pick) {
   __shared__ bool s_last;
   ClassState& cs = P.cs[k];
   const int b = threadIdx.x;
-  const int ngroups = ((1 << d) + SCAN_NODES - 1) / SCAN_NODES;
   double s = s_in;
-  uint8_t any = any_in;
   if (!direct) {
-    const size_t o = ((size_t)k * c.f + f) * c.n_scan_groups_max * kSlots + b;
-    for (int g = 0; g < ngroups; ++g) {
-      s += P.gpart[o + (size_t)g * kSlots];
-      any |= P.gany[o + (size_t)g * kSlots];
-    }
+    const int ngroups = (pairs_at(d) + SCAN_WARPS - 1) / SCAN_WARPS;
+    const double* gp = P.gpart + ((size_t)k * c.f + f) * c.n_scan_groups_max * kSlots + b;
+#pragma unroll 8
+    for (int g = 0; g < ngroups; ++g) s += __ldcg(gp + (size_t)g * kSlots);
   }
-  const bool cand = b < c.nb_scan && (d > 0 || any);
-  s_g[b] = cand ? s : -1e300;
-  s_2[b] = -1e300;
-  s_b[b] = cand ? b : 0x7fffffff;
-  __syncthreads();
-  for (int stride = 128; stride > 0; stride >>= 1) {
-    if (b < stride) {
-      const int q = b + stride;
-      const double rest = fmax(s_2[b], s_2[q]);
-      if (better(s_g[q], 0, s_b[q], s_g[b], 0, s_b[b])) {
-        s_2[b] = fmax(s_g[b], rest);
-        s_g[b] = s_g[q];
-        s_b[b] = s_b[q];
-      } else {
-        s_2[b] = fmax(s_g[q], rest);
-      }
-    }
-    __syncthreads();
-  }
+  const bool cand = b < c.nb_scan && any_in;
+  PickCand best = block_pick(PickCand{cand ? s : -1e300, -1e300, cand ? (f << 8 | b) : 0x7fffffff}, s_pick);
   if (b == 0) {
-    FeatBest fb;
-    fb.gain = s_g[0];
-    fb.second = s_2[0];
-    fb.b = s_b[0];
-    fb.valid = s_b[0] != 0x7fffffff;
-    P.fbest[(size_t)k * c.f + f] = fb;
+    P.fbest[(size_t)k * c.f + f] = FeatBest{best.g, best.second, best.key, 0};
     __threadfence();
     const uint32_t prev = atomicAdd(&P.counters[k], 1u);
     s_last = prev == c.f - 1;
@@ -944,48 +984,23 @@ __device__ void pick_body(const DevCfg& c, const DevPtrs& P, int d, int f, int k
   if (!s_last) return;
   // last block of class k: reduce the features (fixed order per thread, then a tree)
   __threadfence();
-  double bg = -1e300, b2 = -1e300;
-  int bf = 0x7fffffff, bbin = 0x7fffffff;
+  best = PickCand{-1e300, -1e300, 0x7fffffff};
   for (int ff = b; ff < (int)c.f; ff += blockDim.x) {
-    const FeatBest fb = P.fbest[(size_t)k * c.f + ff];
-    if (!fb.valid) continue;
-    const double rest = fmax(b2, fb.second);
-    if (better(fb.gain, ff, fb.b, bg, bf, bbin)) {
-      b2 = fmax(bg, rest);
-      bg = fb.gain; bf = ff; bbin = fb.b;
-    } else {
-      b2 = fmax(fb.gain, rest);
-    }
+    const FeatBest* fb = P.fbest + (size_t)k * c.f + ff;
+    const PickCand o{__ldcg(&fb->gain), __ldcg(&fb->second), __ldcg(&fb->key)};
+    if (o.key != 0x7fffffff) pick_merge(best, o);
   }
-  __syncthreads();
-  s_g[b] = bg; s_2[b] = b2; s_b[b] = bbin;
-  __shared__ int s_f[256];
-  s_f[b] = bf;
-  __syncthreads();
-  for (int stride = 128; stride > 0; stride >>= 1) {
-    if (b < stride) {
-      const int q = b + stride;
-      const double rest = fmax(s_2[b], s_2[q]);
-      if (better(s_g[q], s_f[q], s_b[q], s_g[b], s_f[b], s_b[b])) {
-        s_2[b] = fmax(s_g[b], rest);
-        s_g[b] = s_g[q]; s_f[b] = s_f[q]; s_b[b] = s_b[q];
-      } else {
-        s_2[b] = fmax(s_g[q], rest);
-      }
-    }
-    __syncthreads();
-  }
+  best = block_pick(best, s_pick);
   if (b == 0) {
     P.counters[k] = 0;  // re-armed for the next level / graph replay
-    const double best = s_g[0];
-    const int bf0 = s_f[0], bb0 = s_b[0];
     const int t = *P.iter * c.KT + c.k0 + k;
     // no candidate (the reference's gain stays -1e30) or below
     // min_split_gain (src/tree/symmetric_tree.cpp:276-278; FP32 compare there)
-    if (bf0 == 0x7fffffff || (float)best < c.msg) {
+    if (best.key == 0x7fffffff || (float)best.g < c.msg) {
       cs.done = 1;
       return;
     }
+    const int bf0 = best.key >> 8, bb0 = best.key & 255;
     float thr = 0.0f;
     const int ne = P.n_edges[bf0];
     if (bb0 < ne) thr = P.edges[(size_t)bf0 * kSlots + bb0];
@@ -993,8 +1008,8 @@ __device__ void pick_body(const DevCfg& c, const DevPtrs& P, int d, int f, int k
     P.m_feat[(size_t)t * c.D + d] = (uint16_t)bf0;
     P.m_bin[(size_t)t * c.D + d] = (uint8_t)bb0;
     P.m_thr[(size_t)t * c.D + d] = thr;
-    P.m_gain[(size_t)t * c.D + d] = best;
-    P.m_second[(size_t)t * c.D + d] = s_2[0];
+    P.m_gain[(size_t)t * c.D + d] = best.g;
+    P.m_second[(size_t)t * c.D + d] = best.second;
     cs.f = bf0;
     cs.b = bb0;
     cs.depth = d + 1;
@@ -1094,99 +1109,124 @@ __global__ void __launch_bounds__(PART_THREADS) k_partition(DevCfg c, DevPtrs P,
   for (int q = threadIdx.x; q < nch; q += blockDim.x) {
     uint32_t cn = 0;
     for (int w = 0; w < ncopy; ++w) cn += sC[w * nch + q];  // the warps' copies
-    P.pcnt[((size_t)k * c.PB + blockIdx.x) * L + q] = cn;
+    P.pcnt[((size_t)k * L + q) * c.PB + blockIdx.x] = cn;
   }
 }
 
-// grid (pairs, K), 512 threads (>= PB).  Child totals (fixed-order FP64
-// sums over blocks), the smaller sibling (left on a tie,
-// src/tree/symmetric_tree.cpp:337-339) and each block's scatter offset of
-// its rows of the smaller child (exclusive scan over blocks).
-__device__ __forceinline__ void node_reduce_body(const DevCfg& c, const DevPtrs& P, int d) {
-  const int k = blockIdx.y, p = blockIdx.x;
-  const ClassState cs = P.cs[k];
-  const bool root = d < 0;  // root reduction after the gradient pass
-  if (!root && (cs.done || cs.depth != d + 1)) return;
-  const int L = 1 << c.D;
-  __shared__ double s_g[2][512], s_h[2][512];
-  __shared__ uint32_t s_c[2][512];
-  __shared__ uint32_t s_w[16];
-  const int nkids = root ? 1 : 2;
-  const int blk = threadIdx.x;
-  uint32_t my_cnt[2] = {0, 0};
-  // row counts per child from the partition blocks; (G, H) of the root from
-  // the gradient pass's block sums, of two children from their parent's
-  // histogram row of the split feature: left = NaN slot + bins 0 .. b,
-  // right = bins b+1 .. 254 (exact sums of the level's histogram)
-  const double2* hrow = root ? nullptr : P.hist[d & 1] + hist_index(c, k, p, cs.f, 0);
-  for (int kid = 0; kid < nkids; ++kid) {
-    const int child = root ? 0 : 2 * p + kid;
-    double g = 0.0, h = 0.0;
-    uint32_t cn = 0;
-    if (blk < c.PB) {
-      const size_t o = ((size_t)k * c.PB + blk) * L + child;
-      if (root) {
-        const double2 v = P.psum[o];
-        g = v.x;
-        h = v.y;
-      }
-      cn = P.pcnt[o];
-    }
-    if (!root && blk < kSlots) {
-      const bool left = blk == kNanBin || blk <= cs.b;
-      if (left == (kid == 0)) {
-        const double2 v = hrow[blk];
-        g = v.x;
-        h = v.y;
-      }
-    }
-    my_cnt[kid] = cn;
-    s_g[kid][blk] = g; s_h[kid][blk] = h; s_c[kid][blk] = cn;
+// grid (ceil(2^d / 16), K), 512 threads: a warp per pair of children (the
+// root: warp 0 of its class).  Row counts per child from the partition
+// blocks; (G, H) of the root from the gradient pass's block sums, of two
+// children from their parent's histogram row of the split feature: left = NaN
+// slot + bins 0 .. b, right = bins b+1 .. 254 (exact sums of the level's
+// histogram).  Then the smaller sibling (left on a tie,
+// src/tree/symmetric_tree.cpp:337-339) and each block's scatter offset of its
+// rows of the smaller child (exclusive scan over blocks).
+//
+// What bounds it: latency, one launch per level in which the whole device
+// waits.  A warp has all its loads (the blocks' counts lie contiguously per
+// node) in flight at once and reduces by shuffles; levels of at most 16 pairs
+// take one block per class and no exchange between blocks before the plan.
+// With a block per pair and nine block barriers per sum: 75 us an iteration
+// on 50k x 20, here 60.
+constexpr int RED_WARPS = 16;   // 128 registers: a pair's loads are all in flight
+constexpr int RED_CHUNKS = 10;  // partition blocks / 32 at most
+
+__device__ __forceinline__ double warp_sum(double v) {
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+__device__ __forceinline__ void root_reduce(const DevCfg& c, const DevPtrs& P, int k) {
+  const int lane = threadIdx.x & 31, L = 1 << c.D;
+  double2 v[RED_CHUNKS];
+  uint32_t n[RED_CHUNKS];
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) {
+    const int b = 32 * i + lane;
+    v[i] = b < c.PB ? P.psum[(size_t)k * c.PB + b] : make_double2(0.0, 0.0);
+    n[i] = b < c.PB ? P.pcnt[(size_t)k * L * c.PB + b] : 0u;
   }
-  __syncthreads();
-  for (int s = 256; s > 0; s >>= 1) {
-    if (blk < s) {
-      for (int kid = 0; kid < nkids; ++kid) {
-        s_g[kid][blk] += s_g[kid][blk + s];
-        s_h[kid][blk] += s_h[kid][blk + s];
-        s_c[kid][blk] += s_c[kid][blk + s];
-      }
-    }
-    __syncthreads();
+  double g = 0.0, h = 0.0;
+  uint32_t cn = 0;
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) {
+    g += v[i].x;
+    h += v[i].y;
+    cn += n[i];
   }
-  const int lvl = root ? 0 : d + 1;
-  NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + lvl) * L;
-  if (root) {
-    if (blk == 0) ns[0] = NodeStat{s_g[0][0], s_h[0][0], s_c[0][0], 0};
-    return;
+  g = warp_sum(g);
+  h = warp_sum(h);
+  cn = __reduce_add_sync(0xffffffffu, cn);
+  if (lane == 0) P.nstat[(size_t)k * (c.D + 1) * L] = NodeStat{g, h, cn, 0};
+}
+
+__device__ __forceinline__ void pair_reduce(const DevCfg& c, const DevPtrs& P, int d, int k, int p,
+                                            const ClassState& cs) {
+  const int lane = threadIdx.x & 31, L = 1 << c.D, Pmax = 1 << (c.D - 1);
+  const uint32_t* pl = P.pcnt + ((size_t)k * L + 2 * p) * c.PB;
+  const uint32_t* pr = pl + c.PB;
+  const double2* hrow = P.hist[d & 1] + hist_index(c, k, p, cs.f, 0);
+  uint32_t nl[RED_CHUNKS], nr[RED_CHUNKS];
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) {
+    const int b = 32 * i + lane;
+    nl[i] = b < c.PB ? pl[b] : 0u;
+    nr[i] = b < c.PB ? pr[b] : 0u;
   }
-  const uint32_t cl = s_c[0][0], cr = s_c[1][0];
-  const int sm = (cl <= cr) ? 0 : 1;
-  const int Pmax = 1 << (c.D - 1);
-  if (blk == 0) {
+  double gl = 0.0, hl = 0.0, gr = 0.0, hr = 0.0;
+#pragma unroll
+  for (int i = 0; i < kSlots / 32; ++i) {
+    const int b = 32 * i + lane;
+    const double2 v = hrow[b];
+    const bool left = b == kNanBin || b <= cs.b;
+    gl += left ? v.x : 0.0;
+    hl += left ? v.y : 0.0;
+    gr += left ? 0.0 : v.x;
+    hr += left ? 0.0 : v.y;
+  }
+  uint32_t cl = 0, cr = 0;
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) {
+    cl += nl[i];
+    cr += nr[i];
+  }
+  cl = __reduce_add_sync(0xffffffffu, cl);
+  cr = __reduce_add_sync(0xffffffffu, cr);
+  gl = warp_sum(gl);
+  hl = warp_sum(hl);
+  gr = warp_sum(gr);
+  hr = warp_sum(hr);
+  const bool sm = cl > cr;  // the smaller child: 1 = right
+  if (lane == 0) {
     // an empty child has zero sums (its parent's histogram row is not
     // written when the parent itself is empty)
-    ns[2 * p] = cl ? NodeStat{s_g[0][0], s_h[0][0], cl, 0} : NodeStat{0.0, 0.0, 0u, 0};
-    ns[2 * p + 1] = cr ? NodeStat{s_g[1][0], s_h[1][0], cr, 0} : NodeStat{0.0, 0.0, 0u, 0};
+    NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + d + 1) * L;
+    ns[2 * p] = cl ? NodeStat{gl, hl, cl, 0} : NodeStat{0.0, 0.0, 0u, 0};
+    ns[2 * p + 1] = cr ? NodeStat{gr, hr, cr, 0} : NodeStat{0.0, 0.0, 0u, 0};
     if (d + 1 < c.D) {
-      P.small[k * Pmax + p] = 2 * p + sm;
+      P.small[k * Pmax + p] = 2 * p + (sm ? 1 : 0);
       P.seg_len[k * Pmax + p] = (int)(sm ? cr : cl);
     }
   }
   if (d + 1 >= c.D) return;
-  // exclusive scan over blocks of the smaller child's counts
-  const uint32_t v = my_cnt[sm];
-  const int lane = blk & 31, warp = blk >> 5;
-  uint32_t x = v;
+  uint32_t x[RED_CHUNKS];
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) x[i] = sm ? nr[i] : nl[i];
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+#pragma unroll
+    for (int i = 0; i < RED_CHUNKS; ++i) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x[i], o);
+      if (lane >= o) x[i] += y;
+    }
   }
-  if (lane == 31) s_w[warp] = x;
-  __syncthreads();
   uint32_t before = 0;
-  for (int w = 0; w < warp; ++w) before += s_w[w];
-  if (blk < c.PB) P.blk_off[((size_t)k * c.PB + blk) * Pmax + p] = before + x - v;
+#pragma unroll
+  for (int i = 0; i < RED_CHUNKS; ++i) {
+    const int b = 32 * i + lane;
+    if (b < c.PB) P.blk_off[((size_t)k * c.PB + b) * Pmax + p] = before + x[i] - (sm ? nr[i] : nl[i]);
+    before += __shfl_sync(0xffffffffu, x[i], 31);
+  }
 }
 
 // One block.  For the level d about to be histogrammed: per class the stop
@@ -1196,13 +1236,13 @@ __device__ __forceinline__ void node_reduce_body(const DevCfg& c, const DevPtrs&
 // (class, pair, feature group), which the histogram kernel decodes into work
 // items.
 constexpr int kPlanSegs = 4096;  // (class, pair) segment lengths the plan keeps in shared memory
+constexpr int kPlanTries = 16;   // candidates for the rows per chunk, a warp each
 
 __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int d) {
   __shared__ long long s_rows;
   __shared__ int s_nodes;
   __shared__ int s_live;            // non-empty segments of the level
   __shared__ int s_warp[32];
-  __shared__ int s_carry;
   __shared__ int s_len[kPlanSegs];  // [class][pair] rows of level d (0: the class grows no more)
   const int Pmax = 1 << (c.D - 1);
   const int L = 1 << c.D;
@@ -1216,29 +1256,35 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   for (int k = warp; k < c.K; k += nwarps) {
     ClassState& cs = P.cs[k];
     int done = cs.done, depth = cs.depth;
+    const NodeStat* nd = P.nstat + ((size_t)k * (c.D + 1) + d) * L;
+    // (read before the state is known: one round of loads)
+    const uint32_t tot = P.nstat[((size_t)k * (c.D + 1)) * L].cnt;  // rows of the level (the root's count)
+    const int len0 = d > 0 && lane < np2 ? P.seg_len[k * Pmax + lane] : (int)c.n;
+    uint32_t maxcnt = 0;
+    int go = 0, hot = INT32_MAX;  // the largest node, the lowest index on a tie
+#pragma unroll 4
+    for (int q = lane; q < (1 << d); q += 32) {
+      const uint32_t cnt = nd[q].cnt;
+      const float H = (float)nd[q].H;
+      if (cnt >= (uint32_t)c.msl * 2u && H >= c.mcw * 2.0f) go = 1;
+      if (cnt > maxcnt || hot == INT32_MAX) {
+        maxcnt = cnt;
+        hot = q;
+      }
+    }
     if (d == 0) { done = 0; depth = 0; }
     if (d == 0 && c.nv > 0 && P.es->stopped) done = 2;  // early-stopped: no more trees
     const bool alive = !done && (d == 0 || depth == d) && d < c.D;
-    int go = 0;
     if (alive) {
-      const NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + d) * L;
-      uint32_t maxcnt = 0;
-      for (int q = lane; q < (1 << d); q += 32) {
-        const uint32_t cnt = ns[q].cnt;
-        if (cnt >= (uint32_t)c.msl * 2u && (float)ns[q].H >= c.mcw * 2.0f) go = 1;
-        maxcnt = max(maxcnt, cnt);
-      }
       go = __any_sync(0xffffffffu, go);
-      for (int o = 16; o; o >>= 1) maxcnt = max(maxcnt, __shfl_xor_sync(0xffffffffu, maxcnt, o));
-      int hot = INT32_MAX;  // the largest node, the lowest index on a tie
-      for (int q = lane; q < (1 << d); q += 32)
-        if (ns[q].cnt == maxcnt) hot = min(hot, q);
-      for (int o = 16; o; o >>= 1) hot = min(hot, __shfl_xor_sync(0xffffffffu, hot, o));
+      const uint32_t top = __reduce_max_sync(0xffffffffu, maxcnt);
+      hot = __reduce_min_sync(0xffffffffu, maxcnt == top ? hot : INT32_MAX);
       if (lane == 0) {
-        const uint32_t tot = P.nstat[((size_t)k * (c.D + 1)) * L].cnt;  // rows of the level (the root's count)
-        cs.skew = (uint64_t)maxcnt * 8u > (uint64_t)tot ? 1 : 0;
+        cs.skew = (uint64_t)top * 8u > (uint64_t)tot ? 1 : 0;
         cs.hot = hot == INT32_MAX ? 0 : hot;
       }
+    } else {
+      go = 0;
     }
     if (!done && !(alive && go)) done = 1;
     if (done == 1) {
@@ -1268,7 +1314,7 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
       int carry = 0, live = 0;
       for (int base = 0; base < np2; base += 32) {
         const int p = base + lane;
-        const int len = p < np2 ? (d == 0 ? (int)c.n : P.seg_len[k * Pmax + p]) : 0;
+        const int len = p < np2 ? (base == 0 ? len0 : P.seg_len[k * Pmax + p]) : 0;
         int x = len;
         for (int o = 1; o < 32; o <<= 1) {
           const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1315,46 +1361,35 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   // one wave: 135 us on level 1, 829k rows; 23 chunks whose narrow items run
   // after the wide ones: 157).  Segments that do not fill a wave between them
   // add an item each.
-  __shared__ int s_R;
-  __shared__ long long s_cnt;
+  // Sixteen candidates for that R, 1 to 4.5 times the start, a warp each (one
+  // barrier instead of a search with three per step; R need not be exact).
+  __shared__ long long s_items[kPlanTries];
   const int waves = max(1, c.target_items / c.hist_grid);
   const int gw = waves == 1 || c.gwide == 0 ? c.G : c.gwide;
-  const long long load = (s_rows * c.row_words / 8 + (long long)s_live * c.G * kHistItemRows) / c.hist_grid + 1;
-  long long allowed = 0;
-  {
-    long long R = c.rows_fixed;
-    if (R <= 0) R = max((long long)c.rows_min, min(load, max(load / waves, (long long)kHistRowsSplit)));
-    R = min(R, (long long)kHistRowsMax);
-    allowed = max(1LL, (load + R / 2) / R) * c.hist_grid;
-    if (2LL * s_live * gw > allowed) allowed += (long long)s_live * gw;
-    if (tid == 0) s_R = (int)R;
-  }
-  __syncthreads();
-  for (int round = 0; c.rows_fixed <= 0 && round < 16; ++round) {
-    const int Rt = s_R;
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
+  // (FP32: neither the share nor R need more)
+  const float load = ((float)s_rows * (float)c.row_words * 0.125f + (float)s_live * (float)(c.G * kHistItemRows)) /
+                         (float)c.hist_grid + 1.0f;
+  const float r0 = fminf(fmaxf((float)c.rows_min, fminf(load, fmaxf(load / (float)waves, (float)kHistRowsSplit))),
+                         (float)kHistRowsMax);
+  long long allowed = (long long)fmaxf(1.0f, rintf(load / r0)) * c.hist_grid;
+  if (2LL * s_live * gw > allowed) allowed += (long long)s_live * gw;
+  auto candidate = [&](int j) { return (int)fminf((float)kHistRowsMax, r0 + r0 * (float)(j * j) * (1.0f / 64.0f)); };
+  if (warp < kPlanTries) {
+    const uint32_t Rt = (uint32_t)candidate(warp);
     long long mine = 0;
-    for (int sgi = tid; sgi < nsg; sgi += blockDim.x) mine += (seg_rows(sgi) + Rt - 1) / Rt;
+    for (int sgi = lane; sgi < nsg; sgi += 32) mine += ((uint32_t)seg_rows(sgi) + Rt - 1) / Rt;
     for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0 && mine) atomicAdd(reinterpret_cast<unsigned long long*>(&s_cnt), (unsigned long long)mine);
-    __syncthreads();
-    const long long items = s_cnt * gw;
-    __syncthreads();
-    if (items <= allowed || Rt >= kHistRowsMax) break;
-    if (tid == 0) s_R = (int)min((long long)kHistRowsMax, (long long)Rt * items / allowed + 1);
-    __syncthreads();
-  }
-  if (tid == 0) {
-    *P.rchunk = s_R;
-    s_carry = 0;
+    if (lane == 0) s_items[warp] = mine * gw;
   }
   __syncthreads();
-  const int R = s_R;
+  int pick = 0;
+  while (pick < kPlanTries - 1 && s_items[pick] > allowed) ++pick;
+  const int R = c.rows_fixed > 0 ? c.rows_fixed : candidate(pick);
   // cumulative item counts over segments (class, pair): chunks x groups
+  int carry = 0;
   for (int base = 0; base < nsg; base += blockDim.x) {
     const int sgi = base + tid;
-    const int chunks = sgi < nsg ? (seg_rows(sgi) + R - 1) / R * c.G : 0;
+    const int chunks = sgi < nsg ? (int)(((uint32_t)seg_rows(sgi) + (uint32_t)R - 1) / (uint32_t)R) * c.G : 0;
     int x = chunks;
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -1362,15 +1397,18 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    int before = s_carry;
-    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    int before = carry, all = 0;
+    for (int w = 0; w < nwarps; ++w) {
+      if (w < warp) before += s_warp[w];
+      all += s_warp[w];
+    }
     if (sgi < nsg) P.cum[sgi] = before + x - chunks;
-    __syncthreads();
-    if (tid == blockDim.x - 1) s_carry = before + x;
-    __syncthreads();
+    carry += all;
+    if (base + (int)blockDim.x < nsg) __syncthreads();  // s_warp is written again
   }
   if (tid == 0) {
-    P.cum[nsg] = s_carry;
+    *P.rchunk = R;
+    P.cum[nsg] = carry;
     *P.hist_ctr = c.hist_grid;  // items 0 .. grid - 1 belong to the blocks by index
     if (d < 16) {
       P.lvl_rows[d] = (uint64_t)s_rows;
@@ -1381,13 +1419,24 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
 
 __global__ void __launch_bounds__(PLAN_THREADS) k_plan(DevCfg c, DevPtrs P, int d) { plan_body(c, P, d); }
 
-// grid (nodes of level d, K): the reduce above; with FUSE_PLAN the last block
-// to finish (completion counter, nobody waits) also plans level d + 1, so a
-// level needs one launch less.
+// The reduce above for level d (-1: the root); with FUSE_PLAN the last block
+// to finish (completion counter, nobody waits; a single block at once) also
+// plans level d + 1, so a level needs one launch less.
 template <bool FUSE_PLAN>
-__global__ void __launch_bounds__(512) k_node_reduce(DevCfg c, DevPtrs P, int d) {
-  node_reduce_body(c, P, d);
+__global__ void __launch_bounds__(32 * RED_WARPS) k_node_reduce(DevCfg c, DevPtrs P, int d) {
+  const int k = blockIdx.y, p = blockIdx.x * RED_WARPS + (int)(threadIdx.x >> 5);
+  if (d < 0) {
+    if (p == 0) root_reduce(c, P, k);
+  } else if (p < (1 << d)) {
+    const ClassState cs = P.cs[k];
+    if (!cs.done && cs.depth == d + 1) pair_reduce(c, P, d, k, p, cs);
+  }
   if (FUSE_PLAN) {
+    if (gridDim.x * gridDim.y == 1) {
+      __syncthreads();
+      plan_body(c, P, d + 1);
+      return;
+    }
     __shared__ bool s_last;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1632,7 +1681,6 @@ struct tc_trainer {
   DevBuf<uint32_t> pcnt, blk_off;
   DevBuf<double2> psum;
   DevBuf<double> gpart;
-  DevBuf<uint8_t> gany;
   DevBuf<ClassState> cs;
   DevBuf<int32_t> m_depth;
   DevBuf<uint16_t> m_feat;
@@ -1720,11 +1768,10 @@ tc_status tc_trainer::setup(int) {
   const uint32_t n = ds->n, f = ds->f;
   const int K = prm.loss == TC_LOSS_SOFTMAX ? prm.n_classes : 1;
   const int D = prm.max_depth;
-  const int PB = ctx->sm_count * 2;
-  if (PB > 512) return ctx->fail(TC_ERR_INVALID_ARG, "too many SMs for the partition reduction");
+  const int PB = std::min(ctx->sm_count * 2, 32 * RED_CHUNKS);
   const int Pmax = 1 << (D - 1);
   const int L = 1 << D;
-  const int ngroups_max = (L / 2 + SCAN_NODES - 1) / SCAN_NODES;
+  const int ngroups_max = (Pmax / 2 + SCAN_WARPS - 1) / SCAN_WARPS;  // pairs of the deepest level, 8 per block
   const int G = 1, W = 32;  // placeholders until configure()
 
   cfg.n = n; cfg.f = f; cfg.np = ds->np;
@@ -1762,10 +1809,9 @@ tc_status tc_trainer::setup(int) {
   TC_TRY(iter.alloc(ctx, 1, "iteration"));
   TC_TRY(nstat.alloc(ctx, (size_t)K * (D + 1) * L, "node stats"));
   TC_TRY(pcnt.alloc(ctx, (size_t)K * PB * L, "partition counts"));
-  TC_TRY(psum.alloc(ctx, (size_t)K * PB * L, "partition sums"));
+  TC_TRY(psum.alloc(ctx, (size_t)K * PB, "root partial sums"));
   TC_TRY(blk_off.alloc(ctx, (size_t)K * PB * Pmax, "scatter offsets"));
   TC_TRY(gpart.alloc(ctx, (size_t)K * f * cfg.n_scan_groups_max * kSlots, "gain partials"));
-  TC_TRY(gany.alloc(ctx, (size_t)K * f * cfg.n_scan_groups_max * kSlots, "gain flags"));
   TC_TRY(fbest.alloc(ctx, (size_t)K * f, "feature bests"));
   TC_TRY(counters.alloc(ctx, K, "pick counters"));
   TC_TRY(hist_ctr.alloc(ctx, 1, "histogram item counter"));
@@ -1792,7 +1838,7 @@ tc_status tc_trainer::setup(int) {
   ptr.y = ds->y.p; ptr.pred = pred.p; ptr.gh = gh.p; ptr.cgh = cgh.p; ptr.leaf = leaf.p; ptr.rows = rows.p;
   ptr.hist[0] = hist0.p; ptr.hist[1] = hist1.p; ptr.acc = acc.p; ptr.rchunk = rchunk.p;
   ptr.seg_start = seg_start.p; ptr.seg_len = seg_len.p; ptr.small = small.p; ptr.nstat = nstat.p;
-  ptr.pcnt = pcnt.p; ptr.psum = psum.p; ptr.blk_off = blk_off.p; ptr.gpart = gpart.p; ptr.gany = gany.p;
+  ptr.pcnt = pcnt.p; ptr.psum = psum.p; ptr.blk_off = blk_off.p; ptr.gpart = gpart.p;
   ptr.fbest = fbest.p; ptr.counters = counters.p; ptr.hist_ctr = hist_ctr.p; ptr.red_ctr = red_ctr.p; ptr.fcnt = fcnt.p; ptr.cs = cs.p; ptr.iter = iter.p;
   ptr.m_depth = m_depth.p; ptr.m_feat = m_feat.p; ptr.m_bin = m_bin.p; ptr.m_thr = m_thr.p; ptr.m_gain = m_gain.p;
   ptr.m_second = m_second.p; ptr.m_leaves = m_leaves.p; ptr.root_hist_out = nullptr;
@@ -1975,7 +2021,7 @@ void tc_trainer::launch_level(const DevCfg& c, const DevPtrs& P, int d, cudaStre
     prof->back().level = d;
     prof->back().rows = hist_rows;
   }
-  const int ng = ((1 << d) + SCAN_NODES - 1) / SCAN_NODES;
+  const int ng = (pairs_at(d) + SCAN_WARPS - 1) / SCAN_WARPS;
   mark_begin(KC_SCAN, st);
   k_scan<<<dim3(c.f, ng, K), SCAN_WARPS * 32, 0, st>>>(c, P, d);  // + pick
   mark_end(st);
@@ -1996,7 +2042,7 @@ void tc_trainer::launch_level(const DevCfg& c, const DevPtrs& P, int d, cudaStre
   mark_end(st, (double)c.n * K * (1 + 2 + 2));
   if (prof) prof->back().level = d;
   mark_begin(KC_REDUCE, st);
-  k_node_reduce<true><<<dim3(1 << d, K), 512, 0, st>>>(c, P, d);  // + plan of level d + 1
+  k_node_reduce<true><<<dim3(((1 << d) + RED_WARPS - 1) / RED_WARPS, K), 32 * RED_WARPS, 0, st>>>(c, P, d);  // + plan of level d + 1
   mark_end(st);
   if (d + 1 < D) {
     mark_begin(KC_SCATTER, st);
@@ -2023,7 +2069,7 @@ tc_status tc_trainer::enqueue_iteration(cudaStream_t st) {
 tc_status tc_trainer::enqueue_rest(cudaStream_t st) {
   const int K = cfg.K, D = cfg.D;
   mark_begin(KC_REDUCE, st);
-  k_node_reduce<true><<<dim3(1, K), 512, 0, st>>>(cfg, ptr, -1);  // + plan of level 0
+  k_node_reduce<true><<<dim3(1, K), 32 * RED_WARPS, 0, st>>>(cfg, ptr, -1);  // + plan of level 0
   mark_end(st);
   for (int d = 0; d < D; ++d) launch_level(cfg, ptr, d, st);
   if (cfg.nv > 0) {
@@ -2052,9 +2098,8 @@ static DevPtrs class_view(const DevCfg& c, const DevPtrs& P, int k, DevCfg* one)
   pk.seg_start += k * Pmax; pk.seg_len += k * Pmax;
   pk.small += k * Pmax; pk.nstat += (size_t)k * (c.D + 1) * L;
   pk.fbest += (size_t)k * c.f; pk.counters += k; pk.fcnt += (size_t)k * c.f;
-  pk.pcnt += (size_t)k * c.PB * L; pk.psum += (size_t)k * c.PB * L; pk.blk_off += (size_t)k * c.PB * Pmax;
+  pk.pcnt += (size_t)k * c.PB * L; pk.psum += (size_t)k * c.PB; pk.blk_off += (size_t)k * c.PB * Pmax;
   pk.gpart += (size_t)k * c.f * c.n_scan_groups_max * kSlots;
-  pk.gany += (size_t)k * c.f * c.n_scan_groups_max * kSlots;
   pk.cs += k;
   return pk;
 }
@@ -2064,7 +2109,7 @@ static DevPtrs class_view(const DevCfg& c, const DevPtrs& P, int k, DevCfg* one)
 tc_status tc_trainer::run_plain_iteration(cudaStream_t st, bool grad) {
   const int K = cfg.K, D = cfg.D;
   if (grad) launch_grad(cfg, ptr, 0, st);
-  k_node_reduce<false><<<dim3(1, K), 512, 0, st>>>(cfg, ptr, -1);
+  k_node_reduce<false><<<dim3(1, K), 32 * RED_WARPS, 0, st>>>(cfg, ptr, -1);
   for (int k = 0; k < K; ++k) {
     DevCfg one;
     DevPtrs pk = class_view(cfg, ptr, k, &one);
@@ -2819,7 +2864,7 @@ tc_status tc_build_tree(tc_ctx* ctx, tc_dataset* ds, const float* grad, const fl
   // one iteration with the given gradients
   const int D = tr->cfg.D;
   launch_grad(tr->cfg, tr->ptr, 1, st);
-  k_node_reduce<false><<<dim3(1, 1), 512, 0, st>>>(tr->cfg, tr->ptr, -1);
+  k_node_reduce<false><<<dim3(1, 1), 32 * RED_WARPS, 0, st>>>(tr->cfg, tr->ptr, -1);
   k_plan<<<1, PLAN_THREADS, 0, st>>>(tr->cfg, tr->ptr, 0);
   for (int d = 0; d < D; ++d) {
     tr->launch_level(tr->cfg, tr->ptr, d, st);
