@@ -427,8 +427,11 @@ __device__ __forceinline__ int fix_exponent(double S, double rows) {
   if (!(S > 0.0)) return 0;
   // a relative margin for the rounding of the FP64 sum S itself
   const double room = kFixLimit * (1.0 - 0x1p-20) - 0.5 * rows;
-  int e = ilogb(room / S);      // floor(log2(room / S))
-  if (ldexp(S, e) > room) --e;  // against rounding of the division
+  // the largest e with 2^e * S <= room, from the exponents and mantissas (a
+  // subnormal or infinite S ends at the limits)
+  const long long s = __double_as_longlong(S), r = __double_as_longlong(room);
+  constexpr long long kMant = (1LL << 52) - 1;
+  const int e = (int)(r >> 52) - (int)(s >> 52) - ((s & kMant) > (r & kMant) ? 1 : 0);
   return max(-126, min(100, e));
 }
 __device__ __forceinline__ float exp2i(int e) { return __int_as_float((e + 127) << 23); }
@@ -488,12 +491,13 @@ __device__ __forceinline__ void load_slice(uint32_t (&w)[W4], const uint8_t* src
 // took 110 instructions and 21 wavefronts per 128 pairs.  Root level of 2.5M
 // rows x 200 features: 518 -> 372 us (5.0 pairs / clk / SM over the launch);
 // 1M x 50, ten classes, all levels: 2098 -> 1473 us.
-// `scales` (the pass that fixes the item's scales, with the block's barrier)
-// runs behind the first loads.
-template <bool CNT, int W4, class Scales>
+// `sums` (the pass over the item's (grad, hess)) runs behind the load of the
+// first row ids, `scales` (the block's reduction to the item's scales, with its
+// barrier) behind the load of the first rows.
+template <bool CNT, int W4, class Sums, class Scales>
 __device__ __forceinline__ void hist_rows(uint32_t hbase, int start, int end, bool gathered,
                                           const uint32_t* __restrict__ rows, const float2* __restrict__ gh,
-                                          const uint8_t* __restrict__ tile, Scales scales) {
+                                          const uint8_t* __restrict__ tile, Sums sums, Scales scales) {
   constexpr int B = HIST_BATCH, NW = HIST_THREADS / 32;
   constexpr uint32_t FB = 4 * HistShape::W;  // bytes between two fields of a slot
   const uint32_t lane = threadIdx.x & 31;
@@ -525,6 +529,7 @@ __device__ __forceinline__ void hist_rows(uint32_t hbase, int start, int end, bo
   for (int j = 0; j < W4; ++j) nxt[j] = 0u;
   int bi = (int)(threadIdx.x >> 5);
   fetch_id(bi);
+  sums();
   fetch_row(bi);
   fetch_id(bi + NW);
   float sg, sh;
@@ -600,7 +605,6 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
   const int nseg = c.K * P2;
   const int n_items = P.cum[nseg];
   const int Pmax = 1 << (c.D - 1);
-  if ((int)blockIdx.x >= n_items) return;  // the first item by index, the others from the counter
   const int R = *P.rchunk;
   // Items are claimed from a counter (blocks that drew cheap items take
   // more), the next one while the current one runs.  Item ci*G + g is chunk
@@ -613,20 +617,22 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     if (gw == 0 || gw == c.G || cl >= n_items) return cl;
     return cl < n_chunks * gw ? (cl / gw) * c.G + cl % gw : (cl - n_chunks * gw) * c.G + gw;
   };
-  // The one thread whose segment holds the item publishes it: one load for
-  // every thread instead of a search with a load per step.
+  // The one thread whose segment holds the item publishes it: one round of
+  // loads for every thread instead of a search with a load per step.
+  const int log_p2 = d == 0 ? 0 : d - 1;
   auto decode = [&](int it, int ph) {
     for (int q = threadIdx.x; q < nseg; q += HIST_THREADS) {
-      const int c0 = P.cum[q];
-      if (c0 <= it && it < P.cum[q + 1]) {
+      const int k = q >> log_p2, p = q - (k << log_p2);
+      const int c0 = P.cum[q], c1 = P.cum[q + 1];
+      const int s0 = d == 0 ? 0 : P.seg_start[k * Pmax + p];
+      const int sl = d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
+      if (c0 <= it && it < c1) {
         const int ch = (it - c0) / c.G;
-        const int k = q / P2, p = q - k * P2;
         // the segment's ceil(len / R) chunks have equal sizes (within one row)
-        const int s0 = d == 0 ? 0 : P.seg_start[k * Pmax + p];
-        const int sl = d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
-        const int nch = (sl + R - 1) / R;
-        s_item[ph] = HistItem{k, p, (it - c0) - ch * c.G, s0 + (int)((long long)sl * ch / nch),
-                              s0 + (int)((long long)sl * (ch + 1) / nch)};
+        const int nch = (int)(((uint32_t)sl + (uint32_t)R - 1) / (uint32_t)R);
+        const int len = (int)((uint32_t)sl / (uint32_t)nch), more = sl - len * nch;  // `more` chunks of len + 1
+        const int start = s0 + ch * len + min(ch, more);
+        s_item[ph] = HistItem{k, p, (it - c0) - ch * c.G, start, start + len + (ch < more ? 1 : 0)};
       }
     }
   };
@@ -636,6 +642,7 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     for (int q = threadIdx.x; q < kSlots * S_::FIELDS * W / 4; q += HIST_THREADS) z[q] = make_uint4(0u, 0u, 0u, 0u);
   }
   __syncthreads();
+  if ((int)blockIdx.x >= n_items) return;  // the first item by index, the others from the counter
   for (int ph = 0;; ph ^= 1) {
     const int k = s_item[ph].k, p = s_item[ph].p, g = s_item[ph].g, start = s_item[ph].start, end = s_item[ph].end;
     if (threadIdx.x == 0) s_next = claim_to_item(atomicAdd(P.hist_ctr, 1));
@@ -647,37 +654,39 @@ __global__ void __launch_bounds__(HIST_THREADS, 1) k_hist(DevCfg c, DevPtrs P, i
     // child's were copied next to its row ids by the scatter kernel
     const float2* gh = (d == 0 ? P.gh : P.cgh) + (size_t)k * c.n;
     // the item's scales: FP64 sums of |grad| and |hess| over its rows
+    double sa = 0.0, sb = 0.0;
     int eg = 0, eh = 0;
-    auto scales = [&](float& sg, float& sh) {
-      double sa = 0.0, sb = 0.0;
+    auto sums = [&]() {
 #pragma unroll 4
       for (int r = start + threadIdx.x; r < end; r += HIST_THREADS) {
         const float2 v = gh[r];
         sa += (double)fabsf(v.x);
         if (!CNT) sb += (double)fabsf(v.y);
       }
-      for (int o = 16; o; o >>= 1) {
-        sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        if (!CNT) sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      }
-      if (lane == 0) { s_sum[0][warp] = sa; s_sum[1][warp] = sb; }
+    };
+    // The lower lanes reduce |grad|, the upper ones |hess|: half the shuffles of
+    // a reduction each (reductions and exponents were a quarter of a small item:
+    // 50k x 20, a whole iteration 199 -> 192 us with them, the shorter decode and
+    // the sums behind the row ids; 1M x 50, ten classes: 1979 -> 1936).
+    auto scales = [&](float& sg, float& sh) {
+      const bool up = lane >= 16;
+      double x = (up ? sb : sa) + __shfl_xor_sync(0xffffffffu, up ? sa : sb, 16);
+      for (int o = 8; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      if ((lane & 15) == 0) s_sum[up][warp] = x;
       __syncthreads();
-      sa = s_sum[0][lane];
-      sb = s_sum[1][lane];
-      for (int o = 16; o; o >>= 1) {
-        sa += __shfl_xor_sync(0xffffffffu, sa, o);
-        if (!CNT) sb += __shfl_xor_sync(0xffffffffu, sb, o);
-      }
-      eg = fix_exponent(sa, (double)(end - start));
-      eh = CNT ? 0 : fix_exponent(sb, (double)(end - start));
+      x = s_sum[up][lane & 15] + s_sum[up][16 + (lane & 15)];
+      for (int o = 8; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+      const int e = fix_exponent(x, (double)(end - start));
+      eg = __shfl_sync(0xffffffffu, e, 0);
+      eh = CNT ? 0 : __shfl_sync(0xffffffffu, e, 16);
       sg = exp2i(eg);
       sh = exp2i(eh);
     };
     const uint8_t* tile = P.bins_t + (uint64_t)g * c.gstride;
-    if (wid == 32) hist_rows<CNT, 8>(hbase, start, end, d > 0, rows, gh, tile, scales);
-    else if (wid == 16) hist_rows<CNT, 4>(hbase, start, end, d > 0, rows, gh, tile, scales);
-    else if (wid == 8) hist_rows<CNT, 2>(hbase, start, end, d > 0, rows, gh, tile, scales);
-    else hist_rows<CNT, 1>(hbase, start, end, d > 0, rows, gh, tile, scales);
+    if (wid == 32) hist_rows<CNT, 8>(hbase, start, end, d > 0, rows, gh, tile, sums, scales);
+    else if (wid == 16) hist_rows<CNT, 4>(hbase, start, end, d > 0, rows, gh, tile, sums, scales);
+    else if (wid == 8) hist_rows<CNT, 2>(hbase, start, end, d > 0, rows, gh, tile, sums, scales);
+    else hist_rows<CNT, 1>(hbase, start, end, d > 0, rows, gh, tile, sums, scales);
     __syncthreads();
     const int next = s_next;
     if (next < n_items) decode(next, ph ^ 1);  // its loads run behind the flush
