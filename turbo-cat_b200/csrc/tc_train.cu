@@ -113,6 +113,7 @@ struct DevCfg {
   uint32_t nv;                   // validation rows (0: no validation set)
   int32_t es_rounds;             // early_stopping_rounds (< 0: never stop)
   int32_t es_min_iter;           // first iteration the stopping rule may fire at
+  int32_t advance;               // 1: the plan after the last level starts the next iteration
   int32_t sampled;               // 1: only the rows of smask grow this iteration's trees
 };
 
@@ -1136,7 +1137,7 @@ __global__ void __launch_bounds__(PART_THREADS) k_partition(DevCfg c, DevPtrs P,
 // node) in flight at once and reduces by shuffles; levels of at most 16 pairs
 // take one block per class and no exchange between blocks before the plan.
 // With a block per pair and nine block barriers per sum: 75 us an iteration
-// on 50k x 20, here 60.
+// on 50k x 20, here 53 with the plan.
 constexpr int RED_WARPS = 16;   // 128 registers: a pair's loads are all in flight
 constexpr int RED_CHUNKS = 10;  // partition blocks / 32 at most
 
@@ -1201,10 +1202,20 @@ __device__ __forceinline__ void pair_reduce(const DevCfg& c, const DevPtrs& P, i
   }
   cl = __reduce_add_sync(0xffffffffu, cl);
   cr = __reduce_add_sync(0xffffffffu, cr);
-  gl = warp_sum(gl);
-  hl = warp_sum(hl);
-  gr = warp_sum(gr);
-  hr = warp_sum(hr);
+  // four sums in 9 shuffles: the upper lanes take the right child's, then
+  // every other eight lanes H
+  {
+    const bool up = lane & 16, sw = lane & 8;
+    double x = (up ? gr : gl) + __shfl_xor_sync(0xffffffffu, up ? gl : gr, 16);
+    double y = (up ? hr : hl) + __shfl_xor_sync(0xffffffffu, up ? hl : hr, 16);
+    x = (sw ? y : x) + __shfl_xor_sync(0xffffffffu, sw ? x : y, 8);
+#pragma unroll
+    for (int o = 4; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    gl = x;
+    hl = __shfl_sync(0xffffffffu, x, 8);
+    gr = __shfl_sync(0xffffffffu, x, 16);
+    hr = __shfl_sync(0xffffffffu, x, 24);
+  }
   const bool sm = cl > cr;  // the smaller child: 1 = right
   if (lane == 0) {
     // an empty child has zero sums (its parent's histogram row is not
@@ -1247,10 +1258,19 @@ __device__ __forceinline__ void pair_reduce(const DevCfg& c, const DevPtrs& P, i
 constexpr int kPlanSegs = 4096;  // (class, pair) segment lengths the plan keeps in shared memory
 constexpr int kPlanTries = 16;   // candidates for the rows per chunk, a warp each
 
+// What bounds it: a chain of loads, shuffles and barriers on one SM while the
+// others wait, and its instructions, which are fetched anew where the block
+// that finishes last happens to run: so the code is there once, short, and
+// without 64-bit shuffles, shared 64-bit atomics or a search, and a finished
+// tree's leaves take the whole block.  With a second copy of the code for
+// single blocks, a warp per class for the leaves and the counter kernel of its
+// own behind it: 98 -> 78 us of reductions an iteration on 2.5M x 200, 115 ->
+// 72 on 1M x 50 with ten classes; a whole iteration 1125 -> 1095 and 1931 ->
+// 1880, 50k x 20 197 -> 188, 1M x 100 578 -> 546.
 __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int d) {
-  __shared__ long long s_rows;
-  __shared__ int s_nodes;
-  __shared__ int s_live;            // non-empty segments of the level
+  __shared__ uint32_t s_krows[kSoftmaxMaxK];  // rows of a class's segments (0: it grows no more)
+  __shared__ int s_klive[kSoftmaxMaxK];       // its non-empty segments, -1: it grows no more
+  __shared__ int s_kleaf[kSoftmaxMaxK];       // 1 + depth of a tree completed here, else 0
   __shared__ int s_warp[32];
   __shared__ int s_len[kPlanSegs];  // [class][pair] rows of level d (0: the class grows no more)
   const int Pmax = 1 << (c.D - 1);
@@ -1259,8 +1279,6 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   const int np2 = pairs_at(d);
   const int nsg = c.K * np2;
   const bool cached = nsg <= kPlanSegs;
-  if (tid == 0) { s_rows = 0; s_nodes = 0; s_live = 0; }
-  __syncthreads();
   // Per class, one warp each (classes w, w + warps, ...): no block barriers.
   for (int k = warp; k < c.K; k += nwarps) {
     ClassState& cs = P.cs[k];
@@ -1268,17 +1286,24 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     const NodeStat* nd = P.nstat + ((size_t)k * (c.D + 1) + d) * L;
     // (read before the state is known: one round of loads)
     const uint32_t tot = P.nstat[((size_t)k * (c.D + 1)) * L].cnt;  // rows of the level (the root's count)
-    const int len0 = d > 0 && lane < np2 ? P.seg_len[k * Pmax + lane] : (int)c.n;
+    int len4[4];  // segments lane, 32 + lane, ...
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int p = 32 * j + lane;
+      len4[j] = p >= np2 || d >= c.D ? 0 : d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
+    }
     uint32_t maxcnt = 0;
     int go = 0, hot = INT32_MAX;  // the largest node, the lowest index on a tie
+    if (d < c.D) {
 #pragma unroll 4
-    for (int q = lane; q < (1 << d); q += 32) {
-      const uint32_t cnt = nd[q].cnt;
-      const float H = (float)nd[q].H;
-      if (cnt >= (uint32_t)c.msl * 2u && H >= c.mcw * 2.0f) go = 1;
-      if (cnt > maxcnt || hot == INT32_MAX) {
-        maxcnt = cnt;
-        hot = q;
+      for (int q = lane; q < (1 << d); q += 32) {
+        const uint32_t cnt = nd[q].cnt;
+        const float H = (float)nd[q].H;
+        if (cnt >= (uint32_t)c.msl * 2u && H >= c.mcw * 2.0f) go = 1;
+        if (cnt > maxcnt || hot == INT32_MAX) {
+          maxcnt = cnt;
+          hot = q;
+        }
       }
     }
     if (d == 0) { done = 0; depth = 0; }
@@ -1296,66 +1321,85 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
       go = 0;
     }
     if (!done && !(alive && go)) done = 1;
-    if (done == 1) {
-      // the tree is complete: its leaves (src/tree/symmetric_tree.cpp:357-367, 753-775)
-      const int t = *P.iter * c.KT + c.k0 + k;
-      const NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + depth) * L;
-      for (int q = lane; q < L; q += 32) {
-        float v = 0.0f;
-        if (q < (1 << depth)) {
-          const double H = ns[q].H;
-          if (H >= 1e-10) {
-            double x = -ns[q].G / (H + (double)c.lam);
-            const double l1 = (double)c.l1;
-            if (l1 > 0) x = x > l1 ? x - l1 : (x < -l1 ? x + l1 : 0.0);
-            const double md = (double)c.mds;
-            if (md > 0) x = fmax(-md, fmin(md, x));
-            v = (float)x;
-          }
-        }
-        P.m_leaves[(size_t)t * L + q] = v;
-      }
-      if (lane == 0) P.m_depth[t] = depth;
-      done = 2;
-    }
+    int rows = 0, live = -1;
     if (!done) {
       // segment starts (exclusive scan over the pairs' lengths), 32 at a time
-      int carry = 0, live = 0;
+      live = 0;
       for (int base = 0; base < np2; base += 32) {
         const int p = base + lane;
-        const int len = p < np2 ? (base == 0 ? len0 : P.seg_len[k * Pmax + p]) : 0;
+        int len = 0;
+        if (base < 128) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) len = base == 32 * j ? len4[j] : len;
+        } else if (p < np2) {
+          len = P.seg_len[k * Pmax + p];
+        }
         int x = len;
+#pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const int y = __shfl_up_sync(0xffffffffu, x, o);
           if (lane >= o) x += y;
         }
         if (p < np2) {
-          P.seg_start[k * Pmax + p] = carry + x - len;
+          P.seg_start[k * Pmax + p] = rows + x - len;
           if (cached) s_len[k * np2 + p] = len;
         }
-        carry += __shfl_sync(0xffffffffu, x, 31);
+        rows += __shfl_sync(0xffffffffu, x, 31);
         live += __popc(__ballot_sync(0xffffffffu, len > 0));
-      }
-      if (lane == 0) {
-        atomicAdd(&s_live, live);
-        atomicAdd(reinterpret_cast<unsigned long long*>(&s_rows), (unsigned long long)carry);
-        atomicAdd(&s_nodes, np2);
       }
     } else if (cached) {
       for (int p = lane; p < np2; p += 32) s_len[k * np2 + p] = 0;
     }
-    __syncwarp();
     if (lane == 0) {
+      s_krows[k] = (uint32_t)rows;
+      s_klive[k] = live;
+      s_kleaf[k] = done == 1 ? 1 + depth : 0;
       if (d == 0) cs.depth = 0;
-      cs.done = done;
+      cs.done = done == 1 ? 2 : done;
+      if (done == 1) P.m_depth[*P.iter * c.KT + c.k0 + k] = depth;
     }
   }
   __syncthreads();
+  // the leaves of the trees complete (src/tree/symmetric_tree.cpp:357-367, 753-775)
+  long long n_rows = 0;
+  int n_live = 0, n_nodes = 0;
+  for (int k = 0; k < c.K; ++k) {
+    n_rows += s_krows[k];
+    n_live += max(s_klive[k], 0);
+    n_nodes += s_klive[k] >= 0 ? np2 : 0;
+    if (s_kleaf[k] == 0) continue;
+    const int depth = s_kleaf[k] - 1;
+    const int t = *P.iter * c.KT + c.k0 + k;
+    const NodeStat* ns = P.nstat + ((size_t)k * (c.D + 1) + depth) * L;
+    for (int q = tid; q < L; q += (int)blockDim.x) {
+      float v = 0.0f;
+      if (q < (1 << depth)) {
+        const double H = ns[q].H;
+        if (H >= 1e-10) {
+          double x = -ns[q].G / (H + (double)c.lam);
+          const double l1 = (double)c.l1;
+          if (l1 > 0) x = x > l1 ? x - l1 : (x < -l1 ? x + l1 : 0.0);
+          const double md = (double)c.mds;
+          if (md > 0) x = fmax(-md, fmin(md, x));
+          v = (float)x;
+        }
+      }
+      P.m_leaves[(size_t)t * L + q] = v;
+    }
+  }
+  if (d >= c.D) {
+    // the last level: nothing to plan (the counters below are not read)
+    if (c.advance) {
+      __syncthreads();
+      if (tid == 0) *P.iter += 1;
+    }
+    return;
+  }
   // rows of segment sgi (class, pair) for the chunking below
   auto seg_rows = [&](int sgi) -> int {
     if (cached) return s_len[sgi];
     const int k = sgi / np2, p = sgi % np2;
-    if (P.cs[k].done) return 0;
+    if (s_klive[k] < 0) return 0;
     return d == 0 ? (int)c.n : P.seg_len[k * Pmax + p];
   };
   // Rows per chunk R for this level.  `load` is a block's even share of the
@@ -1372,27 +1416,28 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
   // add an item each.
   // Sixteen candidates for that R, 1 to 4.5 times the start, a warp each (one
   // barrier instead of a search with three per step; R need not be exact).
-  __shared__ long long s_items[kPlanTries];
+  __shared__ uint32_t s_chunks[kPlanTries];
   const int waves = max(1, c.target_items / c.hist_grid);
   const int gw = waves == 1 || c.gwide == 0 ? c.G : c.gwide;
   // (FP32: neither the share nor R need more)
-  const float load = ((float)s_rows * (float)c.row_words * 0.125f + (float)s_live * (float)(c.G * kHistItemRows)) /
+  const float load = ((float)n_rows * (float)c.row_words * 0.125f + (float)n_live * (float)(c.G * kHistItemRows)) /
                          (float)c.hist_grid + 1.0f;
   const float r0 = fminf(fmaxf((float)c.rows_min, fminf(load, fmaxf(load / (float)waves, (float)kHistRowsSplit))),
                          (float)kHistRowsMax);
   long long allowed = (long long)fmaxf(1.0f, rintf(load / r0)) * c.hist_grid;
-  if (2LL * s_live * gw > allowed) allowed += (long long)s_live * gw;
+  if (2LL * n_live * gw > allowed) allowed += (long long)n_live * gw;
   auto candidate = [&](int j) { return (int)fminf((float)kHistRowsMax, r0 + r0 * (float)(j * j) * (1.0f / 64.0f)); };
   if (warp < kPlanTries) {
     const uint32_t Rt = (uint32_t)candidate(warp);
-    long long mine = 0;
+    uint32_t mine = 0;
     for (int sgi = lane; sgi < nsg; sgi += 32) mine += ((uint32_t)seg_rows(sgi) + Rt - 1) / Rt;
-    for (int o = 16; o; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-    if (lane == 0) s_items[warp] = mine * gw;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) s_chunks[warp] = mine;
   }
   __syncthreads();
-  int pick = 0;
-  while (pick < kPlanTries - 1 && s_items[pick] > allowed) ++pick;
+  // the first candidate whose items fit, else the last
+  const unsigned fit = __ballot_sync(0xffffffffu, lane < kPlanTries && (long long)s_chunks[lane & (kPlanTries - 1)] * gw <= allowed);
+  const int pick = fit ? __ffs(fit) - 1 : kPlanTries - 1;
   const int R = c.rows_fixed > 0 ? c.rows_fixed : candidate(pick);
   // cumulative item counts over segments (class, pair): chunks x groups
   int carry = 0;
@@ -1400,19 +1445,17 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     const int sgi = base + tid;
     const int chunks = sgi < nsg ? (int)(((uint32_t)seg_rows(sgi) + (uint32_t)R - 1) / (uint32_t)R) * c.G : 0;
     int x = chunks;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    int before = carry, all = 0;
-    for (int w = 0; w < nwarps; ++w) {
-      if (w < warp) before += s_warp[w];
-      all += s_warp[w];
-    }
+    const int w = lane < nwarps ? s_warp[lane] : 0;
+    const int before = carry + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
     if (sgi < nsg) P.cum[sgi] = before + x - chunks;
-    carry += all;
+    carry += __reduce_add_sync(0xffffffffu, w);
     if (base + (int)blockDim.x < nsg) __syncthreads();  // s_warp is written again
   }
   if (tid == 0) {
@@ -1420,8 +1463,8 @@ __device__ __forceinline__ void plan_body(const DevCfg& c, const DevPtrs& P, int
     P.cum[nsg] = carry;
     *P.hist_ctr = c.hist_grid;  // items 0 .. grid - 1 belong to the blocks by index
     if (d < 16) {
-      P.lvl_rows[d] = (uint64_t)s_rows;
-      P.lvl_nodes[d] = (uint32_t)s_nodes;
+      P.lvl_rows[d] = (uint64_t)n_rows;
+      P.lvl_nodes[d] = (uint32_t)n_nodes;
     }
   }
 }
@@ -1443,22 +1486,20 @@ __global__ void __launch_bounds__(32 * RED_WARPS) k_node_reduce(DevCfg c, DevPtr
   if (FUSE_PLAN) {
     if (gridDim.x * gridDim.y == 1) {
       __syncthreads();
-      plan_body(c, P, d + 1);
-      return;
-    }
-    __shared__ bool s_last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      const uint32_t prev = atomicAdd(P.red_ctr, 1u);
-      s_last = prev == gridDim.x * gridDim.y - 1;
-    }
-    __syncthreads();
-    if (s_last) {
+    } else {
+      __shared__ bool s_last;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        __threadfence();
+        const uint32_t prev = atomicAdd(P.red_ctr, 1u);
+        s_last = prev == gridDim.x * gridDim.y - 1;
+      }
+      __syncthreads();
+      if (!s_last) return;
       __threadfence();
       if (threadIdx.x == 0) *P.red_ctr = 0;  // re-armed for the next launch / graph replay
-      plan_body(c, P, d + 1);
     }
+    plan_body(c, P, d + 1);
   }
 }
 
@@ -2080,7 +2121,10 @@ tc_status tc_trainer::enqueue_rest(cudaStream_t st) {
   mark_begin(KC_REDUCE, st);
   k_node_reduce<true><<<dim3(1, K), 32 * RED_WARPS, 0, st>>>(cfg, ptr, -1);  // + plan of level 0
   mark_end(st);
-  for (int d = 0; d < D; ++d) launch_level(cfg, ptr, d, st);
+  DevCfg c = cfg;
+  c.advance = cfg.nv == 0 ? 1 : 0;
+  for (int d = 0; d < D; ++d) launch_level(c, ptr, d, st);
+  if (c.advance) return TC_OK;
   if (cfg.nv > 0) {
     mark_begin(KC_OTHER, st);
     k_valid<<<VALID_BLOCKS, 256, 0, st>>>(cfg, ptr);
