@@ -48,12 +48,13 @@ __device__ __forceinline__ float key_float(uint32_t k) {
 
 // X [n][f] row-major -> keys [f][n] via shared-memory tiles of 128 rows x 32
 // features, 16 loads of a thread in flight (32 x 32 tiles with four: 390 us on
-// 100M values, 320 here).
+// 100M values, 320 so).  The feature groups of a tile's rows are adjacent
+// blocks, so the lines that two groups share are read once: 320 -> 290 us.
 constexpr int MK_ROWS = 128;
 __global__ void __launch_bounds__(256) k_make_keys(const float* __restrict__ X, uint32_t n, uint32_t f,
                                                    uint32_t* __restrict__ keys) {
   __shared__ uint32_t t[MK_ROWS][33];
-  const uint32_t r0 = blockIdx.x * MK_ROWS, c0 = blockIdx.y * 32;
+  const uint32_t groups = (f + 31) / 32, r0 = blockIdx.x / groups * MK_ROWS, c0 = blockIdx.x % groups * 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float v[MK_ROWS / 8];
 #pragma unroll
@@ -1060,7 +1061,7 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   TC_CUDA(ctx, cudaMemsetAsync(ds->edges.p, 0, ds->edges.bytes(), st));
 
   if (n > 0) {
-    k_make_keys<<<dim3((n + MK_ROWS - 1) / MK_ROWS, (f + 31) / 32), 256, 0, st>>>(ds->X.p, n, f, ka.p);
+    k_make_keys<<<(n + MK_ROWS - 1) / MK_ROWS * ((f + 31) / 32), 256, 0, st>>>(ds->X.p, n, f, ka.p);
     uint32_t* src = ka.p;
     uint32_t* dst = kb.p;
     for (int shift = 0; shift < 32; shift += 8) {
