@@ -818,90 +818,107 @@ __global__ void k_cat_tile_sums(const float* __restrict__ X, const float* __rest
   }
 }
 
-// Exclusive scan of the tile totals of each column, in place (one thread per
-// column: a few thousand tiles).
+// Exclusive scan of the tile totals of each column, in place: a warp per
+// column, 32 tiles at a time (a thread walking them alone: 60 us at 245 tiles,
+// 7 so).
 __global__ void k_cat_tile_scan(long long* __restrict__ tsum, uint32_t* __restrict__ tcnt, uint32_t n_tiles) {
-  if (threadIdx.x != 0) return;
+  const uint32_t lane = threadIdx.x;
   long long a = 0;
   uint32_t b = 0;
   long long* ts = tsum + (size_t)blockIdx.x * n_tiles;
   uint32_t* tc = tcnt + (size_t)blockIdx.x * n_tiles;
-  for (uint32_t t = 0; t < n_tiles; ++t) {
-    const long long x = ts[t];
-    const uint32_t y = tc[t];
-    ts[t] = a;
-    tc[t] = b;
-    a += x;
-    b += y;
+  for (uint32_t t0 = 0; t0 < n_tiles; t0 += 32) {
+    const uint32_t t = t0 + lane;
+    const long long x = t < n_tiles ? ts[t] : 0;
+    const uint32_t y = t < n_tiles ? tc[t] : 0;
+    long long xs = x;
+    uint32_t ys = y;
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long xo = __shfl_up_sync(0xffffffffu, xs, o);
+      const uint32_t yo = __shfl_up_sync(0xffffffffu, ys, o);
+      if ((int)lane >= o) {
+        xs += xo;
+        ys += yo;
+      }
+    }
+    if (t < n_tiles) {
+      ts[t] = a + xs - x;
+      tc[t] = b + ys - y;
+    }
+    a += __shfl_sync(0xffffffffu, xs, 31);
+    b += __shfl_sync(0xffffffffu, ys, 31);
   }
 }
 
 // P[c][i] / C[c][i]: label sum / row count of the non-NaN rows at sorted
-// positions before i (i = 0 .. n).
+// positions before i (i = 0 .. n).  A warp takes 512 positions in a row, their
+// rows, values and labels loaded at once (sums within a tile fit 32 bits: the
+// labels' magnitudes sum to at most 2^24), one barrier for the warps' totals.
+// What bounds it: the gathers by row.  With 256 positions at a time and three
+// barriers for each: 78 us on four columns of 1M rows, 66 so.
 __global__ void k_cat_prefix(const float* __restrict__ X, const float* __restrict__ y, uint32_t n, uint32_t f,
                              const uint16_t* __restrict__ feats, const uint32_t* __restrict__ rows, uint32_t n_tiles,
                              const long long* __restrict__ toff, const uint32_t* __restrict__ tcoff,
                              long long* __restrict__ P, uint32_t* __restrict__ C) {
-  __shared__ long long ws[RS_THREADS / 32];
-  __shared__ uint32_t wc[RS_THREADS / 32];
-  __shared__ long long run_s;
-  __shared__ uint32_t run_c;
+  constexpr int NW = RS_THREADS / 32;
+  __shared__ int ws[NW];
+  __shared__ uint32_t wc[NW];
   const uint32_t c = blockIdx.y, tile = blockIdx.x, feat = feats[c];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const size_t base = (size_t)c * (n + 1);
-  if (threadIdx.x == 0) {
-    run_s = toff[(size_t)c * n_tiles + tile];
-    run_c = tcoff[(size_t)c * n_tiles + tile];
+  const uint32_t i0 = tile * RS_TILE + warp * (32 * RS_ITEMS) + lane;
+  uint32_t row[RS_ITEMS];
+  int v[RS_ITEMS];
+  uint32_t on = 0;  // bit per item: the row is not NaN
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) row[it] = i0 + 32 * it < n ? rows[(size_t)c * n + i0 + 32 * it] : 0u;
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) {
+    const bool in = i0 + 32 * it < n;
+    const float x = in ? X[(size_t)row[it] * f + feat] : 0.0f;
+    const float lab = in ? y[row[it]] : 0.0f;
+    const bool k = in && !isnan(x);
+    v[it] = k ? (int)lab : 0;
+    on |= (k ? 1u : 0u) << it;
+  }
+  int sv = 0;
+#pragma unroll
+  for (int it = 0; it < RS_ITEMS; ++it) sv += v[it];
+  sv = __reduce_add_sync(0xffffffffu, sv);
+  const uint32_t sc = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(on));
+  if (lane == 0) {
+    ws[warp] = sv;
+    wc[warp] = sc;
   }
   __syncthreads();
+  long long bs = toff[(size_t)c * n_tiles + tile];
+  uint32_t bc = tcoff[(size_t)c * n_tiles + tile];
+  for (int w = 0; w < warp; ++w) {
+    bs += ws[w];
+    bc += wc[w];
+  }
+#pragma unroll
   for (int it = 0; it < RS_ITEMS; ++it) {
-    const uint32_t idx = tile * RS_TILE + it * RS_THREADS + threadIdx.x;
-    long long v = 0;
-    uint32_t k = 0;
-    if (idx < n) {
-      const uint32_t row = rows[(size_t)c * n + idx];
-      if (!isnan(X[(size_t)row * f + feat])) {
-        v = (long long)y[row];
-        k = 1;
-      }
-    }
-    long long xs = v;
-    uint32_t xc = k;
+    const uint32_t idx = i0 + 32 * it;
+    const bool k = (on >> it) & 1u;
+    const unsigned m = __ballot_sync(0xffffffffu, k);
+    int xs = v[it];
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-      const long long a = __shfl_up_sync(0xffffffffu, xs, o);
-      const uint32_t b = __shfl_up_sync(0xffffffffu, xc, o);
-      if (lane >= o) {
-        xs += a;
-        xc += b;
-      }
-    }
-    if (lane == 31) {
-      ws[warp] = xs;
-      wc[warp] = xc;
-    }
-    __syncthreads();
-    long long bs = run_s;
-    uint32_t bc = run_c;
-    for (int w = 0; w < warp; ++w) {
-      bs += ws[w];
-      bc += wc[w];
+      const int a = __shfl_up_sync(0xffffffffu, xs, o);
+      if (lane >= o) xs += a;
     }
     if (idx < n) {
-      P[base + idx] = bs + xs - v;
-      C[base + idx] = bc + xc - k;
+      const uint32_t before = bc + __popc(m & ((1u << lane) - 1u));
+      P[base + idx] = bs + xs - v[it];
+      C[base + idx] = before;
       if (idx == n - 1) {
         P[base + n] = bs + xs;
-        C[base + n] = bc + xc;
+        C[base + n] = before + (k ? 1u : 0u);
       }
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int w = 0; w < RS_THREADS / 32; ++w) {
-        run_s += ws[w];
-        run_c += wc[w];
-      }
-    }
-    __syncthreads();
+    bs += __shfl_sync(0xffffffffu, xs, 31);
+    bc += __popc(m);
   }
 }
 
