@@ -53,3 +53,23 @@ def test_kept_blocks_count_against_the_budget(capi):
         eng.upload(np.repeat(X, 6, axis=0)[:5000])
     eng.upload(X).close()
     eng.close()
+
+
+def test_the_longest_kept_blocks_make_room(capi):
+    """More than 4 GiB released: at most 4 GiB stay mapped, and a block of
+    another size released after that is kept all the same."""
+    import torch
+
+    eng = capi.Engine(0)
+    X = np.zeros((600_000, 256), np.float32)  # 586 MiB
+    eng.upload(X[:1000]).close()
+    free0 = torch.cuda.mem_get_info(0)[0]
+    for ds in [eng.upload(X) for _ in range(8)]:
+        ds.close()
+    eng.upload(X[:250_000]).close()  # too small for any of the kept blocks
+    left = torch.cuda.mem_get_info(0)[0]
+    assert free0 - left <= (4 << 30) + (64 << 20)
+    ds = eng.upload(X[:250_000])
+    assert torch.cuda.mem_get_info(0)[0] == left
+    ds.close()
+    eng.close()

@@ -1,4 +1,5 @@
 // Context: device selection, stream, device-memory accounting, errors.
+#include <algorithm>
 #include <chrono>
 #include <thread>
 
@@ -24,7 +25,7 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
       // the smallest kept block that holds `bytes` with at most a quarter to spare
       const auto it = pool.lower_bound(bytes);
       if (it != pool.end() && it->first <= bytes + bytes / 4 + 4096 && (!budget || in_use + it->first <= budget)) {
-        *p = it->second;
+        *p = it->second.p;
         const size_t size = it->first;
         pool_bytes -= size;
         pool.erase(it);
@@ -59,6 +60,8 @@ void tc_ctx::release(void* p, bool pooled) {
   // a kept block may go to work on another stream (or a synchronous call) next:
   // wait for what the context's stream still does with it, as cudaFree would
   const bool idle = pooled && cudaStreamSynchronize(stream) == cudaSuccess;
+  std::vector<void*> back;  // kept blocks that make room for this one
+  bool keep = false;
   {
     std::lock_guard<std::mutex> g(mu);
     auto it = allocs.find(p);
@@ -66,25 +69,34 @@ void tc_ctx::release(void* p, bool pooled) {
       const size_t bytes = it->second;
       allocs.erase(it);
       in_use -= bytes;
-      if (idle && bytes <= tc::kPoolBlockMax && pool_bytes + bytes <= tc::kPoolMax &&
-          (!budget || in_use + pool_bytes + bytes <= budget)) {
-        pool.emplace(bytes, p);
+      const size_t room = !budget ? tc::kPoolMax : std::min(tc::kPoolMax, budget > in_use ? budget - in_use : 0);
+      keep = idle && bytes <= tc::kPoolBlockMax && bytes <= room;
+      if (keep) {
+        while (pool_bytes + bytes > room) {  // the longest kept first
+          auto old = pool.begin();
+          for (auto b = pool.begin(); b != pool.end(); ++b)
+            if (b->second.order < old->second.order) old = b;
+          back.push_back(old->second.p);
+          pool_bytes -= old->first;
+          pool.erase(old);
+        }
+        pool.emplace(bytes, tc::KeptBlock{p, pool_order++});
         pool_bytes += bytes;
-        return;
       }
     }
   }
-  cudaFree(p);
+  if (!keep) cudaFree(p);
+  for (void* q : back) cudaFree(q);
 }
 
 void tc_ctx::trim_pool() {
-  std::multimap<size_t, void*> blocks;
+  std::multimap<size_t, tc::KeptBlock> blocks;
   {
     std::lock_guard<std::mutex> g(mu);
     blocks.swap(pool);
     pool_bytes = 0;
   }
-  for (auto& kv : blocks) cudaFree(kv.second);
+  for (auto& kv : blocks) cudaFree(kv.second.p);
 }
 
 extern "C" {
