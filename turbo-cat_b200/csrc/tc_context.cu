@@ -57,8 +57,9 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
 
 void tc_ctx::release(void* p, bool pooled) {
   if (!p) return;
-  // a kept block may go to work on another stream (or a synchronous call) next:
-  // wait for what the context's stream still does with it, as cudaFree would
+  // wait for what the context's stream still does with the block: its next owner
+  // may hand it to a synchronous call.  (Nothing else is waited for, so pooled
+  // memory must not be written on any other stream, the default one included.)
   const bool idle = pooled && cudaStreamSynchronize(stream) == cudaSuccess;
   std::vector<void*> back;  // kept blocks that make room for this one
   bool keep = false;

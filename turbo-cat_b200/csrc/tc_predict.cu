@@ -1662,7 +1662,7 @@ static tc_status predict_small(tc_ctx* ctx, const tc_model* m, const float* X, u
     // [256 B counter][partials: SMs x SMALL_ROWS x PRED_MAX_K][inputs: in_cap]
     const size_t bytes = 256 + ((size_t)ctx->sm_count * SMALL_ROWS * PRED_MAX_K + in_cap) * sizeof(float);
     TC_TRY(ctx->alloc(&ctx->small_scratch, bytes, "small predict partials"));
-    TC_CUDA(ctx, cudaMemset(ctx->small_scratch, 0, bytes));
+    TC_CUDA(ctx, cudaMemsetAsync(ctx->small_scratch, 0, bytes, ctx->pred_stream));
     ctx->small_scratch_bytes = bytes;
   }
   cudaStream_t st = ctx->pred_stream;

@@ -1851,7 +1851,7 @@ tc_status tc_trainer::setup(int) {
   TC_TRY(hist0.alloc(ctx, hsz, "level histograms"));
   TC_TRY(hist1.alloc(ctx, hsz, "level histograms"));
   TC_TRY(acc.alloc(ctx, hsz, "histogram accumulators"));
-  TC_CUDA(ctx, cudaMemset(acc.p, 0, acc.bytes()));
+  TC_CUDA(ctx, cudaMemsetAsync(acc.p, 0, acc.bytes(), ctx->stream));
   TC_TRY(rchunk.alloc(ctx, 1, "chunk rows"));
   TC_TRY(seg_start.alloc(ctx, (size_t)K * Pmax, "segments"));
   TC_TRY(seg_len.alloc(ctx, (size_t)K * Pmax, "segments"));
@@ -1877,11 +1877,11 @@ tc_status tc_trainer::setup(int) {
   TC_TRY(m_leaves.alloc(ctx, (size_t)T_cap * L, "model"));
   TC_TRY(lvl_rows.alloc(ctx, 16, "level rows"));
   TC_TRY(lvl_nodes.alloc(ctx, 16, "level nodes"));
-  TC_CUDA(ctx, cudaMemset(lvl_rows.p, 0, lvl_rows.bytes()));
-  TC_CUDA(ctx, cudaMemset(lvl_nodes.p, 0, lvl_nodes.bytes()));
-  TC_CUDA(ctx, cudaMemset(counters.p, 0, counters.bytes()));
-  TC_CUDA(ctx, cudaMemset(red_ctr.p, 0, red_ctr.bytes()));
-  TC_CUDA(ctx, cudaMemset(fcnt.p, 0, fcnt.bytes()));
+  TC_CUDA(ctx, cudaMemsetAsync(lvl_rows.p, 0, lvl_rows.bytes(), ctx->stream));
+  TC_CUDA(ctx, cudaMemsetAsync(lvl_nodes.p, 0, lvl_nodes.bytes(), ctx->stream));
+  TC_CUDA(ctx, cudaMemsetAsync(counters.p, 0, counters.bytes(), ctx->stream));
+  TC_CUDA(ctx, cudaMemsetAsync(red_ctr.p, 0, red_ctr.bytes(), ctx->stream));
+  TC_CUDA(ctx, cudaMemsetAsync(fcnt.p, 0, fcnt.bytes(), ctx->stream));
 
   ptr.bins_t = ds->bins_t.p; ptr.bins_cm = ds->bins_cm.p; ptr.edges = ds->edges.p; ptr.n_edges = ds->n_edges.p;
   ptr.nan_any = ds->nan_any.p;
