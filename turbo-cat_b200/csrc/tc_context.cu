@@ -22,15 +22,19 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
       return TC_ERR_OOM;
     }
     if (pooled) {
-      // the smallest kept block that holds `bytes` with at most a quarter to spare
+      // the smallest kept block that holds `bytes` with at most a quarter to
+      // spare; under a budget only one of that very size, since what a block is
+      // larger would count against the budget and so make what fits depend on
+      // the blocks of earlier objects
+      const size_t spare = budget ? 0 : bytes / 4 + 4096;
       const auto it = pool.lower_bound(bytes);
-      if (it != pool.end() && it->first <= bytes + bytes / 4 + 4096 && (!budget || in_use + it->first <= budget)) {
+      if (it != pool.end() && it->first <= bytes + spare) {
         *p = it->second.p;
         const size_t size = it->first;
         pool_bytes -= size;
         pool.erase(it);
-        allocs[*p] = size;
-        in_use += size;
+        allocs[*p] = tc::Block{bytes, size};
+        in_use += bytes;
         if (in_use > peak) peak = in_use;
         return TC_OK;
       }
@@ -49,7 +53,7 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
     return fail(TC_ERR_OOM, "cudaMalloc(%zu) for %s: %s", bytes, what, cudaGetErrorString(e));
   }
   std::lock_guard<std::mutex> g(mu);
-  allocs[*p] = bytes;
+  allocs[*p] = tc::Block{bytes, bytes};
   in_use += bytes;
   if (in_use > peak) peak = in_use;
   return TC_OK;
@@ -67,9 +71,9 @@ void tc_ctx::release(void* p, bool pooled) {
     std::lock_guard<std::mutex> g(mu);
     auto it = allocs.find(p);
     if (it != allocs.end()) {
-      const size_t bytes = it->second;
+      in_use -= it->second.asked;
+      const size_t bytes = it->second.size;
       allocs.erase(it);
-      in_use -= bytes;
       const size_t room = !budget ? tc::kPoolMax : std::min(tc::kPoolMax, budget > in_use ? budget - in_use : 0);
       keep = idle && bytes <= tc::kPoolBlockMax && bytes <= room;
       if (keep) {

@@ -23,6 +23,11 @@ constexpr int kMaxClasses = 64;
 
 inline size_t round_up(size_t x, size_t m) { return (x + m - 1) / m * m; }
 
+// A device block in use: the bytes asked for (what in_use counts) and its size,
+// which is larger when a kept block of more bytes serves the request.
+struct Block {
+  size_t asked, size;
+};
 // A device block kept for reuse; order: when it was kept.
 struct KeptBlock {
   void* p;
@@ -41,7 +46,7 @@ struct tc_ctx {
   cudaStream_t pred_stream = nullptr;  // tc_predict / tc_predict_device (NULL stream)
   std::string err;
   std::mutex mu;                     // guards allocation accounting and err
-  std::map<void*, size_t> allocs;
+  std::map<void*, tc::Block> allocs;
   // training calls (tc_train, tc_build_tree, tc_trainer_*) on one context
   // run one at a time: they share the context's stream and tuner state
   std::recursive_mutex train_mu;
