@@ -73,8 +73,12 @@ const char* tc_last_error(const tc_ctx* ctx);
 /* Bytes currently allocated by the context and its objects, and the peak.
  * Buffers that a destroyed object gave back and the context keeps for its next
  * one (at most 4 GiB; they count against the budget and are given back to the
- * device when an allocation needs the room) are not among them. */
+ * device when an allocation of this or another context of the process needs the
+ * room, or by tc_ctx_trim) are not among them. */
 tc_status tc_ctx_memory(const tc_ctx* ctx, size_t* in_use, size_t* peak);
+/* Gives the kept buffers back to the device, for a host whose other libraries
+ * need the memory; objects that are alive are not touched. */
+tc_status tc_ctx_trim(tc_ctx* ctx);
 /* Fault-injection hook for host-side tests: the next `count` device
  * allocations made through this context fail with TC_ERR_OOM. */
 tc_status tc_ctx_fail_next_allocs(tc_ctx* ctx, int count);

@@ -748,6 +748,11 @@ void print_info() {
   py::print("TurboCat B200 engine: symmetric-tree training and inference on sm_100a (libtcgpu.so)");
 }
 
+void release_device_memory() {
+  std::lock_guard<std::mutex> g(g_ctx_mu);
+  if (g_ctx) check(tc_ctx_trim(g_ctx), g_ctx);
+}
+
 }  // namespace
 
 // ------------------------------------------------------------------- metrics
@@ -857,6 +862,8 @@ PYBIND11_MODULE(_turbocat, m) {
       .def_property_readonly("train_seconds", &TurboCatRegressor::train_seconds);
 
   m.def("print_info", &print_info, "Print TurboCat library information");
+  m.def("release_device_memory", &release_device_memory,
+        "Give the device buffers kept between fits back to the device");
 
   auto metrics = m.def_submodule("metrics", "Evaluation metrics for TurboCat");
   py::enum_<MetricType>(metrics, "MetricType")

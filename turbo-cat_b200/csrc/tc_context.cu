@@ -5,6 +5,19 @@
 
 #include "tc_internal.h"
 
+namespace {
+// The process's contexts: an allocation that fails in one takes the blocks that
+// the others keep on its device.
+std::mutex g_contexts_mu;
+std::vector<tc_ctx*> g_contexts;
+
+void trim_all(int device) {
+  std::lock_guard<std::mutex> g(g_contexts_mu);
+  for (tc_ctx* c : g_contexts)
+    if (c->device == device) c->trim_pool();
+}
+}  // namespace
+
 tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
   bool trim = false;
   {
@@ -45,7 +58,7 @@ tc_status tc_ctx::alloc(void** p, size_t bytes, const char* what, bool pooled) {
   cudaError_t e = cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();
-    trim_pool();
+    trim_all(device);
     e = cudaMalloc(p, bytes);
   }
   if (e != cudaSuccess) {
@@ -132,12 +145,20 @@ tc_status tc_ctx_create(int device, size_t mem_budget, tc_ctx** out) {
     delete c;
     return TC_ERR_CUDA;
   }
+  {
+    std::lock_guard<std::mutex> g(g_contexts_mu);
+    g_contexts.push_back(c);
+  }
   *out = c;
   return TC_OK;
 }
 
 void tc_ctx_destroy(tc_ctx* ctx) {
   if (!ctx) return;
+  {
+    std::lock_guard<std::mutex> g(g_contexts_mu);
+    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+  }
   cudaSetDevice(ctx->device);
   {
     std::lock_guard<std::mutex> g(ctx->pred_mu);
@@ -169,6 +190,13 @@ tc_status tc_ctx_memory(const tc_ctx* ctx, size_t* in_use, size_t* peak) {
   if (!ctx) return TC_ERR_INVALID_ARG;
   if (in_use) *in_use = ctx->in_use;
   if (peak) *peak = ctx->peak;
+  return TC_OK;
+}
+
+tc_status tc_ctx_trim(tc_ctx* ctx) {
+  if (!ctx) return TC_ERR_INVALID_ARG;
+  cudaSetDevice(ctx->device);
+  ctx->trim_pool();
   return TC_OK;
 }
 

@@ -103,8 +103,8 @@ struct tc_ctx {
   // blocks of at most kPoolBlockMax are kept, the longest kept ones make room
   // for new ones (a context that has served other shapes before would else free
   // every buffer of the present ones: tc_quantize 7.4 instead of 3.6 ms), and all
-  // are given back when an allocation fails or would pass the budget, and with
-  // the context.
+  // are given back when an allocation fails (of any context on the device) or
+  // would pass the budget, by tc_ctx_trim, and with the context.
   tc_status alloc(void** p, size_t bytes, const char* what, bool pooled = false);
   void release(void* p, bool pooled = false);
   void trim_pool();                         // gives every kept block back to the device

@@ -19,6 +19,7 @@ from ._turbocat import (  # noqa: E402  (fails loudly when the extension is not 
     TurboCatClassifier as _TurboCatClassifier,
     TurboCatRegressor as _TurboCatRegressor,
     print_info,
+    release_device_memory,
 )
 
 
@@ -193,4 +194,4 @@ class TurboCatRegressor:
         return self
 
 
-__all__ = ["TurboCatClassifier", "TurboCatRegressor", "print_info", "__version__"]
+__all__ = ["TurboCatClassifier", "TurboCatRegressor", "print_info", "release_device_memory", "__version__"]

@@ -24,7 +24,7 @@ TRANSFORM = {"raw": 0, "sigmoid": 1, "softmax": 2}
 
 # every symbol include/tcgpu.h declares
 SYMBOLS = [
-    "tc_ctx_create", "tc_ctx_destroy", "tc_last_error", "tc_ctx_memory", "tc_ctx_fail_next_allocs",
+    "tc_ctx_create", "tc_ctx_destroy", "tc_last_error", "tc_ctx_memory", "tc_ctx_trim", "tc_ctx_fail_next_allocs",
     "tc_ctx_synchronize", "tc_ctx_set_latency_worker", "tc_dataset_upload", "tc_dataset_destroy", "tc_quantize",
     "tc_apply_bins", "tc_dataset_bins", "tc_dataset_features", "tc_encode_categorical", "tc_category_table",
     "tc_trainer_create", "tc_trainer_step", "tc_trainer_reset", "tc_trainer_stats", "tc_trainer_profile",
@@ -375,6 +375,10 @@ class Engine:
         a, b = C.c_size_t(), C.c_size_t()
         self._chk(lib().tc_ctx_memory(self.ctx, C.byref(a), C.byref(b)))
         return a.value, b.value
+
+    def trim(self):
+        """Gives the device buffers kept for reuse back to the device."""
+        self._chk(lib().tc_ctx_trim(self.ctx))
 
     def fail_next_allocs(self, k):
         self._chk(lib().tc_ctx_fail_next_allocs(self.ctx, C.c_int(k)))
