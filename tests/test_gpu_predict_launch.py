@@ -1,0 +1,53 @@
+"""Launch shapes of the tile prediction kernel, by their times on the device
+(the least of many; each bound lies between the two shapes' measured ratios)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _sms():
+    import torch
+
+    return torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def _model(engine, capi, T, D, F, levels=0):
+    """T trees; thresholds of `levels` values a feature (0: all different, so
+    many that the model has no binned form)."""
+    rng = np.random.default_rng(T + D)
+    feature = rng.integers(0, F, (T, D)).astype(np.uint16)
+    thr = rng.standard_normal((T, D)).astype(np.float32)
+    if levels:
+        q = np.sort(rng.standard_normal((F, levels)).astype(np.float32), 1)
+        thr = q[feature, rng.integers(0, levels, (T, D))]
+    a = dict(depth=np.full(T, D, np.int32), feature=feature, threshold=thr,
+             leaves=rng.standard_normal((T, 1 << D)).astype(np.float32), weights=np.full(T, 0.1, np.float32))
+    return engine.import_model(capi.ModelInfo(T, 1, D, F, 0, 0.0, 0.1, 1.0), a)
+
+
+def _least_us(m, n, F, reps=12):
+    import torch
+
+    X = torch.randn(n, F, device="cuda")
+    out = torch.empty(n, device="cuda")
+    st = torch.cuda.Stream()
+    t = []
+    for _ in range(reps):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record(st)
+        m.predict_device(X.data_ptr(), n, F, out.data_ptr(), "raw", st.cuda_stream)
+        b.record(st)
+        b.synchronize()
+        t.append(a.elapsed_time(b) * 1e3)
+    return min(t)
+
+
+def test_float_walk_takes_128_row_tiles(engine, capi):
+    """One 128-row tile more than the device has multiprocessors: about a third
+    longer than one each (two blocks share a multiprocessor), not twice, as
+    256-row tiles, which walk their halves one after the other, would take."""
+    F, rows = 100, _sms() * 128
+    m = _model(engine, capi, 7600, 10, F)
+    assert _least_us(m, rows + 128, F) < 1.65 * _least_us(m, rows, F)
+    m.close()
