@@ -51,3 +51,40 @@ def test_float_walk_takes_128_row_tiles(engine, capi):
     m = _model(engine, capi, 7600, 10, F)
     assert _least_us(m, rows + 128, F) < 1.65 * _least_us(m, rows, F)
     m.close()
+
+
+def test_rows_past_a_whole_wave(engine, capi):
+    """A 256-row tile for every multiprocessor and almost half as many rows
+    again: the rest in 128-row tiles takes about half as long again; as 256-row
+    tiles beside half of the others it took 1.8 times as long."""
+    F, rows = 37, _sms() * 256
+    m = _model(engine, capi, 1000, 10, F, 254)
+    assert _least_us(m, rows + rows // 2 - 128, F, 30) < 1.66 * _least_us(m, rows, F, 30)
+    m.close()
+
+
+def test_a_long_model_in_a_mixed_burst(engine, capi):
+    """A burst's tiles of a model of many trees end a burst of other rows: they
+    take 128 rows while the multiprocessors hold one each, and start first.  (A
+    256-row tile takes about 1.45 times as long.)"""
+    F, heavy_rows, light_rows = 8, 12_800, 15_000
+    heavy, light = _model(engine, capi, 30_000, 6, F, 254), _model(engine, capi, 200, 4, F, 254)
+    srv = capi.Server(engine, staging_bytes=0, max_batch_rows=131_072, coalesce=True, max_inflight=4)
+    h, li = srv.add_model(heavy), srv.add_model(light)
+    rng = np.random.default_rng(0)
+
+    def request(mid, n):
+        import torch
+
+        X = torch.empty((n, F), pin_memory=True).numpy()
+        X[:] = rng.standard_normal((n, F))
+        return 0.0, mid, X, torch.empty((n, 1), pin_memory=True).numpy(), "raw"
+
+    alone = [request(h, heavy_rows)]
+    # (a first request takes the server's first launch; the others share the next)
+    mixed = [request(li, 1)] + alone + [request(li, light_rows) for _ in range(4)]
+    t = [float(np.median([srv.replay(reqs)[1] for _ in range(25)])) for reqs in (alone, mixed)]
+    assert t[1] < 1.25 * t[0], t
+    srv.close()
+    heavy.close()
+    light.close()

@@ -261,7 +261,7 @@ struct ReqDesc {
   const float* X;     // device pointer to the request's rows [n][f]
   float* out;         // device pointer to its outputs [n][K]
   uint32_t n;
-  uint32_t row_begin; // first global row of this request in the batch
+  uint32_t wide;      // its first tiles: so many of 256 rows, then 128-row ones
   int32_t model;      // index into the model table
   int32_t transform;
 };
@@ -282,23 +282,30 @@ struct ModelDesc {
   int32_t bin_stride;
 };
 // Launch shape of a batch: dynamic shared memory and stage sizes that fit
-// every model of the batch, and the largest tile they allow.
+// every model of the batch.
 struct PredictPlan {
   size_t smem;
   int leaf_stage;   // floats of one leaf stage
   int split_stage;  // 8-byte units of one split stage
   int chunk;        // trees per chunk at most
   int stage_rows;   // rows staged at a time (binned walk)
-  int max_tile;     // 256 rows, or 128
 };
 PredictPlan predict_plan(const tc_model* const* models, int n);
-// Rows of a launch's tiles, from its count of 128-row tiles.
-int predict_tile_rows(const tc_ctx* ctx, const PredictPlan& plan, uint64_t tiles_of_half);
-uint32_t predict_tiles(uint32_t n, int tile_rows);
+// One request of a launch, as its tiles are cut.
+struct TileJob {
+  float cost;     // of a 256-row tile of its model, up to a factor
+  bool narrow;    // 128-row tiles only
+  uint32_t n;
+  uint32_t wide;  // its 256-row tiles (set by predict_tiling)
+};
+TileJob tile_job(const tc_model* m, uint32_t n);
+// Sets every job's 256-row tiles and the order in which the jobs' tiles start.
+void predict_tiling(const tc_ctx* ctx, TileJob* jobs, int* order, int n_jobs);
+uint32_t predict_tiles(const TileJob& j);
 // Coalesced prediction over a request table: job j covers tiles
-// [tile_begin[j], tile_begin[j+1]) of tile_rows rows each.
+// [tile_begin[j], tile_begin[j+1]).
 tc_status predict_batched(tc_ctx* ctx, const ModelDesc* d_models, const ReqDesc* d_reqs, int n_reqs,
-                          const uint32_t* d_tile_begin, int tile_rows, uint32_t n_tiles, const PredictPlan& plan,
+                          const uint32_t* d_tile_begin, uint32_t n_tiles, const PredictPlan& plan,
                           cudaStream_t stream);
 ModelDesc model_desc(const tc_model* m);
 

@@ -104,7 +104,6 @@ struct JobTable {
   int split_stage;             // 8-byte units of one split stage
   int chunk;                   // trees per chunk at most
   int stage_rows;              // rows staged at a time (binned walk): 128 or 64
-  int tile_rows;               // rows of a tile: PRED_ROWS or PRED_HALF
   ReqDesc one_req;
   ModelDesc one_model;
 };
@@ -498,11 +497,12 @@ __global__ void __launch_bounds__(PRED_THREADS, 2) k_predict(JobTable jt) {
     md = jt.models[rq.model];
     tile = blockIdx.x - jt.tile_begin[lo];
   }
-  const uint32_t r0 = tile * (uint32_t)jt.tile_rows;
+  const bool wide = tile < rq.wide;
+  const uint32_t r0 = wide ? tile * PRED_ROWS : rq.wide * PRED_ROWS + (tile - rq.wide) * PRED_HALF;
   if (r0 >= rq.n) return;
-  const int nr = (int)min((uint32_t)jt.tile_rows, rq.n - r0);
+  const int nr = (int)min((uint32_t)(wide ? PRED_ROWS : PRED_HALF), rq.n - r0);
   if (md.bsplits == nullptr) {
-    for (int h0 = 0; h0 < nr; h0 += PRED_HALF) float_tile(jt, rq, md, r0 + h0, min(PRED_HALF, nr - h0), smp);
+    float_tile(jt, rq, md, r0, nr, smp);
   } else if (md.bin_stride == PRED_HALF) {
     binned_tile<1, PRED_HALF>(jt, rq, md, r0, nr, smp);
   } else if (nr > PRED_HALF) {
@@ -958,14 +958,12 @@ size_t model_smem(int n_features, int n_classes, int n_virtual, int n_bord, int 
 constexpr size_t PRED_SMEM_MAX = 220 * 1024;
 constexpr size_t PRED_SMEM_TWO = 112 * 1024;  // two blocks per SM
 
-tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, int tile_rows, uint32_t n_tiles,
-                         cudaStream_t stream) {
+tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, uint32_t n_tiles, cudaStream_t stream) {
   if (n_tiles == 0) return TC_OK;
   jt.leaf_stage = plan.leaf_stage;
   jt.split_stage = plan.split_stage;
   jt.chunk = plan.chunk;
   jt.stage_rows = plan.stage_rows;
-  jt.tile_rows = tile_rows;
   static bool attr_done = false;
   if (!attr_done) {
     cudaFuncSetAttribute(k_predict, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PRED_SMEM_MAX);
@@ -983,13 +981,8 @@ tc_status launch_predict(tc_ctx* ctx, JobTable& jt, const PredictPlan& plan, int
 }  // namespace
 
 PredictPlan predict_plan(const tc_model* const* models, int n) {
-  int max_depth = 0, max_tile = PRED_ROWS;
-  for (int i = 0; i < n; ++i) {
-    max_depth = std::max(max_depth, models[i]->info.max_depth);
-    // (the float walk takes 128 rows at a time: a larger tile is two of them one
-    // after the other, half as many blocks; 20k rows, 12000 x d13: 7.4 ms, 4.1 so)
-    max_tile = std::min(max_tile, models[i]->bin_stride ? models[i]->bin_stride : PRED_HALF);
-  }
+  int max_depth = 0;
+  for (int i = 0; i < n; ++i) max_depth = std::max(max_depth, models[i]->info.max_depth);
   // the first layout that leaves room for two blocks per SM, else the first that fits
   PredictPlan best{};
   for (const Layout& y : kLayouts) {
@@ -997,7 +990,6 @@ PredictPlan predict_plan(const tc_model* const* models, int n) {
     p.leaf_stage = y.leaf_stage;
     p.chunk = y.chunk;
     p.stage_rows = y.stage_rows;
-    p.max_tile = max_tile;
     p.split_stage = split_stage(max_depth, y);
     for (int i = 0; i < n; ++i) {
       const tc_model* m = models[i];
@@ -1010,27 +1002,75 @@ PredictPlan predict_plan(const tc_model* const* models, int n) {
   return best;
 }
 
-// Rows of a tile: 256, or 128 while that leaves at most one tile per SM: then
-// more SMs beat more rows per split (1000 x d6, device buffers, 128- and
-// 256-row tiles: 4096 rows 27 and 38 us, 16384 rows 27 and 39, 32768 rows 44
-// and 40).
-int predict_tile_rows(const tc_ctx* ctx, const PredictPlan& plan, uint64_t tiles_of_half) {
-  if (plan.max_tile < PRED_ROWS) return PRED_HALF;
-  return tiles_of_half <= (uint64_t)ctx->sm_count ? PRED_HALF : PRED_ROWS;
+TileJob tile_job(const tc_model* m, uint32_t n) {
+  // a tree costs about its levels and a leaf
+  return TileJob{(float)m->info.n_trees * (float)(m->info.max_depth + 1), m->bin_stride != PRED_ROWS, n, 0};
+}
+
+namespace {
+uint32_t half_tiles(uint32_t n) { return n / PRED_HALF + (n % PRED_HALF ? 1 : 0); }
+}  // namespace
+
+uint32_t predict_tiles(const TileJob& j) {
+  const uint64_t rows = (uint64_t)j.wide * PRED_ROWS;
+  return j.wide + (j.n > rows ? half_tiles((uint32_t)(j.n - rows)) : 0u);
+}
+
+// A launch's tiles.  256 rows cost fewer instructions a row, 128-row tiles spread
+// over more multiprocessors, so 128 rows are taken where they leave none with
+// two tiles:
+//  * for a model whose 256-row tile would take longer than a multiprocessor's even
+//    share of the launch, while the 128-row tiles of all such models are at most
+//    one per multiprocessor (1000 x d6 alone, 128- and 256-row tiles: 16384 rows
+//    27 and 39 us; with two 128-row tiles on a multiprocessor no more: 32768 rows
+//    44 and 40);
+//  * for the rows past the last whole wave of 256-row tiles, while they are
+//    fewer 128-row tiles than multiprocessors, the cheapest models' rows (50k rows,
+//    1000 x d10, 196 tiles of 256 rows and 148 with 95 half ones: 136 and 114 us;
+//    147 half ones 105 and 148 of them, every block slot taken, 125 as before).
+// The tiles that take longest start first.  Bursts on models of 200 x d4 to
+// 2000 x d10, all tiles of one size and in the order of the requests, and so: 60
+// requests of 77k rows of 20 features 845 -> 737 us, 69k x 32 856 -> 738, 12 of
+// 23k x 73 425 -> 370.
+void predict_tiling(const tc_ctx* ctx, TileJob* jobs, int* order, int n_jobs) {
+  const uint64_t sms = (uint64_t)ctx->sm_count;
+  double work = 0.0;
+  for (int j = 0; j < n_jobs; ++j) {
+    work += (double)jobs[j].cost * jobs[j].n / PRED_ROWS;
+    order[j] = j;
+  }
+  const double share = work / (double)sms;
+  uint64_t longer = 0, rest = 0;
+  for (int j = 0; j < n_jobs; ++j)
+    if (jobs[j].cost >= share) longer += half_tiles(jobs[j].n);
+  for (int j = 0; j < n_jobs; ++j) {
+    jobs[j].wide = jobs[j].narrow || (jobs[j].cost >= share && longer <= sms) ? 0 : half_tiles(jobs[j].n) / 2;
+    if (jobs[j].wide) rest += half_tiles(jobs[j].n);
+  }
+  auto time = [&](int j) { return jobs[j].wide ? jobs[j].cost : 0.6f * jobs[j].cost; };
+  if (n_jobs > 1)
+    std::stable_sort(order, order + n_jobs, [&](int a, int b) { return time(a) > time(b); });
+  rest %= 2 * sms;  // 128-row tiles past the last whole wave
+  if (rest >= sms) return;
+  for (int q = n_jobs - 1; q >= 0 && rest > 0; --q) {
+    TileJob& j = jobs[order[q]];
+    if (j.wide == 0) continue;
+    const uint64_t h = half_tiles(j.n), cut = std::min(h, rest);
+    j.wide = (uint32_t)((h - cut) / 2);
+    rest -= cut;
+  }
 }
 
 tc_status predict_batched(tc_ctx* ctx, const ModelDesc* d_models, const ReqDesc* d_reqs, int n_reqs,
-                          const uint32_t* d_tile_begin, int tile_rows, uint32_t n_tiles, const PredictPlan& plan,
+                          const uint32_t* d_tile_begin, uint32_t n_tiles, const PredictPlan& plan,
                           cudaStream_t stream) {
   JobTable jt{};
   jt.reqs = d_reqs;
   jt.models = d_models;
   jt.tile_begin = d_tile_begin;
   jt.n_jobs = n_reqs;
-  return launch_predict(ctx, jt, plan, tile_rows, n_tiles, stream);
+  return launch_predict(ctx, jt, plan, n_tiles, stream);
 }
-
-uint32_t predict_tiles(uint32_t n, int tile_rows) { return (n + tile_rows - 1) / tile_rows; }
 
 }  // namespace tc
 
@@ -1215,10 +1255,11 @@ tc_status predict_device(tc_ctx* ctx, const tc_model* m, const float* X, uint32_
   jt.reqs = nullptr;
   jt.n_jobs = 1;
   jt.one_model = model_desc(m);
-  jt.one_req = ReqDesc{X, out, n, 0, 0, transform};
-  const PredictPlan plan = predict_plan(&m, 1);
-  const int rows = predict_tile_rows(ctx, plan, predict_tiles(n, PRED_HALF));
-  return launch_predict(ctx, jt, plan, rows, predict_tiles(n, rows), stream);
+  TileJob job = tile_job(m, n);
+  int order = 0;
+  predict_tiling(ctx, &job, &order, 1);
+  jt.one_req = ReqDesc{X, out, n, job.wide, 0, transform};
+  return launch_predict(ctx, jt, predict_plan(&m, 1), predict_tiles(job), stream);
 }
 
 }  // namespace tc

@@ -58,6 +58,9 @@ struct Slot {
   ReqDesc* h_reqs = nullptr;
   uint32_t* h_tiles = nullptr;
   std::vector<Request*> reqs;
+  std::vector<uint32_t> row0;    // first row of each request in the staging buffers
+  std::vector<TileJob> jobs;
+  std::vector<int> order;        // the requests in the order of the table
   bool busy = false;
 };
 
@@ -74,6 +77,7 @@ struct tc_server {
   std::vector<std::unique_ptr<Slot>> slots;
   std::vector<ModelDesc> models;
   std::vector<const tc_model*> model_ptrs;
+  std::vector<TileJob> tile_jobs;  // per model, without rows
   AnyStreamBuf<ModelDesc> d_models;
   std::mutex mu;
   std::condition_variable cv_work;   // worker wake-up
@@ -101,12 +105,13 @@ static bool is_pinned(const void* p) {
 }
 
 bool tc_server::launch(Slot& s, std::vector<Request*>& batch) {
-  uint32_t row = 0, tile = 0;
-  int j = 0;
-  uint64_t half_tiles = 0;
-  for (Request* r : batch) half_tiles += predict_tiles(r->n, 128);
-  const int tile_rows = predict_tile_rows(ctx, plan, half_tiles);
-  for (Request* r : batch) {
+  const int nb = (int)batch.size();
+  uint32_t row = 0;
+  s.row0.resize(nb);
+  s.jobs.resize(nb);
+  s.order.resize(nb);
+  for (int j = 0; j < nb; ++j) {
+    Request* r = batch[j];
     float* din = s.d_in.p + (size_t)row * max_f;
     const size_t bytes = (size_t)r->n * r->f * sizeof(float);
     if (r->pinned_in) {
@@ -115,25 +120,34 @@ bool tc_server::launch(Slot& s, std::vector<Request*>& batch) {
       std::memcpy(s.h_in + (size_t)row * max_f, r->X, bytes);
       cudaMemcpyAsync(din, s.h_in + (size_t)row * max_f, bytes, cudaMemcpyHostToDevice, s.stream);
     }
-    s.h_reqs[j] = ReqDesc{din, s.d_out.p + (size_t)row * 16, r->n, row, r->model, r->transform};
-    s.h_tiles[j] = tile;
-    tile += predict_tiles(r->n, tile_rows);
+    s.row0[j] = row;
+    s.jobs[j] = tile_jobs[r->model];
+    s.jobs[j].n = r->n;
     row += r->n;
-    ++j;
   }
-  s.h_tiles[j] = tile;
-  cudaMemcpyAsync(s.d_reqs.p, s.h_reqs, j * sizeof(ReqDesc), cudaMemcpyHostToDevice, s.stream);
-  cudaMemcpyAsync(s.d_tiles.p, s.h_tiles, (j + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s.stream);
-  if (predict_batched(ctx, d_models.p, s.d_reqs.p, j, s.d_tiles.p, tile_rows, tile, plan, s.stream) != TC_OK)
-    return false;
-  for (int q = 0; q < j; ++q) {
-    Request* r = batch[q];
+  // the table lists the requests in the order their tiles start
+  predict_tiling(ctx, s.jobs.data(), s.order.data(), nb);
+  uint32_t tile = 0;
+  for (int q = 0; q < nb; ++q) {
+    const int j = s.order[q];
+    const Request* r = batch[j];
+    s.h_reqs[q] = ReqDesc{s.d_in.p + (size_t)s.row0[j] * max_f, s.d_out.p + (size_t)s.row0[j] * 16, r->n,
+                          s.jobs[j].wide, r->model, r->transform};
+    s.h_tiles[q] = tile;
+    tile += predict_tiles(s.jobs[j]);
+  }
+  s.h_tiles[nb] = tile;
+  cudaMemcpyAsync(s.d_reqs.p, s.h_reqs, nb * sizeof(ReqDesc), cudaMemcpyHostToDevice, s.stream);
+  cudaMemcpyAsync(s.d_tiles.p, s.h_tiles, (nb + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s.stream);
+  if (predict_batched(ctx, d_models.p, s.d_reqs.p, nb, s.d_tiles.p, tile, plan, s.stream) != TC_OK) return false;
+  for (int j = 0; j < nb; ++j) {
+    Request* r = batch[j];
     const size_t bytes = (size_t)r->n * r->K * sizeof(float);
-    const float* src = s.d_out.p + (size_t)s.h_reqs[q].row_begin * 16;
+    const float* src = s.d_out.p + (size_t)s.row0[j] * 16;
     if (r->pinned_out) {
       cudaMemcpyAsync(r->out, src, bytes, cudaMemcpyDeviceToHost, s.stream);
     } else {
-      cudaMemcpyAsync(s.h_out + (size_t)s.h_reqs[q].row_begin * 16, src, bytes, cudaMemcpyDeviceToHost, s.stream);
+      cudaMemcpyAsync(s.h_out + (size_t)s.row0[j] * 16, src, bytes, cudaMemcpyDeviceToHost, s.stream);
     }
   }
   cudaEventRecord(s.done, s.stream);
@@ -148,8 +162,7 @@ void tc_server::complete(Slot& s) {
   const auto now = Clock::now();
   for (Request* r : s.reqs) {
     if (!r->pinned_out) {
-      // rows of request q start at its row_begin in the slot
-      std::memcpy(r->out, s.h_out + (size_t)s.h_reqs[q].row_begin * 16, (size_t)r->n * r->K * sizeof(float));
+      std::memcpy(r->out, s.h_out + (size_t)s.row0[q] * 16, (size_t)r->n * r->K * sizeof(float));
     }
     n_rows.fetch_add(r->n);
     ++q;
@@ -275,6 +288,7 @@ tc_status tc_server_add_model(tc_server* s, const tc_model* m, int32_t* model_id
   cudaSetDevice(ctx->device);
   s->models.push_back(model_desc(m));
   s->model_ptrs.push_back(m);
+  s->tile_jobs.push_back(tile_job(m, 0));
   s->max_f = std::max(s->max_f, m->info.n_features);
   s->max_depth = std::max(s->max_depth, m->info.max_depth);
   s->plan = predict_plan(s->model_ptrs.data(), (int)s->model_ptrs.size());
