@@ -289,7 +289,9 @@ __device__ void float_tile(const JobTable& jt, const ReqDesc& rq, const ModelDes
     const float* lvc = leaves_global ? md.leaves + (size_t)t0 * L : s_leaf + buf * LS;
     const uint2* spc = s_split + buf * SS;
     if (row < nr) {
-      for (int t = tg; t < tn; t += TG) {
+      // tree t belongs to group t % TG of the whole ensemble, so a row's sum does
+      // not depend on the chunks, which the launch's models share
+      for (int t = (tg - t0) & (TG - 1); t < tn; t += TG) {
         const uint2* sp = spc + t * D;
         uint32_t idx = 0;
 #pragma unroll
