@@ -63,6 +63,18 @@ def test_rows_past_a_whole_wave(engine, capi):
     m.close()
 
 
+def test_few_tiles_take_the_larger_chunks(engine, capi):
+    """With at most a block per multiprocessor the room for a second one is worth
+    nothing: 73 features (two blocks fit, with the smallest chunks of trees) take
+    no longer than 120 (they do not fit)."""
+    t = []
+    for F in (73, 120):
+        m = _model(engine, capi, 2000, 10, F, 254)
+        t.append(_least_us(m, 200, F, 30))
+        m.close()
+    assert t[0] < 1.15 * t[1], t
+
+
 def test_a_long_model_in_a_mixed_burst(engine, capi):
     """A burst's tiles of a model of many trees end a burst of other rows: they
     take 128 rows while the multiprocessors hold one each, and start first.  (A

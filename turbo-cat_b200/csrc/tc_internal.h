@@ -290,7 +290,8 @@ struct PredictPlan {
   int chunk;        // trees per chunk at most
   int stage_rows;   // rows staged at a time (binned walk)
 };
-PredictPlan predict_plan(const tc_model* const* models, int n);
+// one_each: for launches of at most one block per multiprocessor.
+PredictPlan predict_plan(const tc_model* const* models, int n, bool one_each);
 // One request of a launch, as its tiles are cut.
 struct TileJob {
   float cost;     // of a 256-row tile of its model, up to a factor

@@ -73,7 +73,7 @@ struct tc_server {
   int req_cap = 1024;
   int max_f = 0;
   int max_depth = 0;
-  PredictPlan plan{};
+  PredictPlan plan[2] = {};        // of launches of more blocks than multiprocessors, and of the others
   std::vector<std::unique_ptr<Slot>> slots;
   std::vector<ModelDesc> models;
   std::vector<const tc_model*> model_ptrs;
@@ -139,7 +139,9 @@ bool tc_server::launch(Slot& s, std::vector<Request*>& batch) {
   s.h_tiles[nb] = tile;
   cudaMemcpyAsync(s.d_reqs.p, s.h_reqs, nb * sizeof(ReqDesc), cudaMemcpyHostToDevice, s.stream);
   cudaMemcpyAsync(s.d_tiles.p, s.h_tiles, (nb + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s.stream);
-  if (predict_batched(ctx, d_models.p, s.d_reqs.p, nb, s.d_tiles.p, tile, plan, s.stream) != TC_OK) return false;
+  if (predict_batched(ctx, d_models.p, s.d_reqs.p, nb, s.d_tiles.p, tile, plan[tile <= (uint32_t)ctx->sm_count ? 1 : 0],
+                      s.stream) != TC_OK)
+    return false;
   for (int j = 0; j < nb; ++j) {
     Request* r = batch[j];
     const size_t bytes = (size_t)r->n * r->K * sizeof(float);
@@ -291,7 +293,8 @@ tc_status tc_server_add_model(tc_server* s, const tc_model* m, int32_t* model_id
   s->tile_jobs.push_back(tile_job(m, 0));
   s->max_f = std::max(s->max_f, m->info.n_features);
   s->max_depth = std::max(s->max_depth, m->info.max_depth);
-  s->plan = predict_plan(s->model_ptrs.data(), (int)s->model_ptrs.size());
+  for (int i = 0; i < 2; ++i)
+    s->plan[i] = predict_plan(s->model_ptrs.data(), (int)s->model_ptrs.size(), i == 1);
   TC_CUDA(ctx, cudaMemcpy(s->d_models.p, s->models.data(), s->models.size() * sizeof(ModelDesc),
                           cudaMemcpyHostToDevice));
   *model_id = (int32_t)s->models.size() - 1;
