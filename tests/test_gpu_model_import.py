@@ -1,0 +1,125 @@
+"""Importing a model: the binned form is built in less time than the rest of the
+import takes, several classes keep within a budget that holds the model alone,
+and the arrays are complete on the device when the call returns."""
+import time
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _arrays(capi, T, D, F, K, levels=254, seed=0):
+    rng = np.random.default_rng(seed + T + D + F)
+    q = np.sort(rng.standard_normal((F, max(levels, 1))).astype(np.float32), 1)
+    feature = rng.integers(0, F, (T, D)).astype(np.uint16)
+    thr = q[feature, rng.integers(0, max(levels, 1), (T, D))]
+    if not levels:
+        thr[:] = np.nan  # every split's bit is 0: nothing to sort, one empty virtual feature
+    a = dict(depth=np.full(T, D, np.int32), feature=feature, bin=np.zeros((T, D), np.uint8), threshold=thr,
+             gain=np.zeros((T, D), np.float32), leaves=rng.standard_normal((T, 1 << D)).astype(np.float32),
+             weights=np.full(T, 0.1, np.float32))
+    return capi.ModelInfo(T, K, D, F, 1 if K > 1 else 0, 0.0, 0.1, 1.0), a
+
+
+def _median_import(engine, info, a, reps=21):
+    t = []
+    for _ in range(reps):
+        t0 = time.perf_counter()
+        m = engine.import_model(info, a)
+        t.append(time.perf_counter() - t0)
+        m.close()
+    return sorted(t)[reps // 2]
+
+
+@pytest.mark.parametrize("T,D,F,K", [(2000, 6, 50, 10), (2000, 6, 120, 3)])
+def test_the_binned_form_is_quick_to_build(engine, capi, T, D, F, K):
+    """Against the same model without thresholds (3 times as long before)."""
+    with_thresholds = _median_import(engine, *_arrays(capi, T, D, F, K))
+    without = _median_import(engine, *_arrays(capi, T, D, F, K, levels=0))
+    assert with_thresholds < 2.0 * without
+
+
+def test_several_classes_within_a_budget_for_one_copy(engine, capi):
+    """Under a budget that holds the splits and one copy of the leaves, a model
+    of several classes is imported all the same and predicts within FP32
+    rounding of the one with room."""
+    T, D, F, K = 3000, 8, 20, 3
+    info, a = _arrays(capi, T, D, F, K)
+    X = np.random.default_rng(5).standard_normal((400, F)).astype(np.float32)
+    m = engine.import_model(info, a)
+    want = m.predict(X, "raw")
+    m.close()
+    once = T * D * 8 + T * (1 << D) * 4
+    staging = 1 << 20  # the host path's device staging, allocated with the first prediction
+    eng = capi.Engine(0, mem_budget=once + staging + 1024)
+    m = eng.import_model(info, a)
+    got = m.predict(X, "raw")
+    mag = 0.1 * np.abs(a["leaves"]).max(1).sum()
+    assert np.abs(got - want).max() <= 2 * T * 2.0 ** -24 * mag
+    m.close()
+    eng.close()
+    tight = capi.Engine(0, mem_budget=once - 1024)
+    with pytest.raises(capi.TCError):
+        tight.import_model(info, a)
+    tight.close()
+
+
+def _walk64(a, X, K):
+    out = np.zeros((len(X), K))
+    for t in range(len(a["depth"])):
+        idx = np.zeros(len(X), np.int64)
+        for d in range(a["depth"][t]):
+            with np.errstate(invalid="ignore"):
+                idx = 2 * idx + (X[:, a["feature"][t, d]] >= a["threshold"][t, d])
+        out[:, t % K] += a["leaves"][t, idx].astype(np.float64) * float(a["weights"][t])
+    return out
+
+
+@pytest.mark.parametrize("T,D,F,K", [(1, 1, 1, 1), (5, 9, 2, 3), (130, 13, 4, 4), (257, 8, 300, 1), (40, 3, 65535, 2)])
+def test_threshold_ranks(engine, capi, T, D, F, K):
+    """Signed zeros, infinities, denormals, NaN thresholds, features of exactly
+    127, 128 and 254 distinct thresholds, classes of unequal tree counts."""
+    info, a = _arrays(capi, T, D, F, K, levels=min(254, 127 + T % 128), seed=3)
+    rng = np.random.default_rng(T)
+    special = np.array([0.0, -0.0, np.inf, -np.inf, 1e-42, -1e-42, np.nan, 3.4e38], np.float32)
+    pick = rng.random((T, D)) < 0.2
+    a["threshold"][pick] = rng.choice(special, pick.sum())
+    a["depth"] = rng.integers(0, D + 1, T).astype(np.int32)
+    X = rng.standard_normal((300, min(F, 400))).astype(np.float32)
+    X[:, ::3] = rng.choice(special, X[:, ::3].shape)
+    n = 300 if F <= 400 else 3
+    if F > 400:
+        X = np.zeros((n, F), np.float32)
+        X[:, a["feature"].ravel()] = rng.standard_normal((n, a["feature"].size))
+    m = engine.import_model(info, a)
+    want = _walk64(a, X, K)
+    for rows in ((65, 300) if F <= 400 else ()):
+        got = m.predict(X[:rows], "raw")
+        assert np.abs(got - want[:rows]).max() <= (T + 8) * 2.0 ** -24 * (1 + 0.1 * np.abs(a["leaves"]).max(1).sum())
+    m.close()
+
+
+def test_complete_when_the_call_returns(engine, capi):
+    """The first prediction after an import, on the prediction stream and on
+    another one, while the default stream is busy."""
+    import torch
+
+    info, a = _arrays(capi, 1500, 9, 30, 1)
+    X = torch.randn(5000, 30, device="cuda")
+    ref = engine.import_model(info, a)
+    want = torch.empty(5000, device="cuda")
+    ref.predict_device(X.data_ptr(), 5000, 30, want.data_ptr(), "raw", 1)
+    torch.cuda.synchronize()
+    st = torch.cuda.Stream()
+    got = [torch.empty(5000, device="cuda") for _ in range(2)]
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)
+    m = engine.import_model(info, a)
+    m.predict_device(X.data_ptr(), 5000, 30, got[0].data_ptr(), "raw", 0)
+    m.predict_device(X.data_ptr(), 5000, 30, got[1].data_ptr(), "raw", st.cuda_stream)
+    torch.cuda.synchronize()
+    for o in got:
+        assert torch.equal(o, want)
+    m.close()
+    ref.close()

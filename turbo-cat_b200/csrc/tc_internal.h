@@ -107,6 +107,10 @@ struct tc_ctx {
   // would pass the budget, by tc_ctx_trim, and with the context.
   tc_status alloc(void** p, size_t bytes, const char* what, bool pooled = false);
   void release(void* p, bool pooled = false);
+  bool has_room(size_t bytes) {             // whether the budget leaves `bytes`
+    std::lock_guard<std::mutex> g(mu);
+    return !budget || in_use + bytes <= budget;
+  }
   void trim_pool();                         // gives every kept block back to the device
   std::multimap<size_t, tc::KeptBlock> pool;  // kept blocks by size (guarded by mu)
   size_t pool_bytes = 0;
@@ -217,24 +221,26 @@ struct tc_model {
   std::vector<float> weights;       // [T]
   std::vector<float> edges;         // [f][255]
   std::vector<uint16_t> n_edges;    // [f]
-  // device copies used by the predict kernels
-  AnyStreamBuf<uint2> d_splits;           // [T][D] (feature, threshold bits), padded to depth D
-  AnyStreamBuf<float> d_leaves;           // [T][2^D] (weights folded in, padded trees' leaves spread)
-  AnyStreamBuf<uint32_t> d_bsplits;       // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class
-  AnyStreamBuf<float> d_bleaves;          // binned form, several classes: leaves in the order of d_bsplits
-  AnyStreamBuf<float> d_bord;             // binned form: borders of every virtual feature, Eytzinger order
-  AnyStreamBuf<uint2> d_vdesc;            // binned form: (feature, border offset | search steps << 24)
+  // device arrays used by the predict kernels, in one allocation
+  AnyStreamBuf<uint8_t> d_mem;
+  const uint2* d_splits = nullptr;        // [T][D] (feature, threshold bits), padded to depth D
+  const float* d_leaves = nullptr;        // [T][2^D] (weights folded in, padded trees' leaves spread)
+  const uint32_t* d_bsplits = nullptr;    // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class
+  const float* d_bleaves = nullptr;       // binned form: leaves in the order of d_bsplits (one class: d_leaves)
+  const float* d_bord = nullptr;          // binned form: borders of every virtual feature, Eytzinger order
+  const uint2* d_vdesc = nullptr;         // binned form: (feature, border offset | search steps << 24)
   int n_virtual = 0, n_bord = 0;
   int bin_stride = 0;               // bytes of a bin column: 256 or 128 rows (0: no binned form)
   // regular (depth-wise) trees of a model the reference trained with
   // mode="small" (served for prediction only; tc_predict.cu)
   bool regular = false;
   std::vector<uint8_t> tcat;        // the stream as loaded (saved back byte for byte)
-  AnyStreamBuf<uint4> d_rnodes;           // (feature | bin << 16 | leaf << 24, left, right, value bits), global indices
-  AnyStreamBuf<uint32_t> d_rroots;        // [T] first node of each tree
-  AnyStreamBuf<float> d_rweights;         // [T]
-  AnyStreamBuf<float> d_redges;           // [f][255] bin edges
-  AnyStreamBuf<int32_t> d_rnedges;        // [f]
+  const uint4* d_rnodes = nullptr;        // (feature | bin << 16 | leaf << 24, left, right, value bits), global indices
+  int n_rnodes = 0;
+  const uint32_t* d_rroots = nullptr;     // [T] first node of each tree
+  const float* d_rweights = nullptr;      // [T]
+  const float* d_redges = nullptr;        // [f][255] bin edges
+  const int32_t* d_rnedges = nullptr;     // [f]
   tc_status upload();
 };
 

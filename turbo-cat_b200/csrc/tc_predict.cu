@@ -57,6 +57,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <memory>
 
 #include "tc_internal.h"
 
@@ -923,6 +924,14 @@ __global__ void __launch_bounds__(128) k_predict_regular(RegDesc rd, const float
   out[r0 + r] = transform == TC_TRANSFORM_SIGMOID ? sigmoidf_ref(raw) : raw;
 }
 
+// The leaves of a model of K classes, tree t of class t % K, class by class.
+__global__ void k_class_leaves(const float* __restrict__ from, float* __restrict__ to, int n_trees, int L, int K) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)n_trees * L) return;
+  const int t = (int)(i / L), per = n_trees / K, more = n_trees - per * K, k = t % K;
+  to[((size_t)k * per + min(k, more) + t / K) * L + i % L] = from[i];
+}
+
 // One way to lay out a block's shared memory: floats of a leaf stage (at least
 // the warps' sums of a tile), trees per chunk at most, rows staged at a time.
 // Larger chunks cost fewer barriers and copies per tree (64 trees of depth 6 a
@@ -1083,16 +1092,77 @@ using namespace tc;
 
 namespace {
 
-// Fills t[base + 1 .. base + n) (n = 2^h) with vals in Eytzinger
-// (breadth-first) order, node 1 the root: an in-order walk of the implicit
-// tree visits vals in sorted order.
-void eytzinger_fill(const std::vector<float>& vals, std::vector<float>& t, size_t base, size_t n, size_t i,
-                    size_t& next) {
+// Fills t[1 .. n) (n = 2^h) with the cnt values in Eytzinger (breadth-first)
+// order, node 1 the root, NaN past them: an in-order walk of the implicit tree
+// visits vals in sorted order.
+void eytzinger_fill(const float* vals, int cnt, float* t, size_t n, size_t i, int& next) {
   if (i >= n) return;
-  eytzinger_fill(vals, t, base, n, 2 * i, next);
-  t[base + i] = next < vals.size() ? vals[next] : std::nanf("");
+  eytzinger_fill(vals, cnt, t, n, 2 * i, next);
+  t[i] = next < cnt ? vals[next] : std::nanf("");
   ++next;
-  eytzinger_fill(vals, t, base, n, 2 * i + 1, next);
+  eytzinger_fill(vals, cnt, t, n, 2 * i + 1, next);
+}
+
+// A model's device arrays, each on a 16-byte boundary of one block: laid out
+// (part; device_part, after those, for what the device writes itself), filled on
+// the host (at), then allocated and copied at once.
+struct ModelImage {
+  size_t size = 0, device_size = 0;
+  std::unique_ptr<uint8_t[]> host;
+  template <class T>
+  size_t part(size_t count) {
+    const size_t at = size;
+    size = device_size = align16(size + count * sizeof(T));
+    return at;
+  }
+  template <class T>
+  size_t device_part(size_t count) {
+    const size_t at = device_size;
+    device_size = align16(device_size + count * sizeof(T));
+    return at;
+  }
+  template <class T>
+  T* at(size_t offset) {
+    if (!host) host.reset(new uint8_t[size]);
+    return reinterpret_cast<T*>(host.get() + offset);
+  }
+  // (on pred_stream: the caller waits for it before the model is used)
+  tc_status upload(tc_ctx* ctx, AnyStreamBuf<uint8_t>& mem) {
+    TC_TRY(mem.alloc(ctx, device_size, "model arrays"));
+    TC_CUDA(ctx, cudaMemcpyAsync(mem.p, host.get(), size, cudaMemcpyHostToDevice, ctx->pred_stream));
+    return TC_OK;
+  }
+};
+
+// A split and its threshold as an unsigned key of the same order (-0.0 and +0.0
+// one key).
+struct SplitKey {
+  uint32_t key, at;
+};
+uint32_t threshold_key(float x) {
+  uint32_t u;
+  if (x == 0.0f) x = 0.0f;
+  std::memcpy(&u, &x, 4);
+  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+float key_threshold(uint32_t k) {
+  const uint32_t u = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
+  float x;
+  std::memcpy(&x, &u, 4);
+  return x;
+}
+
+// Stable counting pass of `in` to `out` by digit(entry); start: entries of each
+// digit, turned into the digits' places.
+template <class F>
+void counting_pass(const std::vector<SplitKey>& in, std::vector<SplitKey>& out, std::vector<uint32_t>& start, F digit) {
+  uint32_t run = 0;
+  for (uint32_t& s : start) {
+    const uint32_t n = s;
+    s = run;
+    run += n;
+  }
+  for (const SplitKey& s : in) out[start[digit(s)]++] = s;
 }
 
 }  // namespace
@@ -1103,107 +1173,152 @@ void eytzinger_fill(const std::vector<float>& vals, std::vector<float>& t, size_
 // (w * leaf in FP32, the product the reference forms per tree), the float
 // splits (feature, threshold bits) and the binned form (virtual features,
 // Eytzinger-ordered borders, binned splits).
+//
+// A program that trains or loads a model for each use pays for this every time:
+// the distinct thresholds come from a radix sort of all splits by (feature,
+// threshold), which also gives every split its rank; the arrays go to the device
+// as one block, and the second copy of several classes' leaves is made there.
+// With a sort and searches per feature and an allocation and a copy per array,
+// an import of 2000 x d6 in ten classes took 1690 us (520 without a binned
+// form), of 1000 x d6 900, of 2000 x d10 4800; here 760, 520 and 2250.
 tc_status tc_model::upload() {
-  const int T = info.n_trees, D = info.max_depth, L = 1 << D, F = info.n_features;
-  std::vector<uint2> sp((size_t)std::max(1, T * D));
-  std::vector<float> lv((size_t)std::max(1, T * L), 0.0f);
-  for (int t = 0; t < T; ++t) {
-    const int dt = depth[t];
-    for (int d = 0; d < D; ++d) {
-      uint32_t bits = kNaNBits, j = 0;
-      if (d < dt) {
-        std::memcpy(&bits, &threshold[(size_t)t * D + d], 4);
-        j = feature[(size_t)t * D + d];
-      }
-      sp[(size_t)t * D + d] = make_uint2(j, bits);
-    }
-    for (int l = 0; l < (1 << dt); ++l) lv[(size_t)t * L + ((size_t)l << (D - dt))] = weights[t] * leaves[(size_t)t * L + l];
-  }
-  TC_TRY(d_splits.alloc(ctx, sp.size(), "model splits"));
-  TC_TRY(d_leaves.alloc(ctx, lv.size(), "model leaves"));
-  TC_CUDA(ctx, cudaMemcpy(d_splits.p, sp.data(), sp.size() * sizeof(uint2), cudaMemcpyHostToDevice));
-  TC_CUDA(ctx, cudaMemcpy(d_leaves.p, lv.data(), lv.size() * sizeof(float), cudaMemcpyHostToDevice));
-  if (D < 1) return TC_OK;
-  // binned form: distinct thresholds per feature (-0.0 and +0.0 are one)
-  std::vector<std::vector<float>> u((size_t)F);
+  const int T = info.n_trees, D = info.max_depth, L = 1 << D, F = info.n_features, K = info.n_classes;
+  // the splits by feature and threshold
+  std::vector<SplitKey> a, b;
+  std::vector<uint32_t> n0(2048, 0u), n1(2048, 0u), n2(1024, 0u), nf((size_t)F, 0u);
+  a.reserve((size_t)T * D);
   for (int t = 0; t < T; ++t)
     for (int d = 0; d < depth[t]; ++d) {
-      const float th = threshold[(size_t)t * D + d];
-      if (!std::isnan(th)) u[feature[(size_t)t * D + d]].push_back(th);
+      const size_t at = (size_t)t * D + d;
+      if (std::isnan(threshold[at])) continue;
+      const uint32_t key = threshold_key(threshold[at]);
+      a.push_back({key, (uint32_t)at});
+      ++n0[key & 2047u];
+      ++n1[key >> 11 & 2047u];
+      ++n2[key >> 22];
+      ++nf[feature[at]];
     }
-  struct VF { int j, start, cnt; };
+  b.resize(a.size());
+  counting_pass(a, b, n0, [](const SplitKey& s) { return s.key & 2047u; });
+  counting_pass(b, a, n1, [](const SplitKey& s) { return s.key >> 11 & 2047u; });
+  counting_pass(a, b, n2, [](const SplitKey& s) { return s.key >> 22; });
+  counting_pass(b, a, nf, [this](const SplitKey& s) { return (uint32_t)feature[s.at]; });
+  // virtual features: the distinct thresholds of a feature, cut after every
+  // BIN_MAX_BORDERS; b[i].key = split a[i]'s virtual feature << 8 | 128 - rank in it
+  struct VF { int j, cnt; };
   std::vector<VF> vf;
-  std::vector<int> first_v((size_t)F, -1);
-  for (int j = 0; j < F; ++j) {
-    auto& a = u[j];
-    std::sort(a.begin(), a.end());
-    a.erase(std::unique(a.begin(), a.end(), [](float x, float y) { return x == y; }), a.end());
-    for (int s0 = 0; s0 < (int)a.size(); s0 += BIN_MAX_BORDERS) {
-      if (first_v[j] < 0) first_v[j] = (int)vf.size();
-      vf.push_back({j, s0, std::min(BIN_MAX_BORDERS, (int)a.size() - s0)});
+  std::vector<float> u;  // the distinct thresholds, virtual feature by virtual feature
+  for (size_t i = 0; i < a.size(); ++i) {
+    const int j = feature[a[i].at];
+    const bool same_feature = i > 0 && feature[a[i - 1].at] == j;
+    if (!same_feature || a[i - 1].key != a[i].key) {
+      if (!same_feature || vf.back().cnt == BIN_MAX_BORDERS) vf.push_back({j, 0});
+      ++vf.back().cnt;
+      u.push_back(key_threshold(a[i].key));
     }
+    b[i] = {(uint32_t)(vf.size() - 1) << 8 | (uint32_t)(128 - vf.back().cnt), a[i].at};
   }
-  if (vf.empty()) vf.push_back({0, 0, 0});  // padding splits read virtual feature 0
-  if ((int)vf.size() > BIN_MAX_VIRTUAL) return TC_OK;  // served by the float walk
-  std::vector<float> bord;
+  if (vf.empty()) vf.push_back({0, 0});  // padding splits read virtual feature 0
+  // border offsets and search steps; the binned form's shape, if it fits
+  const int V = (int)vf.size();
+  bool binned = D >= 1 && V <= BIN_MAX_VIRTUAL;
   std::vector<uint2> vd;
-  for (const VF& v : vf) {
+  size_t nb = 0;
+  for (int v = 0; v < V && binned; ++v) {
     int h = 0;
-    while ((1 << h) - 1 < v.cnt) ++h;
-    const size_t n = (size_t)1 << h, off = bord.size();
-    if (off + n >= ((size_t)1 << 24)) return TC_OK;
-    bord.resize(off + n, std::nanf(""));
-    std::vector<float> vals;
-    if (v.cnt) vals.assign(u[v.j].begin() + v.start, u[v.j].begin() + v.start + v.cnt);
-    size_t next = 0;
-    eytzinger_fill(vals, bord, off, n, 1, next);
-    vd.push_back(make_uint2((uint32_t)v.j, (uint32_t)off | ((uint32_t)h << 24)));
+    while ((1 << h) - 1 < vf[v].cnt) ++h;
+    vd.push_back(make_uint2((uint32_t)vf[v].j, (uint32_t)nb | ((uint32_t)h << 24)));
+    nb += (size_t)1 << h;
+    binned = nb < ((size_t)1 << 24);
   }
-  const int V = (int)vd.size(), B = (int)bord.size();
   int stride = 0;  // the widest bin columns of which some layout fits (none: the float walk)
   for (int st : {PRED_HALF, PRED_ROWS})
     for (const Layout& y : kLayouts)
-      if (model_smem(F, info.n_classes, V, B, st, y, split_stage(D, y)) <= PRED_SMEM_MAX) stride = st;
-  if (stride == 0) return TC_OK;
-  while (bord.size() % 4) bord.push_back(std::nanf(""));  // whole 16-byte copies
-  if (vd.size() % 2) vd.push_back(make_uint2(0, 0));
-  // binned splits in processing order: levels min(D,8)-1 .. 0, then D-1 .. 8;
-  // a tree's splits are padded to whole 8-byte units
+      if (binned && model_smem(F, K, V, (int)nb, st, y, split_stage(D, y)) <= PRED_SMEM_MAX) stride = st;
+  ModelImage im;
+  const size_t o_sp = im.part<uint2>((size_t)std::max(1, T * D)), o_lv = im.part<float>((size_t)std::max(1, T * L));
+  const size_t plain = im.size;
+  // binned splits: a tree's are padded to whole 8-byte units; borders and virtual
+  // features to whole 16-byte copies (parts are)
   const int DS = 2 * split_units(D, true);
-  std::vector<uint32_t> bs((size_t)T * DS, 0u);  // padding: k = 128, never reached by a bin
-  const int K = info.n_classes;
-  std::vector<int> order;  // class by class (tree t is class t % K)
-  for (int k = 0; k < K; ++k)
-    for (int t = k; t < T; t += K) order.push_back(t);
-  for (int q = 0; q < T; ++q) {
-    const int t = order[q];
-    for (int p = 0; p < D; ++p) {
-      const int lev = D <= 8 ? D - 1 - p : (p < 8 ? 7 - p : D - 1 - (p - 8));
-      if (lev >= depth[t]) continue;
-      const float th = threshold[(size_t)t * D + lev];
-      if (std::isnan(th)) continue;
-      const int j = feature[(size_t)t * D + lev];
-      const int r = (int)(std::lower_bound(u[j].begin(), u[j].end(), th) - u[j].begin());
-      const int v = first_v[j] + r / BIN_MAX_BORDERS;
-      bs[(size_t)q * DS + p] = (uint32_t)v << 8 | (uint32_t)(128 - r % BIN_MAX_BORDERS - 1);
+  size_t o_bs = 0, o_bl = o_lv, o_bd = 0, o_vd = 0;
+  if (stride) {
+    o_bs = im.part<uint32_t>(std::max<size_t>(2, (size_t)T * DS));
+    o_bd = im.part<float>(nb);
+    o_vd = im.part<uint2>((size_t)V);
+    if (K > 1) o_bl = im.device_part<float>((size_t)std::max(1, T * L));
+    // several classes are served by the float walk where the budget has no room
+    // for a second copy of their leaves
+    if (K > 1 && !ctx->has_room(im.device_size) && ctx->has_room(plain)) {
+      im.size = im.device_size = plain;
+      stride = 0;
     }
   }
-  TC_TRY(d_bsplits.alloc(ctx, std::max<size_t>(2, bs.size()), "binned model splits"));
-  if (K > 1) {
-    std::vector<float> bl(lv.size());
-    for (int q = 0; q < T; ++q) std::memcpy(&bl[(size_t)q * L], &lv[(size_t)order[q] * L], L * sizeof(float));
-    TC_TRY(d_bleaves.alloc(ctx, bl.size(), "binned model leaves"));
-    TC_CUDA(ctx, cudaMemcpy(d_bleaves.p, bl.data(), bl.size() * sizeof(float), cudaMemcpyHostToDevice));
+  uint2* sp = im.at<uint2>(o_sp);
+  float* lv = im.at<float>(o_lv);
+  if (T == 0) lv[0] = 0.0f;
+  if (T * D == 0) sp[0] = make_uint2(0, kNaNBits);
+  // the binned form lists the trees class by class (tree t is class t % K),
+  // classes of T / K trees or one more
+  const int per = T / K, more = T - per * K;
+  auto place = [&](int t) { return (size_t)(t % K) * per + std::min(t % K, more) + t / K; };
+  for (int t = 0; t < T; ++t) {
+    const int dt = depth[t];
+    for (int d = 0; d < D; ++d) {
+      const size_t at = (size_t)t * D + d;
+      uint32_t bits = kNaNBits;
+      if (d < dt) std::memcpy(&bits, &threshold[at], 4);
+      sp[at] = make_uint2(d < dt ? feature[at] : 0u, bits);
+    }
+    const float w = weights[t];
+    const float* from = &leaves[(size_t)t * L];
+    float* to = lv + (size_t)t * L;
+    if (dt == D) {
+      for (int l = 0; l < L; ++l) to[l] = w * from[l];
+    } else {
+      std::fill(to, to + L, 0.0f);
+      for (int l = 0; l < (1 << dt); ++l) to[(size_t)l << (D - dt)] = w * from[l];
+    }
   }
-  TC_TRY(d_bord.alloc(ctx, bord.size(), "model borders"));
-  TC_TRY(d_vdesc.alloc(ctx, vd.size(), "model virtual features"));
-  if (!bs.empty())
-    TC_CUDA(ctx, cudaMemcpy(d_bsplits.p, bs.data(), bs.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-  TC_CUDA(ctx, cudaMemcpy(d_bord.p, bord.data(), bord.size() * sizeof(float), cudaMemcpyHostToDevice));
-  TC_CUDA(ctx, cudaMemcpy(d_vdesc.p, vd.data(), vd.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  if (stride) {
+    // binned splits in processing order: levels min(D,8)-1 .. 0, then D-1 .. 8
+    uint32_t* bs = im.at<uint32_t>(o_bs);
+    std::fill(bs, bs + std::max<size_t>(2, (size_t)T * DS), 0u);  // padding: k = 128, never reached by a bin
+    for (size_t i = 0; i < a.size(); ++i) {
+      const int t = (int)(b[i].at / (uint32_t)D), lev = (int)(b[i].at % (uint32_t)D);
+      const int p = lev < 8 ? std::min(D, 8) - 1 - lev : 8 + D - 1 - lev;
+      bs[place(t) * DS + p] = b[i].key;
+    }
+    float* bord = im.at<float>(o_bd);
+    std::fill(bord, bord + align16(nb * 4) / 4, std::nanf(""));
+    const float* vals = u.data();
+    for (int v = 0; v < V; ++v) {
+      int next = 0;
+      eytzinger_fill(vals, vf[v].cnt, bord + (vd[v].y & 0xffffffu), (size_t)1 << (vd[v].y >> 24), 1, next);
+      vals += vf[v].cnt;
+    }
+    if (V % 2) vd.push_back(make_uint2(0, 0));
+    std::memcpy(im.at<uint2>(o_vd), vd.data(), vd.size() * sizeof(uint2));
+  }
+  TC_TRY(im.upload(ctx, d_mem));
+  if (stride && K > 1 && T > 0) {
+    const size_t n = (size_t)T * L;
+    k_class_leaves<<<(unsigned)((n + 255) / 256), 256, 0, ctx->pred_stream>>>(
+        reinterpret_cast<const float*>(d_mem.p + o_lv), reinterpret_cast<float*>(d_mem.p + o_bl), T, L, K);
+    TC_CUDA(ctx, cudaGetLastError());
+  }
+  TC_CUDA(ctx, cudaStreamSynchronize(ctx->pred_stream));  // complete, whatever stream it is read on
+  auto dev = [this](size_t offset) { return d_mem.p + offset; };
+  d_splits = reinterpret_cast<const uint2*>(dev(o_sp));
+  d_leaves = reinterpret_cast<const float*>(dev(o_lv));
+  if (!stride) return TC_OK;
+  d_bsplits = reinterpret_cast<const uint32_t*>(dev(o_bs));
+  d_bleaves = reinterpret_cast<const float*>(dev(o_bl));
+  d_bord = reinterpret_cast<const float*>(dev(o_bd));
+  d_vdesc = reinterpret_cast<const uint2*>(dev(o_vd));
   bin_stride = stride;
   n_virtual = V;
-  n_bord = B;
+  n_bord = (int)nb;
   return TC_OK;
 }
 
@@ -1211,12 +1326,12 @@ namespace tc {
 
 ModelDesc model_desc(const tc_model* m) {
   ModelDesc d{};
-  d.splits = m->d_splits.p;
-  d.leaves = m->d_leaves.p;
-  d.bsplits = m->d_bsplits.p;
-  d.bleaves = m->d_bleaves.p ? m->d_bleaves.p : m->d_leaves.p;
-  d.bord = m->d_bord.p;
-  d.vdesc = m->d_vdesc.p;
+  d.splits = m->d_splits;
+  d.leaves = m->d_leaves;
+  d.bsplits = m->d_bsplits;
+  d.bleaves = m->d_bleaves;
+  d.bord = m->d_bord;
+  d.vdesc = m->d_vdesc;
   d.n_virtual = m->n_virtual;
   d.n_bord = m->n_bord;
   d.bin_stride = m->bin_stride;
@@ -1242,8 +1357,8 @@ tc_status predict_device(tc_ctx* ctx, const tc_model* m, const float* X, uint32_
                          float* out, cudaStream_t stream) {
   if (n == 0) return TC_OK;
   if (m->regular) {
-    RegDesc rd{m->d_rnodes.p, m->d_rroots.p, m->d_rweights.p, m->d_redges.p, m->d_rnedges.p,
-               m->info.n_trees, m->info.n_features, (int)m->d_rnodes.n, m->info.base_prediction};
+    RegDesc rd{m->d_rnodes, m->d_rroots, m->d_rweights, m->d_redges, m->d_rnedges,
+               m->info.n_trees, m->info.n_features, m->n_rnodes, m->info.base_prediction};
     const int rpb = (int)std::max<size_t>(1, std::min<size_t>(128, (size_t)160 * 1024 / std::max<uint32_t>(1, f)));
     const size_t smem = (size_t)rpb * f;
     static bool attr_done = false;
@@ -1504,23 +1619,29 @@ static tc_status load_regular(tc_ctx* ctx, Reader& r, tc_model_info info, const 
   m->regular = true;
   m->tcat.assign(buf, buf + len);
   m->weights = w;
-  auto up = [&]() -> tc_status {
-    TC_TRY(m->d_rnodes.alloc(ctx, std::max<size_t>(1, nodes.size()), "regular tree nodes"));
-    TC_TRY(m->d_rroots.alloc(ctx, std::max<size_t>(1, nt), "regular tree roots"));
-    TC_TRY(m->d_rweights.alloc(ctx, std::max<size_t>(1, nt), "regular tree weights"));
-    TC_TRY(m->d_redges.alloc(ctx, edges.size(), "regular model edges"));
-    TC_TRY(m->d_rnedges.alloc(ctx, ne.size(), "regular model edge counts"));
-    if (!nodes.empty())
-      TC_CUDA(ctx, cudaMemcpy(m->d_rnodes.p, nodes.data(), nodes.size() * sizeof(uint4), cudaMemcpyHostToDevice));
-    if (nt) {
-      TC_CUDA(ctx, cudaMemcpy(m->d_rroots.p, roots.data(), nt * 4, cudaMemcpyHostToDevice));
-      TC_CUDA(ctx, cudaMemcpy(m->d_rweights.p, w.data(), nt * 4, cudaMemcpyHostToDevice));
-    }
-    TC_CUDA(ctx, cudaMemcpy(m->d_redges.p, edges.data(), edges.size() * 4, cudaMemcpyHostToDevice));
-    TC_CUDA(ctx, cudaMemcpy(m->d_rnedges.p, ne.data(), ne.size() * 4, cudaMemcpyHostToDevice));
-    return TC_OK;
+  ModelImage im;
+  const size_t o_nd = im.part<uint4>(std::max<size_t>(1, nodes.size())), o_rt = im.part<uint32_t>(std::max<size_t>(1, nt)),
+               o_w = im.part<float>(std::max<size_t>(1, nt)), o_ed = im.part<float>(edges.size()),
+               o_ne = im.part<int32_t>(ne.size());
+  auto put_part = [&im](size_t offset, const auto& v) {
+    if (!v.empty()) std::memcpy(im.at<uint8_t>(offset), v.data(), v.size() * sizeof(v[0]));
   };
-  const tc_status s = up();
+  put_part(o_nd, nodes);
+  put_part(o_rt, roots);
+  put_part(o_w, w);
+  put_part(o_ed, edges);
+  put_part(o_ne, ne);
+  tc_status s = im.upload(ctx, m->d_mem);
+  if (s == TC_OK) {
+    const cudaError_t e = cudaStreamSynchronize(ctx->pred_stream);
+    if (e != cudaSuccess) s = ctx->cuda_fail(e, "model upload");
+  }
+  m->d_rnodes = reinterpret_cast<const uint4*>(m->d_mem.p + o_nd);
+  m->n_rnodes = (int)std::max<size_t>(1, nodes.size());
+  m->d_rroots = reinterpret_cast<const uint32_t*>(m->d_mem.p + o_rt);
+  m->d_rweights = reinterpret_cast<const float*>(m->d_mem.p + o_w);
+  m->d_redges = reinterpret_cast<const float*>(m->d_mem.p + o_ed);
+  m->d_rnedges = reinterpret_cast<const int32_t*>(m->d_mem.p + o_ne);
   if (s != TC_OK) {
     delete m;
     return s;
