@@ -20,7 +20,8 @@
 // sequence of launches and one copy back (50k x 20, depth 6: 0.55 ms a tree with
 // the host in every level, about 0.2 here); only the smaller child of a pair is
 // counted, in shared memory.  Deeper trees, whose buffers for every possible
-// open node would not be small, are grown with the host deciding each level.
+// open node would not be small, and trees whose buffers the memory budget has no
+// room for are grown with the host deciding each level.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -756,7 +757,7 @@ tc_status train_regular(tc_ctx* ctx, tc_dataset* ds, const tc_train_params* p, t
   // levels that have a next one
   const int pairs = std::max(1, max_open / 2), kept = std::max(1, max_open / 2);
   const size_t fs = (size_t)f * RG_SLOTS;
-  const bool on_device = D <= RGD_MAX_DEPTH && (size_t)(pairs + 2 * kept) * fs * 20 <= RGD_MEM_MAX;
+  bool on_device = D <= RGD_MAX_DEPTH && (size_t)(pairs + 2 * kept) * fs * 20 <= RGD_MEM_MAX;
   DevBuf<longlong2> q;
   DevBuf<short2> rows;
   DevBuf<unsigned long long> BG, BH;
@@ -770,18 +771,32 @@ tc_status train_regular(tc_ctx* ctx, tc_dataset* ds, const tc_train_params* p, t
   RgDev dev{};
   std::vector<RgGrown> h_grown;
   if (on_device) {
-    TC_TRY(q.alloc(ctx, n, "regular-tree fixed-point gradients"));
-    TC_TRY(rows.alloc(ctx, n, "row nodes"));
-    TC_TRY(BG.alloc(ctx, pairs * fs, "counted gradient histograms"));
-    TC_TRY(BH.alloc(ctx, pairs * fs, "counted hessian histograms"));
-    TC_TRY(BC.alloc(ctx, pairs * fs, "counted row histograms"));
-    TC_TRY(LG.alloc(ctx, 2 * kept * fs, "level gradient histograms"));
-    TC_TRY(LH.alloc(ctx, 2 * kept * fs, "level hessian histograms"));
-    TC_TRY(LC.alloc(ctx, 2 * kept * fs, "level row histograms"));
-    TC_TRY(part.alloc(ctx, (size_t)2 * pairs * fgroups, "best splits of the feature groups"));
-    TC_TRY(grown.alloc(ctx, (size_t)2 << D, "grown nodes"));
-    TC_TRY(level.alloc(ctx, 1, "level decisions"));
-    TC_TRY(state.alloc(ctx, 1, "growth state"));
+    auto alloc = [&]() -> tc_status {
+      TC_TRY(q.alloc(ctx, n, "regular-tree fixed-point gradients"));
+      TC_TRY(rows.alloc(ctx, n, "row nodes"));
+      TC_TRY(BG.alloc(ctx, pairs * fs, "counted gradient histograms"));
+      TC_TRY(BH.alloc(ctx, pairs * fs, "counted hessian histograms"));
+      TC_TRY(BC.alloc(ctx, pairs * fs, "counted row histograms"));
+      TC_TRY(LG.alloc(ctx, 2 * kept * fs, "level gradient histograms"));
+      TC_TRY(LH.alloc(ctx, 2 * kept * fs, "level hessian histograms"));
+      TC_TRY(LC.alloc(ctx, 2 * kept * fs, "level row histograms"));
+      TC_TRY(part.alloc(ctx, (size_t)2 * pairs * fgroups, "best splits of the feature groups"));
+      TC_TRY(grown.alloc(ctx, (size_t)2 << D, "grown nodes"));
+      TC_TRY(level.alloc(ctx, 1, "level decisions"));
+      return state.alloc(ctx, 1, "growth state");
+    };
+    const tc_status s = alloc();
+    if (s == TC_ERR_OOM) {
+      // no room for every possible open node: the host decides the levels, with
+      // buffers for the nodes that are open
+      on_device = false;
+      q.reset(); rows.reset(); BG.reset(); BH.reset(); BC.reset(); LG.reset(); LH.reset(); LC.reset();
+      part.reset(); grown.reset(); level.reset(); state.reset();
+    } else if (s != TC_OK) {
+      return s;
+    }
+  }
+  if (on_device) {
     TC_CUDA(ctx, cudaMemsetAsync(BG.p, 0, BG.bytes(), st));
     TC_CUDA(ctx, cudaMemsetAsync(BH.p, 0, BH.bytes(), st));
     TC_CUDA(ctx, cudaMemsetAsync(BC.p, 0, BC.bytes(), st));
