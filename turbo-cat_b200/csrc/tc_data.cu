@@ -498,7 +498,9 @@ __global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
 // Rows per block of k_assign_bins: 1024 amortise the block's 32 KB of edges;
 // fewer while the grid would not give every SM three blocks (50k x 20: 40 us in
 // 196 blocks before, 14 here).
-tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, DevBuf<float>& table, cudaStream_t st) {
+// table: scratch of assign_table(ds) floats.
+size_t assign_table(const tc_dataset* ds) { return (size_t)ds->groups * kSlots * 32; }
+tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, float* table, cudaStream_t st) {
   int rows = AB_MAX_ROWS;
   while (rows > 64 && (ds->n + rows - 1) / rows * ds->groups < 3u * (uint32_t)ds->ctx->sm_count) rows /= 2;
   const size_t smem = 256 * 32 * 4 + (size_t)32 * (rows / 4 + 1) * 4;
@@ -506,9 +508,8 @@ tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, DevBuf<float>& table,
                                         256 * 32 * 4 + 32 * (AB_MAX_ROWS / 4 + 1) * 4));
   // blocks cover the tiles' padding rows (nt: n rounded up to 32) too
   const dim3 grid((ds->nt + rows - 1) / rows, ds->groups);
-  TC_TRY(table.alloc(ds->ctx, (size_t)ds->groups * kSlots * 32, "edge table"));
-  k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(ds->edges.p, ds->n_edges.p, ds->f, table.p);
-  k_assign_bins<<<grid, AB_THREADS, smem, st>>>(ds->X.p, ds->n, ds->f, table.p, ts, ds->bins_t.p,
+  k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(ds->edges.p, ds->n_edges.p, ds->f, table);
+  k_assign_bins<<<grid, AB_THREADS, smem, st>>>(ds->X.p, ds->n, ds->f, table, ts, ds->bins_t.p,
                                                 ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p,
                                                 rows);
   return TC_OK;
@@ -1061,11 +1062,10 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   cudaStream_t st = ctx->stream;
   const uint32_t n_tiles = (uint32_t)((n + RS_TILE - 1) / RS_TILE);
   const uint8_t* ts = ds->h_cat_feats.empty() ? nullptr : ds->ts.p;
-  DevBuf<uint32_t> ka, kb, counts, totals, tcnt, U;
+  DevBuf<uint32_t> ka, kb, counts, tcnt, U;
   TC_TRY(ka.alloc(ctx, (size_t)n * f, "sort keys"));
   TC_TRY(kb.alloc(ctx, (size_t)n * f, "sort keys (alt)"));
   TC_TRY(counts.alloc(ctx, (size_t)f * 256 * n_tiles, "radix counts"));
-  TC_TRY(totals.alloc(ctx, (size_t)f * 256, "digit totals"));
   TC_TRY(tcnt.alloc(ctx, (size_t)f * n_tiles, "unique tile counts"));
   TC_TRY(U.alloc(ctx, f, "unique counts"));
   TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
@@ -1075,29 +1075,40 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   TC_TRY(ds->bins_t.alloc(ctx, (size_t)(ds->groups - 1) * ds->gstride + (size_t)ds->wlast * ds->nt,
                           "feature-group bin tiles"));
   TC_TRY(ds->bins_cm.alloc(ctx, (size_t)f * ds->np, "column-major bins"));
-  TC_CUDA(ctx, cudaMemsetAsync(ds->edges.p, 0, ds->edges.bytes(), st));
 
   if (n > 0) {
+    // the digit totals of a pass lie where the edges go afterwards (256 words a column both)
+    uint32_t* totals = reinterpret_cast<uint32_t*>(ds->edges.p);
     k_make_keys<<<(n + MK_ROWS - 1) / MK_ROWS * ((f + 31) / 32), 256, 0, st>>>(ds->X.p, n, f, ka.p);
     uint32_t* src = ka.p;
     uint32_t* dst = kb.p;
     for (int shift = 0; shift < 32; shift += 8) {
       k_radix_count<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, n, n_tiles, shift, counts.p);
-      k_digit_scan<<<32 * f, 256, 0, st>>>(counts.p, n_tiles, totals.p);
-      k_radix_scatter<false><<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, dst, n, n_tiles, shift, counts.p, totals.p,
+      k_digit_scan<<<32 * f, 256, 0, st>>>(counts.p, n_tiles, totals);
+      k_radix_scatter<false><<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, dst, n, n_tiles, shift, counts.p, totals,
                                                                        nullptr, nullptr);
       std::swap(src, dst);
     }
+    TC_CUDA(ctx, cudaMemsetAsync(ds->edges.p, 0, ds->edges.bytes(), st));
     k_unique_count<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, n, n_tiles, tcnt.p);
     k_segment_scan<<<f, 1024, 0, st>>>(tcnt.p, n_tiles, U.p);
     k_unique_pick<<<dim3(n_tiles, f), RS_THREADS, 0, st>>>(src, n, n_tiles, tcnt.p, U.p, max_bins,
                                                             compat_u8, ts, ds->edges.p);
   } else {
+    TC_CUDA(ctx, cudaMemsetAsync(ds->edges.p, 0, ds->edges.bytes(), st));
     TC_CUDA(ctx, cudaMemsetAsync(U.p, 0, U.bytes(), st));
   }
   k_edge_meta<<<(f + 127) / 128, 128, 0, st>>>(U.p, f, max_bins, compat_u8, ts, ds->edges.p, ds->n_edges.p);
+  // the assignment's table of edges lies in what the sort no longer needs
   DevBuf<float> table;
-  if (n > 0) TC_TRY(launch_assign(ds, ts, table, st));
+  float* tab = nullptr;
+  if (kb.n >= assign_table(ds)) tab = reinterpret_cast<float*>(kb.p);
+  else if (counts.n >= assign_table(ds)) tab = reinterpret_cast<float*>(counts.p);
+  else {
+    TC_TRY(table.alloc(ctx, assign_table(ds), "edge table"));
+    tab = table.p;
+  }
+  if (n > 0) TC_TRY(launch_assign(ds, ts, tab, st));
   else TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   TC_CUDA(ctx, cudaGetLastError());
   // host copy of the edges for model export / thresholds
@@ -1146,7 +1157,8 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
   TC_CUDA(ctx, cudaMemcpyAsync(ds->n_edges.p, ref->n_edges.p, ds->n_edges.bytes(), cudaMemcpyDeviceToDevice, st));
   TC_CUDA(ctx, cudaMemsetAsync(ds->nan_any.p, 0, ds->nan_any.bytes(), st));
   if (n > 0) {
-    TC_TRY(launch_assign(ds, nullptr, table, st));
+    TC_TRY(table.alloc(ctx, assign_table(ds), "edge table"));
+    TC_TRY(launch_assign(ds, nullptr, table.p, st));
     TC_CUDA(ctx, cudaGetLastError());
   } else {
     TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
@@ -1209,10 +1221,12 @@ tc_status encode_categorical(tc_dataset* ds, const uint16_t* feats, uint16_t nc,
   TC_TRY(ra.alloc(ctx, (size_t)nc * n, "category rows"));
   TC_TRY(rb.alloc(ctx, (size_t)nc * n, "category rows (alt)"));
   TC_TRY(counts.alloc(ctx, (size_t)nc * 256 * n_tiles, "radix counts"));
-  TC_TRY(totals.alloc(ctx, (size_t)nc * 256, "digit totals"));
   TC_TRY(tcnt.alloc(ctx, (size_t)nc * n_tiles, "segment tile counts"));
   TC_TRY(nseg.alloc(ctx, nc, "segment counts"));
   TC_TRY(starts.alloc(ctx, (size_t)nc * n, "segment starts"));
+  // the digit totals of a pass lie where the segment starts go afterwards
+  if (n < 256) TC_TRY(totals.alloc(ctx, (size_t)nc * 256, "digit totals"));
+  uint32_t* digit_totals = n < 256 ? totals.p : starts.p;
   TC_TRY(segid.alloc(ctx, (size_t)nc * n, "segment of each position"));
   TC_TRY(prior.alloc(ctx, 1, "label prior"));
   TC_TRY(lab_sum.alloc(ctx, 2, "label sums"));
@@ -1243,9 +1257,9 @@ tc_status encode_categorical(tc_dataset* ds, const uint16_t* feats, uint16_t nc,
   uint32_t *ks = ka.p, *kd = kb.p, *rs = ra.p, *rd = rb.p;
   for (int shift = 0; shift < 32; shift += 8) {
     k_radix_count<<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, n, n_tiles, shift, counts.p);
-    k_digit_scan<<<32 * nc, 256, 0, st>>>(counts.p, n_tiles, totals.p);
-    k_radix_scatter<true><<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, kd, n, n_tiles, shift, counts.p, totals.p, rs,
-                                                                     rd);
+    k_digit_scan<<<32 * nc, 256, 0, st>>>(counts.p, n_tiles, digit_totals);
+    k_radix_scatter<true><<<dim3(n_tiles, nc), RS_THREADS, 0, st>>>(ks, kd, n, n_tiles, shift, counts.p,
+                                                                     digit_totals, rs, rd);
     std::swap(ks, kd);
     std::swap(rs, rd);
   }
