@@ -53,3 +53,25 @@ def test_encode(capi, n, nc):
     assert np.array_equal(ds.features(), want.features())
     for x in (ds, want, eng, free):
         x.close()
+
+
+@pytest.mark.parametrize("n,f", [(1000, 32), (300, 64), (20_000, 96)])
+def test_apply_bins(capi, n, f):
+    """A held-out table's bins and its copy of the edges, in whole groups of 32
+    features (the last group's table takes up to 31 KB more than its edges)."""
+    rng = np.random.default_rng(n + 1)
+    X, T = (rng.standard_normal((n, f)).astype(np.float32) for _ in range(2))
+    free = capi.Engine(0)
+    ref, want = free.upload(X), free.upload(T)
+    ref.quantize(255, compat_u8=False)
+    want.apply_bins(ref)
+    result = f * 256 * 4 + f * 2 + f * 4 + _bins_bytes(n, f)
+    budget = 64 << 20
+    eng = capi.Engine(0, mem_budget=budget)
+    r, t = eng.upload(X), eng.upload(T)
+    r.quantize(255, compat_u8=False)
+    filler = eng.upload(np.zeros(((budget - eng.memory()[0] - result) // 4, 1), np.float32))
+    t.apply_bins(r)
+    assert np.array_equal(t.bins(), want.bins())
+    for x in (r, t, filler, ref, want, eng, free):
+        x.close()

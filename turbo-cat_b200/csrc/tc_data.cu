@@ -498,9 +498,10 @@ __global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
 // Rows per block of k_assign_bins: 1024 amortise the block's 32 KB of edges;
 // fewer while the grid would not give every SM three blocks (50k x 20: 40 us in
 // 196 blocks before, 14 here).
-// table: scratch of assign_table(ds) floats.
+// table: scratch of assign_table(ds) floats; edges, n_edges: of ds's features.
 size_t assign_table(const tc_dataset* ds) { return (size_t)ds->groups * kSlots * 32; }
-tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, float* table, cudaStream_t st) {
+tc_status launch_assign(tc_dataset* ds, const float* edges, const uint16_t* n_edges, const uint8_t* ts, float* table,
+                        cudaStream_t st) {
   int rows = AB_MAX_ROWS;
   while (rows > 64 && (ds->n + rows - 1) / rows * ds->groups < 3u * (uint32_t)ds->ctx->sm_count) rows /= 2;
   const size_t smem = 256 * 32 * 4 + (size_t)32 * (rows / 4 + 1) * 4;
@@ -508,7 +509,7 @@ tc_status launch_assign(tc_dataset* ds, const uint8_t* ts, float* table, cudaStr
                                         256 * 32 * 4 + 32 * (AB_MAX_ROWS / 4 + 1) * 4));
   // blocks cover the tiles' padding rows (nt: n rounded up to 32) too
   const dim3 grid((ds->nt + rows - 1) / rows, ds->groups);
-  k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(ds->edges.p, ds->n_edges.p, ds->f, table);
+  k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(edges, n_edges, ds->f, table);
   k_assign_bins<<<grid, AB_THREADS, smem, st>>>(ds->X.p, ds->n, ds->f, table, ts, ds->bins_t.p,
                                                 ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p,
                                                 rows);
@@ -1108,7 +1109,7 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
     TC_TRY(table.alloc(ctx, assign_table(ds), "edge table"));
     tab = table.p;
   }
-  if (n > 0) TC_TRY(launch_assign(ds, ts, tab, st));
+  if (n > 0) TC_TRY(launch_assign(ds, ds->edges.p, ds->n_edges.p, ts, tab, st));
   else TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   TC_CUDA(ctx, cudaGetLastError());
   // host copy of the edges for model export / thresholds
@@ -1147,22 +1148,24 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
     }
     ds->encoded_by = ref->id;
   }
-  TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
+  ds->edges.reset();
   TC_TRY(ds->n_edges.alloc(ctx, f, "edge counts"));
   TC_TRY(ds->nan_any.alloc(ctx, f, "NaN flags"));
   TC_TRY(ds->bins_t.alloc(ctx, (size_t)(ds->groups - 1) * ds->gstride + (size_t)ds->wlast * ds->nt,
                           "feature-group bin tiles"));
   TC_TRY(ds->bins_cm.alloc(ctx, (size_t)f * ds->np, "column-major bins"));
-  TC_CUDA(ctx, cudaMemcpyAsync(ds->edges.p, ref->edges.p, ds->edges.bytes(), cudaMemcpyDeviceToDevice, st));
-  TC_CUDA(ctx, cudaMemcpyAsync(ds->n_edges.p, ref->n_edges.p, ds->n_edges.bytes(), cudaMemcpyDeviceToDevice, st));
   TC_CUDA(ctx, cudaMemsetAsync(ds->nan_any.p, 0, ds->nan_any.bytes(), st));
   if (n > 0) {
     TC_TRY(table.alloc(ctx, assign_table(ds), "edge table"));
-    TC_TRY(launch_assign(ds, nullptr, table.p, st));
+    TC_TRY(launch_assign(ds, ref->edges.p, ref->n_edges.p, nullptr, table.p, st));
     TC_CUDA(ctx, cudaGetLastError());
+    table.reset();  // makes room for the dataset's own copy of the edges
   } else {
     TC_CUDA(ctx, cudaMemsetAsync(ds->bins_t.p, 0, ds->bins_t.bytes(), st));
   }
+  TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
+  TC_CUDA(ctx, cudaMemcpyAsync(ds->edges.p, ref->edges.p, ds->edges.bytes(), cudaMemcpyDeviceToDevice, st));
+  TC_CUDA(ctx, cudaMemcpyAsync(ds->n_edges.p, ref->n_edges.p, ds->n_edges.bytes(), cudaMemcpyDeviceToDevice, st));
   TC_CUDA(ctx, cudaStreamSynchronize(st));
   ds->h_edges = ref->h_edges;
   ds->h_n_edges = ref->h_n_edges;
