@@ -1069,6 +1069,7 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   TC_TRY(counts.alloc(ctx, (size_t)f * 256 * n_tiles, "radix counts"));
   TC_TRY(tcnt.alloc(ctx, (size_t)f * n_tiles, "unique tile counts"));
   TC_TRY(U.alloc(ctx, f, "unique counts"));
+  ds->quantized = false;  // until all of the new bins are there
   TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
   TC_TRY(ds->n_edges.alloc(ctx, f, "edge counts"));
   TC_TRY(ds->nan_any.alloc(ctx, f, "NaN flags"));
@@ -1148,6 +1149,7 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
     }
     ds->encoded_by = ref->id;
   }
+  ds->quantized = false;  // until all of the new bins are there
   ds->edges.reset();
   TC_TRY(ds->n_edges.alloc(ctx, f, "edge counts"));
   TC_TRY(ds->nan_any.alloc(ctx, f, "NaN flags"));
