@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
     const float* __restrict__ X, uint32_t n, uint32_t f, const float* __restrict__ table,
     const uint8_t* __restrict__ ts, uint8_t* __restrict__ bins_t,
     uint64_t gstride, uint32_t nt, uint32_t wlast, uint8_t* __restrict__ bins_cm, uint32_t np,
-    uint32_t* __restrict__ nan_any, int rows) {
+    int rows) {
   extern __shared__ __align__(16) float s_ab[];
   float* s_e = s_ab;                                            // [256][32]
   uint32_t* s_b = reinterpret_cast<uint32_t*>(s_ab + 256 * 32);  // [32][rows / 4 + 1] four rows' bins a word
@@ -448,7 +448,6 @@ __global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
   const uint32_t w = (blockIdx.y == gridDim.y - 1) ? wlast : 32u;  // the group's bytes per row
   uint8_t* blk = bins_t + (uint64_t)blockIdx.y * gstride;
   const float* se = s_e + lane;
-  bool nan = false;
   for (int i = warp * 4; i < rows; i += NW * 4) {
     float x[4];
     int pos[4];
@@ -480,13 +479,11 @@ __global__ void __launch_bounds__(AB_THREADS) k_assign_bins(
       uint32_t b = (uint32_t)pos[u];
       if (x[u] != x[u]) b = kNanBin;
       if (!live || r >= n) b = 0;
-      else if (b == kNanBin) nan = true;  // NaN, or a target-statistics column's top bin, which shares the slot
       four |= b << (8 * u);
       if (r < nt && (uint32_t)lane < w) blk[(size_t)r * w + lane] = (uint8_t)b;
     }
     s_b[lane * bs + (i >> 2)] = four;
   }
-  if (nan) atomicOr(&nan_any[j], 1u);
   __syncthreads();
   // column-major rows of this tile (np is a multiple of 16, r0 of 32)
   for (int jj = warp; jj < 32 && j0 + jj < f; jj += NW)
@@ -511,8 +508,7 @@ tc_status launch_assign(tc_dataset* ds, const float* edges, const uint16_t* n_ed
   const dim3 grid((ds->nt + rows - 1) / rows, ds->groups);
   k_edge_table<<<dim3(kSlots / 32, ds->groups), dim3(32, 8), 0, st>>>(edges, n_edges, ds->f, table);
   k_assign_bins<<<grid, AB_THREADS, smem, st>>>(ds->X.p, ds->n, ds->f, table, ts, ds->bins_t.p,
-                                                ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, ds->nan_any.p,
-                                                rows);
+                                                ds->gstride, ds->nt, ds->wlast, ds->bins_cm.p, ds->np, rows);
   return TC_OK;
 }
 
@@ -1072,8 +1068,6 @@ tc_status quantize(tc_dataset* ds, int max_bins, int compat_u8) {
   ds->quantized = false;  // until all of the new bins are there
   TC_TRY(ds->edges.alloc(ctx, (size_t)f * kSlots, "bin edges"));
   TC_TRY(ds->n_edges.alloc(ctx, f, "edge counts"));
-  TC_TRY(ds->nan_any.alloc(ctx, f, "NaN flags"));
-  TC_CUDA(ctx, cudaMemsetAsync(ds->nan_any.p, 0, ds->nan_any.bytes(), st));
   TC_TRY(ds->bins_t.alloc(ctx, (size_t)(ds->groups - 1) * ds->gstride + (size_t)ds->wlast * ds->nt,
                           "feature-group bin tiles"));
   TC_TRY(ds->bins_cm.alloc(ctx, (size_t)f * ds->np, "column-major bins"));
@@ -1152,11 +1146,9 @@ tc_status apply_bins(tc_dataset* ds, const tc_dataset* ref) {
   ds->quantized = false;  // until all of the new bins are there
   ds->edges.reset();
   TC_TRY(ds->n_edges.alloc(ctx, f, "edge counts"));
-  TC_TRY(ds->nan_any.alloc(ctx, f, "NaN flags"));
   TC_TRY(ds->bins_t.alloc(ctx, (size_t)(ds->groups - 1) * ds->gstride + (size_t)ds->wlast * ds->nt,
                           "feature-group bin tiles"));
   TC_TRY(ds->bins_cm.alloc(ctx, (size_t)f * ds->np, "column-major bins"));
-  TC_CUDA(ctx, cudaMemsetAsync(ds->nan_any.p, 0, ds->nan_any.bytes(), st));
   if (n > 0) {
     TC_TRY(table.alloc(ctx, assign_table(ds), "edge table"));
     TC_TRY(launch_assign(ds, ref->edges.p, ref->n_edges.p, nullptr, table.p, st));

@@ -122,7 +122,6 @@ struct DevPtrs {
   const uint8_t* bins_cm;
   const float* edges;            // [f][256]
   const uint16_t* n_edges;
-  const uint32_t* nan_any;       // [f] nonzero: the feature has NaN rows
   const float* y;
   float* pred;                   // [K][n]
   float2* gh;                    // [K][n]
@@ -380,22 +379,6 @@ __global__ void k_apply_last(DevCfg c, DevPtrs P) {
 
 // ------------------------------------------------------------------ hist --
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 struct HistShape {
   static constexpr int W = 32;                          // histogram columns (features) of an item at most
   static constexpr int FIELDS = 4;                      // u32 accumulators per (slot, column)
@@ -484,10 +467,10 @@ __device__ __forceinline__ void load_slice(uint32_t (&w)[W4], const uint8_t* src
 //
 // What bounds it: the shared-memory pipe.  32-bit `red.shared.add` with 32
 // different banks per instruction issues at one warp instruction per clock
-// and SM (measured: 31 lanes / clk / SM at 255, 32 and 4 bins), and a slice
-// of 32 bytes per row costs 8 wavefronts per 32 rows, so four atomics per
-// pair allow 7.5 pairs / clk / SM.  With a row per lane nothing else of the
-// loop needs that pipe; with four rows per step and eight lanes per row (each
+// and SM (measured: 31 lanes / clk / SM at 255, 32 and 4 bins): 128 wavefronts
+// for 32 rows of 32 columns at four atomics per pair, beside 19 for the rows'
+// slices, so 1024 pairs take 147 clocks, 7.0 pairs / clk / SM.  With a row per
+// lane nothing else of the loop needs that pipe; with four rows per step and eight lanes per row (each
 // converting the row again, bounds and padding tested per update) the loop
 // took 110 instructions and 21 wavefronts per 128 pairs.  Root level of 2.5M
 // rows x 200 features: 518 -> 372 us (5.0 pairs / clk / SM over the launch);
@@ -871,7 +854,9 @@ __device__ __forceinline__ void node_gains(const double2* tile, double lam, int 
 // node per warp (the pair's accumulators read twice), 16-byte accesses at a
 // 128-byte stride and a pick of two 8-step trees with block barriers, the
 // scans of an iteration took 163 us on 2.5M x 200 (depth 8), here 122; 215 and
-// 150 on 1M x 50, ten classes; 79 and 60 on 50k x 20.
+// 150 on 1M x 50, ten classes; 79 and 60 on 50k x 20.  (A thread holds a pair's
+// two nodes, 64 registers of doubles, beside the gains: 128 registers and 48
+// bytes of spills.)
 __global__ void __launch_bounds__(SCAN_WARPS * 32) k_scan(DevCfg c, DevPtrs P, int d) {
   __shared__ __align__(16) double2 s_tile[SCAN_WARPS][TILE_UNITS];
   __shared__ PickCand s_pick[SCAN_WARPS];
@@ -1700,7 +1685,6 @@ struct tc_trainer {
   tc_train_params prm{};
   DevCfg cfg{};
   DevPtrs ptr{};
-  int J = 2;
   int hist_grid = 0;
   int T_cap = 0;
   int iters_done = 0;
@@ -1795,7 +1779,7 @@ struct tc_trainer {
   void mark_begin(int cls, cudaStream_t st);
   void mark_end(cudaStream_t st, double bytes = 0.0);
   tc_status setup(int given_gh_rows_only);
-  tc_status configure(int J, int waves);
+  tc_status configure(int waves);
   tc_status autotune();
   void launch_level(const DevCfg& c, const DevPtrs& P, int d, cudaStream_t st);
   tc_status enqueue_iteration(cudaStream_t st);
@@ -1884,7 +1868,6 @@ tc_status tc_trainer::setup(int) {
   TC_CUDA(ctx, cudaMemsetAsync(fcnt.p, 0, fcnt.bytes(), ctx->stream));
 
   ptr.bins_t = ds->bins_t.p; ptr.bins_cm = ds->bins_cm.p; ptr.edges = ds->edges.p; ptr.n_edges = ds->n_edges.p;
-  ptr.nan_any = ds->nan_any.p;
   ptr.y = ds->y.p; ptr.pred = pred.p; ptr.gh = gh.p; ptr.cgh = cgh.p; ptr.leaf = leaf.p; ptr.rows = rows.p;
   ptr.hist[0] = hist0.p; ptr.hist[1] = hist1.p; ptr.acc = acc.p; ptr.rchunk = rchunk.p;
   ptr.seg_start = seg_start.p; ptr.seg_len = seg_len.p; ptr.small = small.p; ptr.nstat = nstat.p;
@@ -1900,17 +1883,16 @@ tc_status tc_trainer::setup(int) {
   cudaFuncSetAttribute(k_partition<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 256 * (PART_THREADS / 32));
   TC_CUDA(ctx, cudaEventCreate(&ev0));
   TC_CUDA(ctx, cudaEventCreate(&ev1));
-  return configure(1, 2);  // 32-column feature groups (the only width), 2 waves before tuning
+  return configure(2);  // waves, before tuning
 }
 
-// Feature-group width (32*J columns) and work items per histogram launch
-// (waves x resident histogram blocks).
-tc_status tc_trainer::configure(int J_, int waves) {
+// Work items per histogram launch (waves x resident histogram blocks) of feature
+// groups of 32 columns.
+tc_status tc_trainer::configure(int waves) {
   const uint32_t f = cfg.f;
   const int K = cfg.K, D = cfg.D;
   const int Pmax = 1 << (D - 1);
-  J = J_;
-  const int W = 32 * J;
+  const int W = HistShape::W;
   const int G = (int)((f + W - 1) / W);
   hist_grid = ctx->sm_count;  // one 1024-thread block per SM
   hist_waves = waves;
@@ -1930,7 +1912,7 @@ tc_status tc_trainer::configure(int J_, int waves) {
 
 namespace {
 std::mutex g_tune_mu;
-std::map<std::string, std::array<int, 3>> g_tune_cache;  // shape -> (J, waves, rows_min)
+std::map<std::string, std::array<int, 2>> g_tune_cache;  // shape -> (waves, rows_min)
 }  // namespace
 
 // Project autotuner: times a few iterations for every items-per-launch
@@ -1944,19 +1926,15 @@ tc_status tc_trainer::autotune() {
     std::lock_guard<std::mutex> g(g_tune_mu);
     auto it = g_tune_cache.find(key);
     if (it != g_tune_cache.end()) {
-      hist_rows_min = it->second[2];
-      TC_TRY(configure(it->second[0], it->second[1]));
+      hist_rows_min = it->second[1];
+      TC_TRY(configure(it->second[0]));
       tuned = true;
       return TC_OK;
     }
   }
   cudaStream_t st = ctx->stream;
-  // 64-column groups (one block per SM) measured slower on every configuration
-  // (C2: 1.7 vs 1.2 ms/iteration, C3: 9.3 vs 7.0); they stay available as a
-  // parameter but are not tried
-  const int jmax = 1;
   double best = 1e30;
-  int bj = J, bw = hist_waves, br = hist_rows_min;
+  int bw = hist_waves, br = hist_rows_min;
   // candidates (waves, rows_min): 1, 2, 4, 8 waves of items of at least 512
   // rows; on small shapes also one wave of larger items (fewer items flush
   // fewer partial histograms into the same accumulators)
@@ -1969,36 +1947,33 @@ tc_status tc_trainer::autotune() {
   // first iterations; the best of two timed runs of them counts
   const int trial_iters = 2;  // + 1 warm-up: 3 <= n_estimators iterations (checked by the caller)
   for (int rep = 0; rep < 2; ++rep) {
-    for (int j = 1; j <= jmax; ++j) {
-      for (const auto& wr : cand) {
-        const int waves = wr.first;
-        hist_rows_min = wr.second;
-        TC_TRY(configure(j, waves));
-        TC_TRY(init_predictions());
-        enqueue_iteration(st);  // warm-up (first touch of the buffers)
-        TC_TRY(init_predictions());
-        TC_CUDA(ctx, cudaEventRecord(ev0, st));
-        for (int i = 0; i < trial_iters; ++i) enqueue_iteration(st);
-        TC_CUDA(ctx, cudaEventRecord(ev1, st));
-        TC_CUDA(ctx, cudaEventSynchronize(ev1));
-        float ms = 0.0f;
-        TC_CUDA(ctx, cudaEventElapsedTime(&ms, ev0, ev1));
-        if (ms < best) {
-          best = ms;
-          bj = j;
-          bw = waves;
-          br = hist_rows_min;
-        }
+    for (const auto& wr : cand) {
+      const int waves = wr.first;
+      hist_rows_min = wr.second;
+      TC_TRY(configure(waves));
+      TC_TRY(init_predictions());
+      enqueue_iteration(st);  // warm-up (first touch of the buffers)
+      TC_TRY(init_predictions());
+      TC_CUDA(ctx, cudaEventRecord(ev0, st));
+      for (int i = 0; i < trial_iters; ++i) enqueue_iteration(st);
+      TC_CUDA(ctx, cudaEventRecord(ev1, st));
+      TC_CUDA(ctx, cudaEventSynchronize(ev1));
+      float ms = 0.0f;
+      TC_CUDA(ctx, cudaEventElapsedTime(&ms, ev0, ev1));
+      if (ms < best) {
+        best = ms;
+        bw = waves;
+        br = hist_rows_min;
       }
     }
   }
   hist_rows_min = br;
-  TC_TRY(configure(bj, bw));
+  TC_TRY(configure(bw));
   TC_TRY(init_predictions());
   launches = 0;
   tuned = true;
   std::lock_guard<std::mutex> g(g_tune_mu);
-  g_tune_cache[key] = {bj, bw, br};
+  g_tune_cache[key] = {bw, br};
   return TC_OK;
 }
 
