@@ -21,8 +21,8 @@
 // (src/core/dataset.cpp:346-379) with the model's borders in place of the
 // training edges.
 //
-// Kernel layout: a block of 16 warps owns a tile of 256 rows (128 when the
-// launch has too few rows to fill the device) of one job: one request of a
+// Kernel layout: a block of 16 warps owns a tile of 256 or 128 rows
+// (predict_tiling) of one job: one request of a
 // coalesced serving batch, or the whole input of a single call.  Trees stream
 // through shared memory in chunks (splits, and leaves up to depth 6; two
 // chunks in flight: cp.async, the next chunk lands while the current one is
