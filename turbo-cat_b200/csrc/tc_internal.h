@@ -220,10 +220,8 @@ struct tc_model {
   std::vector<float> weights;       // [T]
   std::vector<float> edges;         // [f][255]
   std::vector<uint16_t> n_edges;    // [f]
-  // device arrays used by the predict kernels, in one block, and the leaves of
-  // several classes class by class
+  // device arrays used by the predict kernels, in one allocation
   AnyStreamBuf<uint8_t> d_mem;
-  AnyStreamBuf<float> d_class_leaves;
   const uint2* d_splits = nullptr;        // [T][D] (feature, threshold bits), padded to depth D
   const float* d_leaves = nullptr;        // [T][2^D] (weights folded in, padded trees' leaves spread)
   const uint32_t* d_bsplits = nullptr;    // binned form: [T][D rounded to even] virtual feature << 8 | 128 - k, class by class

@@ -1108,14 +1108,21 @@ void eytzinger_fill(const float* vals, int cnt, float* t, size_t n, size_t i, in
 }
 
 // A model's device arrays, each on a 16-byte boundary of one block: laid out
-// (part), filled on the host (at), then allocated and copied at once.
+// (part; device_part, after those, for what the device writes itself), filled on
+// the host (at), then allocated and copied at once.
 struct ModelImage {
-  size_t size = 0;
+  size_t size = 0, device_size = 0;
   std::unique_ptr<uint8_t[]> host;
   template <class T>
   size_t part(size_t count) {
     const size_t at = size;
-    size = align16(size + count * sizeof(T));
+    size = device_size = align16(size + count * sizeof(T));
+    return at;
+  }
+  template <class T>
+  size_t device_part(size_t count) {
+    const size_t at = device_size;
+    device_size = align16(device_size + count * sizeof(T));
     return at;
   }
   template <class T>
@@ -1125,7 +1132,7 @@ struct ModelImage {
   }
   // (on pred_stream: the caller waits for it before the model is used)
   tc_status upload(tc_ctx* ctx, AnyStreamBuf<uint8_t>& mem) {
-    TC_TRY(mem.alloc(ctx, size, "model arrays"));
+    TC_TRY(mem.alloc(ctx, device_size, "model arrays"));
     TC_CUDA(ctx, cudaMemcpyAsync(mem.p, host.get(), size, cudaMemcpyHostToDevice, ctx->pred_stream));
     return TC_OK;
   }
@@ -1238,16 +1245,16 @@ tc_status tc_model::upload() {
   // binned splits: a tree's are padded to whole 8-byte units; borders and virtual
   // features to whole 16-byte copies (parts are)
   const int DS = 2 * split_units(D, true);
-  size_t o_bs = 0, o_bd = 0, o_vd = 0;
-  const size_t n_lv = (size_t)T * L;
+  size_t o_bs = 0, o_bl = o_lv, o_bd = 0, o_vd = 0;
   if (stride) {
     o_bs = im.part<uint32_t>(std::max<size_t>(2, (size_t)T * DS));
     o_bd = im.part<float>(nb);
     o_vd = im.part<uint2>((size_t)V);
+    if (K > 1) o_bl = im.device_part<float>((size_t)std::max(1, T * L));
     // several classes are served by the float walk where the budget has no room
     // for a second copy of their leaves
-    if (K > 1 && !ctx->has_room(im.size + n_lv * sizeof(float)) && ctx->has_room(plain)) {
-      im.size = plain;
+    if (K > 1 && !ctx->has_room(im.device_size) && ctx->has_room(plain)) {
+      im.size = im.device_size = plain;
       stride = 0;
     }
   }
@@ -1298,18 +1305,19 @@ tc_status tc_model::upload() {
     std::memcpy(im.at<uint2>(o_vd), vd.data(), vd.size() * sizeof(uint2));
   }
   TC_TRY(im.upload(ctx, d_mem));
-  auto dev = [this](size_t offset) { return d_mem.p + offset; };
-  d_splits = reinterpret_cast<const uint2*>(dev(o_sp));
-  d_leaves = d_bleaves = reinterpret_cast<const float*>(dev(o_lv));
   if (stride && K > 1 && T > 0) {
-    TC_TRY(d_class_leaves.alloc(ctx, n_lv, "model leaves by class"));
-    k_class_leaves<<<(unsigned)((n_lv + 255) / 256), 256, 0, ctx->pred_stream>>>(d_leaves, d_class_leaves.p, T, L, K);
+    const size_t n = (size_t)T * L;
+    k_class_leaves<<<(unsigned)((n + 255) / 256), 256, 0, ctx->pred_stream>>>(
+        reinterpret_cast<const float*>(d_mem.p + o_lv), reinterpret_cast<float*>(d_mem.p + o_bl), T, L, K);
     TC_CUDA(ctx, cudaGetLastError());
-    d_bleaves = d_class_leaves.p;
   }
   TC_CUDA(ctx, cudaStreamSynchronize(ctx->pred_stream));  // complete, whatever stream it is read on
+  auto dev = [this](size_t offset) { return d_mem.p + offset; };
+  d_splits = reinterpret_cast<const uint2*>(dev(o_sp));
+  d_leaves = reinterpret_cast<const float*>(dev(o_lv));
   if (!stride) return TC_OK;
   d_bsplits = reinterpret_cast<const uint32_t*>(dev(o_bs));
+  d_bleaves = reinterpret_cast<const float*>(dev(o_bl));
   d_bord = reinterpret_cast<const float*>(dev(o_bd));
   d_vdesc = reinterpret_cast<const uint2*>(dev(o_vd));
   bin_stride = stride;
