@@ -7,13 +7,20 @@
 
 namespace {
 // The process's contexts: an allocation that fails in one takes the blocks that
-// the others keep on its device.
-std::mutex g_contexts_mu;
-std::vector<tc_ctx*> g_contexts;
+// the others keep on its device.  (Never destroyed: a context may outlive static
+// objects.)
+struct Contexts {
+  std::mutex mu;
+  std::vector<tc_ctx*> all;
+};
+Contexts& contexts() {
+  static Contexts* c = new Contexts();
+  return *c;
+}
 
 void trim_all(int device) {
-  std::lock_guard<std::mutex> g(g_contexts_mu);
-  for (tc_ctx* c : g_contexts)
+  std::lock_guard<std::mutex> g(contexts().mu);
+  for (tc_ctx* c : contexts().all)
     if (c->device == device) c->trim_pool();
 }
 }  // namespace
@@ -146,8 +153,8 @@ tc_status tc_ctx_create(int device, size_t mem_budget, tc_ctx** out) {
     return TC_ERR_CUDA;
   }
   {
-    std::lock_guard<std::mutex> g(g_contexts_mu);
-    g_contexts.push_back(c);
+    std::lock_guard<std::mutex> g(contexts().mu);
+    contexts().all.push_back(c);
   }
   *out = c;
   return TC_OK;
@@ -156,8 +163,9 @@ tc_status tc_ctx_create(int device, size_t mem_budget, tc_ctx** out) {
 void tc_ctx_destroy(tc_ctx* ctx) {
   if (!ctx) return;
   {
-    std::lock_guard<std::mutex> g(g_contexts_mu);
-    g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+    std::lock_guard<std::mutex> g(contexts().mu);
+    auto& all = contexts().all;
+    all.erase(std::remove(all.begin(), all.end(), ctx), all.end());
   }
   cudaSetDevice(ctx->device);
   {
